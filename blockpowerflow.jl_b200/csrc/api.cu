@@ -143,7 +143,8 @@ bpf_status csr_pattern_to_host(bpf_ctx *ctx, const bpf_csr_desc *A, std::vector<
 // numeric factorization and the triangular solves need.  P->fv is allocated, not filled.
 // kind PREC_ILU0 / PREC_LU: unit L + U on the pattern; PREC_IC0: L and L' (lower part).
 bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
-                      const std::vector<int> &ci, const std::vector<int> &diag, bpf_prec **out) {
+                      const std::vector<int> &ci, const std::vector<int> &diag, int fdtype,
+                      const std::vector<int> &perm, bpf_prec **out) {
     *out = nullptr;
     const int nnz = n > 0 ? rp[n] : 0;
     bpf_prec *P = new bpf_prec();
@@ -151,10 +152,39 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     P->kind = kind;
     P->n = n;
     P->nnz = nnz;
+    P->fdtype = fdtype;
     const bool ic = (kind == PREC_IC0);
     TriHost lo = build_tri(n, rp.data(), ci.data(), diag.data(), 0, !ic);
     TriHost up = ic ? build_tri(n, rp.data(), ci.data(), diag.data(), 2, false)
                     : build_tri(n, rp.data(), ci.data(), diag.data(), 1, false);
+    P->col = (kind == PREC_ILU0 || ic) && n > 0 && trsv_col_fits(ctx, n, fdtype);
+    std::vector<int> pos0, pos01(n), pos1, tpos[2];
+    TriStream cs[2];
+    if (kind != PREC_LU) {
+        tpos[0].assign(nnz, -1);
+        tpos[1].assign(nnz, -1);
+    }
+    if (P->col) {
+        const int nring = trsv_col_ring(ctx, n, fdtype);
+        tri_to_stream(lo, fdtype, nring, 0, pos0, cs[0], tpos[0]);
+        tri_to_stream(up, fdtype, nring, (int)cs[0].coff.size() - 1, pos1, cs[1], tpos[1]);
+        for (int q = 0; q < n; q++) pos01[q] = pos0[up.rows[q]];
+        if (!perm.empty()) {   // positions of the block's rows: factor row i is row perm[i]
+            std::vector<int> b0(n), b1(n);
+            for (int i = 0; i < n; i++) {
+                b0[perm[i]] = pos0[i];
+                b1[perm[i]] = pos1[i];
+            }
+            pos0.swap(b0);
+            pos1.swap(b1);
+        }
+    } else if (kind != PREC_LU) {
+        for (int w = 0; w < 2; w++) {
+            const TriHost &t = w == 0 ? lo : up;
+            for (size_t k = 0; k < t.map.size(); k++) tpos[w][t.map[k]] = (int)k;
+            for (size_t q = 0; q < t.dmap.size(); q++) tpos[w][t.dmap[q]] = -2 - (int)q;
+        }
+    }
     std::vector<int> pp;
     PairVec pdst, psrc;
     const char *env_pl = getenv("BPF_LU_PAIRLESS");
@@ -178,8 +208,8 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
         P->npairs = upd;
     }
     bpf_status s;
-    if ((s = tri_upload(ctx, lo, P->lower)) != BPF_SUCCESS) return fail(s);
-    if ((s = tri_upload(ctx, up, P->upper)) != BPF_SUCCESS) return fail(s);
+    if ((s = tri_upload(ctx, lo, P->lower, !P->col)) != BPF_SUCCESS) return fail(s);
+    if ((s = tri_upload(ctx, up, P->upper, !P->col)) != BPF_SUCCESS) return fail(s);
     cudaError_t e = cudaSuccess;
     auto up_i = [&](int **d, const auto &h) {   // std::vector<int> or PairVec
         if (e != cudaSuccess || h.empty()) return;
@@ -197,6 +227,33 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     up_i(&P->pp, pp);
     up_i(&P->pdst, pdst);
     up_i(&P->psrc, psrc);
+    if (P->col) {
+        up_i(&P->pos0, pos0);
+        up_i(&P->pos01, pos01);
+        up_i(&P->pos1, pos1);
+    }
+    if (P->col) {
+        for (int w = 0; w < 2; w++) {
+            P->cs[w].nchunk = (int)cs[w].coff.size() - 1;
+            P->cs[w].nstage = cs[w].nstage;
+            P->cs[w].diag = cs[w].diag;
+            P->cs[w].len = cs[w].bytes.size();
+            P->cs[w].nslab = cs[w].cslab.back();
+            up_i(&P->cs[w].coff, cs[w].coff);
+            up_i(&P->cs[w].cslab, cs[w].cslab);
+            up_i(&P->cs[w].head, cs[w].head);
+            if (e == cudaSuccess && !cs[w].bytes.empty()) {
+                e = cudaMalloc((void **)&P->cs[w].bytes, cs[w].bytes.size());
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(P->cs[w].bytes, cs[w].bytes.data(), cs[w].bytes.size(), cudaMemcpyHostToDevice,
+                                        ctx->stream);
+            }
+        }
+    }
+    up_i(&P->tpos[0], tpos[0]);
+    up_i(&P->tpos[1], tpos[1]);
+    if (kind == PREC_ILU0)
+        for (int i = 0; i < n; i++) P->max_row = std::max(P->max_row, rp[i + 1] - rp[i]);
     if (kind == PREC_LU && n > 0) {
         // column-step levels: step k depends on the steps j < k with L(k, j) != 0 (they update
         // row k) or U(j, k) != 0 (they update column k)
@@ -504,9 +561,8 @@ static bpf_status prec_create(bpf_ctx *ctx, const bpf_csr_desc *A, int nrhs, int
         if (bad >= 0) return set_error(ctx, BPF_ERR_SINGULAR, "structurally zero diagonal at row %d", bad);
     }
     bpf_prec *P = nullptr;
-    BPF_TRY(prec_setup(ctx, kind, n, rp, ci, diag, &P));
+    BPF_TRY(prec_setup(ctx, kind, n, rp, ci, diag, fdtype, perm, &P));
     P->nrhs = nrhs;
-    P->fdtype = fdtype;
     P->ordering = ordering;
     bool ic = (kind == PREC_IC0);
     auto fail = [&](bpf_status s) {
@@ -518,6 +574,11 @@ static bpf_status prec_create(bpf_ctx *ctx, const bpf_csr_desc *A, int nrhs, int
     if (!perm.empty()) {
         cudaError_t e = cudaMalloc((void **)&P->perm, sizeof(int) * n);
         if (e == cudaSuccess && nnz > 0) e = cudaMalloc((void **)&P->amap, sizeof(int) * nnz);
+        std::vector<int> fsrc(nnz);
+        for (int k = 0; k < nnz; k++) fsrc[amap[k]] = k;
+        if (e == cudaSuccess && nnz > 0) e = cudaMalloc((void **)&P->fsrc, sizeof(int) * nnz);
+        if (e == cudaSuccess && nnz > 0)
+            e = cudaMemcpyAsync(P->fsrc, fsrc.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(P->perm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess && nnz > 0)
@@ -527,10 +588,7 @@ static bpf_status prec_create(bpf_ctx *ctx, const bpf_csr_desc *A, int nrhs, int
         P->perm_host = perm;
         if ((s = prec_reserve_z(ctx, P, std::max(nrhs, 1))) != BPF_SUCCESS) return fail(s);
     }
-    if ((s = prec_load_values(ctx, P, (const double *)A->vals)) != BPF_SUCCESS) return fail(s);
-    if ((s = factor_numeric(ctx, P)) != BPF_SUCCESS) return fail(s);
-    if ((s = tri_scatter(ctx, P->lower, P->fv)) != BPF_SUCCESS) return fail(s);
-    if ((s = tri_scatter(ctx, P->upper, P->fv)) != BPF_SUCCESS) return fail(s);
+    if ((s = prec_factor(ctx, P, (const double *)A->vals)) != BPF_SUCCESS) return fail(s);
     if ((s = check_dev_status(ctx, ic ? "ic0" : "ilu0")) != BPF_SUCCESS) return fail(s);
     *out = P;
     return BPF_SUCCESS;
@@ -566,15 +624,18 @@ bpf_status bpf_prec_refactor(bpf_prec *P, const double *vals) {
     if (!P) return BPF_ERR_INVALID_VALUE;
     bpf_ctx *ctx = P->ctx;
     if (P->nnz > 0 && !vals) return set_error(ctx, BPF_ERR_INVALID_VALUE, "null values");
-    BPF_TRY(prec_load_values(ctx, P, vals));
     if (P->kind == PREC_BJ) {
+        BPF_TRY(prec_load_values(ctx, P, vals));
         BPF_TRY(bj_setup(ctx, P));
         return check_dev_status(ctx, "block-Jacobi (singular diagonal block)");
     }
-    BPF_TRY(factor_numeric(ctx, P));
-    BPF_TRY(tri_scatter(ctx, P->lower, P->fv));
-    BPF_TRY(tri_scatter(ctx, P->upper, P->fv));
+    BPF_TRY(prec_factor(ctx, P, vals));
     return check_dev_status(ctx, P->kind == PREC_IC0 ? "ic0 refactor" : "ilu0 refactor");
+}
+
+static bool blocks_disjoint(int n, int p, const double *X, int ldx, const double *Y, int ldy) {
+    const double *xe = X + (size_t)(p - 1) * ldx + n, *ye = Y + (size_t)(p - 1) * ldy + n;
+    return xe <= Y || ye <= X;
 }
 
 bpf_status bpf_prec_apply(bpf_prec *P, int p, const double *X, int ldx, double *Y, int ldy) {
@@ -588,6 +649,12 @@ bpf_status bpf_prec_apply(bpf_prec *P, int p, const double *X, int ldx, double *
     if (n == 0 || p == 0) return BPF_SUCCESS;
     const int chunk = 256;
     bpf_status st;
+    // column by column in shared memory, straight on the caller's blocks (unless they overlap
+    // without being the same block: then through the row-major copy below)
+    if (P->col && (blocks_disjoint(n, p, X, ldx, Y, ldy) || (X == Y && ldx == ldy))) {
+        BPF_TRY(prec_reserve_z(ctx, P, std::min(p, chunk)));
+        return trsv_col(ctx, P, p, X, ldx, Y, ldy);
+    }
     double *buf = (double *)ws_get(ctx, WS_A, sizeof(double) * (size_t)n * std::min(p, chunk), &st);
     if (!buf) return st;
     BPF_TRY(prec_reserve_z(ctx, P, std::min(p, chunk)));
@@ -632,6 +699,17 @@ bpf_status bpf_prec_destroy(bpf_prec *P) {
     cudaFree(P->fv);
     cudaFree(P->perm);
     cudaFree(P->amap);
+    cudaFree(P->fsrc);
+    cudaFree(P->pos0);
+    cudaFree(P->pos01);
+    cudaFree(P->pos1);
+    for (int w = 0; w < 2; w++) {
+        cudaFree(P->tpos[w]);
+        cudaFree(P->cs[w].bytes);
+        cudaFree(P->cs[w].coff);
+        cudaFree(P->cs[w].cslab);
+        cudaFree(P->cs[w].head);
+    }
     cudaFree(P->zbuf);
     cudaFree(P->sf_flags);
     cudaFree(P->cl_lev_ptr);

@@ -59,6 +59,7 @@ enum Slot : int {
     WS_ZB,            // flexible GMRES: preconditioned basis blocks
     WS_FLAGS,         // small device status words (tensor-core GEMM errors)
     WS_DEFL,          // deflated block-GMRES: Q_C, Z R^{-1}, E_j blocks
+    WS_COL,           // column-major copy of a row-major block (column triangular solves)
     WS_COUNT
 };
 

@@ -8,13 +8,14 @@
 //  * One host analysis per sparsity pattern: dependency levels of the forward and backward
 //    solves, rows stored level by level (so a level's rows are contiguous), and for the
 //    numeric factorization the list of (destination, source) update pairs of every L entry.
-//  * The numeric factorization is a cooperative persistent kernel: one warp per row, the
-//    rows of a level spread over the grid, one bounded grid barrier between levels.
-//  * ldiv! is ONE cooperative launch that runs every level of L and then of U (or L'):
-//    a group of G lanes per row, lanes over the p right-hand sides of the row-major block,
-//    the row's (col, val) pairs broadcast by shuffles.  Values written in earlier levels are
-//    read with ld.global.cg (L2, never a stale L1 line).  No scratch vector: the forward
-//    solve writes Y and the backward solve updates Y in place.
+//  * ILU(0) is factored as a data flow (factor_df_kernel: rows wait for the values they read);
+//    IC(0), and rows too long for shared memory, by a cooperative kernel with a grid barrier per
+//    level (factor_coop_kernel).
+//  * ldiv! solves one right-hand side per CTA in shared memory while the column fits
+//    (trsv_col.cu); larger factors run here in ONE cooperative launch, sync-free for 17-256 columns
+//    (trsv_sf_kernel), level by level otherwise (trsv2_coop_kernel): a group of G lanes per row,
+//    lanes over the p right-hand sides of the row-major block, the row's (col, val) pairs broadcast
+//    by shuffles.
 //  * FP32 factors (factor_dtype = BPF_F32) keep float copies of L, U and 1/diag, read half the
 //    factor bytes and compute in FP32; the block stays FP64 in memory.
 #include <algorithm>
@@ -233,7 +234,7 @@ static bpf_status upload(bpf_ctx *ctx, T **dptr, const std::vector<T> &h) {
     return BPF_SUCCESS;
 }
 
-bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d) {
+bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d, bool values) {
     d.n = h.n;
     d.nlev = h.nlev;
     d.nnz = (int)h.ci.size();
@@ -242,6 +243,7 @@ bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d) {
     d.lev_ptr_h = h.lev_ptr;
     BPF_TRY(upload(ctx, &d.lev_ptr, h.lev_ptr));
     BPF_TRY(upload(ctx, &d.rows, h.rows));
+    if (!values) return BPF_SUCCESS;
     BPF_TRY(upload(ctx, &d.rp, h.rp));
     BPF_TRY(upload(ctx, &d.ci, h.ci));
     BPF_TRY(upload(ctx, &d.map, h.map));
@@ -293,6 +295,64 @@ bpf_status tri_scatter(bpf_ctx *ctx, const TriDev &d, const double *fv) {
     int work = std::max(d.nnz, d.n);
     int blocks = std::min(ceil_div(work, 256), ctx->num_sms * 8);
     tri_scatter_kernel<<<blocks, 256, 0, ctx->stream>>>(d.args(), fv);
+    BPF_LAUNCHED(ctx);
+    return BPF_SUCCESS;
+}
+
+// The storage of the two sweeps that a factor entry goes to (bpf_prec::tpos), CSR or stream.
+struct SweepStore {
+    const int *tpos[2];
+    double *val[2], *dinv[2];      // level-sorted storage, FP64 and FP32
+    float *valf[2], *dinvf[2];
+    unsigned char *stream[2];      // or the streams (column solves), of FP32 values if f32
+    int col, f32;
+};
+
+__device__ __forceinline__ void sweep_put(const SweepStore &s, int e, double x) {
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+        const int t = s.tpos[w] ? __ldg(s.tpos[w] + e) : -1;
+        if (t == -1) continue;
+        const double v = t >= 0 ? x : 1.0 / x;
+        const int k = t >= 0 ? t : -2 - t;
+        if (s.col) {
+            if (s.f32) reinterpret_cast<float *>(s.stream[w])[k] = (float)v;
+            else reinterpret_cast<double *>(s.stream[w])[k] = v;
+        } else if (t >= 0) {
+            s.val[w][k] = v;
+            s.valf[w][k] = (float)v;
+        } else {
+            s.dinv[w][k] = v;
+            s.dinvf[w][k] = (float)v;
+        }
+    }
+}
+
+static SweepStore sweep_store(const bpf_prec *P) {
+    SweepStore s;
+    const TriDev *t[2] = {&P->lower, &P->upper};
+    for (int w = 0; w < 2; w++) {
+        s.tpos[w] = P->tpos[w];
+        s.val[w] = t[w]->val;
+        s.valf[w] = t[w]->valf;
+        s.dinv[w] = t[w]->dinv;
+        s.dinvf[w] = t[w]->dinvf;
+        s.stream[w] = P->cs[w].bytes;
+    }
+    s.col = P->col;
+    s.f32 = P->fdtype == BPF_F32;
+    return s;
+}
+
+__global__ void sweep_scatter_kernel(int nnz, const double *__restrict__ fv, SweepStore s) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) sweep_put(s, e, fv[e]);
+}
+
+// Factor values (pattern order) into both sweeps' storage.
+static bpf_status sweep_scatter(bpf_ctx *ctx, const bpf_prec *P) {
+    if (P->nnz == 0) return BPF_SUCCESS;
+    const int blocks = std::min(ceil_div(P->nnz, 256), ctx->num_sms * 8);
+    sweep_scatter_kernel<<<blocks, 256, 0, ctx->stream>>>(P->nnz, P->fv, sweep_store(P));
     BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;
 }
@@ -383,6 +443,128 @@ __global__ void __launch_bounds__(256) factor_coop_kernel(FactorArgs a) {
         if (l + 1 < a.nlev) {
             if (!grid_barrier(a.ds, gen)) return;
         }
+    }
+}
+
+// ILU(0) as a data flow: a warp per row in level order, the row held in shared memory; a row
+// waits only for the values it reads, and a value is its own ready mark.
+//
+// Bound: the chain of dependency levels.  A grid barrier per level cost 5-15 us a level; refactor()
+// of the 9,000-bus pattern took 231 us in natural order (14 levels), 427 us in minimum-degree order
+// (26), 4.7 ms in reverse Cuthill-McKee order (456), and takes 62, 94 and 1,285 us this way (70,000
+// buses: 381 -> 126 us).  Here
+// every factor value starts as a signalling-NaN bit pattern that no arithmetic can produce (results
+// of operations are quiet NaNs, and stores check), a reader polls the value itself until it is
+// something else, and a producer needs no fence: 64-bit accesses are single, and no value vouches for
+// another.  No deadlock: the unfinished row of smallest position reads finished rows only, and the
+// cooperative launch keeps its warp resident.  Polls are bounded by the context's wait limit.
+// The row's entries, its update pairs and the pivots of up to 32 L entries are fetched at once, so
+// a row costs one L2 round trip after its last input appears.  The finished row also goes straight
+// into the level-sorted storage of the sweeps (no separate scatter pass).
+constexpr unsigned long long kPending = 0x7FF4B0F5B0F5B0F5ull;   // signalling NaN
+
+__device__ __forceinline__ double not_pending(double v) {
+    return (unsigned long long)__double_as_longlong(v) == kPending ? __longlong_as_double(0x7FF8000000000000ll) : v;
+}
+
+// v = *p once it is not pending; false if the wait gave up.
+__device__ __forceinline__ bool poll_value(const double *p, double &v, long long lim, const DevStatus *ds) {
+    unsigned long long b;
+    long long it = 0;
+    while (true) {
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(p) : "memory");
+        if (b != kPending) break;
+        if (++it > lim || ((it & 31) == 0 && ld_relaxed_i32(&ds->err) != 0)) return false;
+        __nanosleep(20);
+    }
+    v = __longlong_as_double((long long)b);
+    return true;
+}
+
+__global__ void fill_pending_kernel(size_t len, double *__restrict__ x) {
+    const double s = __longlong_as_double((long long)kPending);
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < len; e += (size_t)gridDim.x * blockDim.x)
+        reinterpret_cast<unsigned long long *>(x)[e] = (unsigned long long)__double_as_longlong(s);
+}
+
+struct FactorDfArgs {
+    int n, max_row;
+    const int *rows, *rp, *ci, *diag, *pp, *pdst, *psrc;
+    const double *vals;   // A's values
+    const int *fsrc;      // source entry per pattern entry (null: the same position)
+    double *fv;
+    SweepStore out;
+    DevStatus *ds;
+};
+
+__global__ void __launch_bounds__(256) factor_df_kernel(FactorDfArgs a) {
+    extern __shared__ double df_rows[];
+    const int lane = threadIdx.x & 31;
+    const int wpb = blockDim.x >> 5;
+    double *w = df_rows + (size_t)(threadIdx.x >> 5) * a.max_row;
+    const int gw = blockIdx.x * wpb + (threadIdx.x >> 5);
+    const int nw = gridDim.x * wpb;
+    const long long lim = a.ds->wait_limit > 0 ? a.ds->wait_limit : kSpinLimit;
+    bool ok = true;
+    for (int q = gw; q < a.n; q += nw) {
+        const int i = __ldg(a.rows + q);
+        const int rs = __ldg(a.rp + i), re = __ldg(a.rp + i + 1), di = __ldg(a.diag + i);
+        int p0 = __ldg(a.pp + rs);
+        const int pend = __ldg(a.pp + di);
+        int cb = p0, d = 0;
+        double v = 0.0;
+        for (int e = rs + lane; e < re; e += 32) w[e - rs] = __ldg(a.vals + (a.fsrc ? __ldg(a.fsrc + e) : e));
+        if (cb + lane < pend) {
+            d = __ldg(a.pdst + cb + lane) - rs;
+            ok = poll_value(a.fv + __ldg(a.psrc + cb + lane), v, lim, a.ds);
+        }
+        for (int eb = rs; eb < di; eb += 32) {
+            double piv = 1.0;
+            int p1 = 0;
+            if (eb + lane < di) {
+                const int k = __ldg(a.ci + eb + lane);
+                p1 = __ldg(a.pp + eb + lane + 1);
+                ok = ok && poll_value(a.fv + __ldg(a.diag + k), piv, lim, a.ds);
+                if (ok && piv == 0.0) {
+                    if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = k;
+                }
+            }
+            __syncwarp();
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const int cnt = min(32, di - eb);
+            for (int u = 0; u < cnt; u++) {
+                const double pv = __shfl_sync(0xffffffffu, piv, u);
+                const int p1u = __shfl_sync(0xffffffffu, p1, u);
+                const double lik = w[eb + u - rs] / pv;
+                __syncwarp();
+                if (lane == 0) w[eb + u - rs] = lik;
+                while (true) {
+                    if (cb + lane >= p0 && cb + lane < p1u) w[d] -= lik * v;
+                    if (p1u <= cb + 32) break;
+                    cb += 32;
+                    if (cb + lane < pend) {
+                        d = __ldg(a.pdst + cb + lane) - rs;
+                        ok = ok && poll_value(a.fv + __ldg(a.psrc + cb + lane), v, lim, a.ds);
+                    }
+                }
+                p0 = p1u;
+                __syncwarp();
+            }
+        }
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (!ok) atomicCAS(&a.ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
+            return;
+        }
+        __syncwarp();
+        for (int e = rs + lane; e < re; e += 32) {
+            const double x = not_pending(w[e - rs]);
+            __stcg(a.fv + e, x);
+            if (e == di && x == 0.0) {
+                if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = i;
+            }
+            sweep_put(a.out, e, x);
+        }
+        __syncwarp();
     }
 }
 
@@ -946,6 +1128,7 @@ bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const dou
         return set_error(ctx, BPF_ERR_NOT_SUPPORTED,
                          "reordered preconditioner: %d right-hand sides exceed the %d-column scratch "
                          "reserved for it", p, P->zcols);
+    if (P->col) return trsv_col_rowmajor(ctx, P, p, X, Y, gate);
     if (P->fdtype == BPF_F32)
         return trsv2_dispatch<float, false, false>(ctx, P->lower, P->upper, p, X, Y, gate, P->perm, P->zbuf,
                                                    P->sf_flags, ++P->sf_epoch);
@@ -956,6 +1139,10 @@ bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const dou
 bpf_status prec_reserve_z(bpf_ctx *ctx, bpf_prec *P, int p) {
     if (!P->perm || p <= P->zcols) return BPF_SUCCESS;
     const int cols = std::min(std::max(p, 1), 256);
+    if (P->col) {   // the column solves need no scratch: only the width is kept
+        P->zcols = cols;
+        return BPF_SUCCESS;
+    }
     double *z = nullptr;
     BPF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     BPF_CUDA(ctx, cudaMalloc((void **)&z, sizeof(double) * (size_t)P->n * cols));
@@ -982,6 +1169,43 @@ bpf_status prec_load_values(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     scatter_map_kernel<<<blocks, 256, 0, ctx->stream>>>(P->nnz, vals, P->amap, P->fv);
     BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;
+}
+
+// Data-flow ILU(0): rows of up to max_row entries in shared memory, eight warps per CTA while
+// they fit (2,800 entries), else as many as do; longer rows use the level kernel.
+static bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const double *vals, bool *taken) {
+    *taken = false;
+    int wpb = 8;
+    const size_t row_bytes = sizeof(double) * (size_t)P->max_row;
+    while (wpb > 1 && wpb * row_bytes > (size_t)ctx->max_smem_optin) wpb >>= 1;
+    if (wpb * row_bytes > (size_t)ctx->max_smem_optin) return BPF_SUCCESS;
+    const size_t smem = wpb * row_bytes;
+    BPF_CUDA(ctx, cudaFuncSetAttribute(factor_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int grid = 1;
+    BPF_TRY(coop_grid(ctx, factor_df_kernel, 32 * wpb, smem, ceil_div(P->n, wpb), &grid));
+    FactorDfArgs a{P->n, P->max_row, P->lower.rows, P->rp, P->ci, P->diag, P->pp, P->pdst, P->psrc, vals, P->fsrc,
+                   P->fv, sweep_store(P), ctx->dstat};
+    void *args[] = {&a};
+    KScope ks(ctx, BPF_KC_FACTOR, 44.0 * P->nnz + 12.0 * (P->n + 1) + 8.0 * P->npairs, 2.0 * P->npairs);
+    const int fb = std::max(1, std::min(ceil_div(P->nnz, 256), ctx->num_sms * 8));
+    fill_pending_kernel<<<fb, 256, 0, ctx->stream>>>((size_t)P->nnz, P->fv);
+    BPF_LAUNCHED(ctx);
+    BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)factor_df_kernel, dim3(grid), dim3(32 * wpb), args, smem,
+                                              ctx->stream));
+    BPF_LAUNCHED(ctx);
+    *taken = true;
+    return BPF_SUCCESS;
+}
+
+bpf_status prec_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
+    if (P->kind == PREC_ILU0 && P->n > 0) {
+        bool taken = false;
+        BPF_TRY(factor_df(ctx, P, vals, &taken));
+        if (taken) return BPF_SUCCESS;
+    }
+    BPF_TRY(prec_load_values(ctx, P, vals));
+    BPF_TRY(factor_numeric(ctx, P));
+    return sweep_scatter(ctx, P);
 }
 
 bpf_status lu_solve_push_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, double *Y) {

@@ -92,7 +92,16 @@ using PairVec = std::vector<int, NoInitAlloc<int>>;
 // false (and empty outputs) when the pair count exceeds INT_MAX
 bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
                  std::vector<int> &pp, PairVec &pdst, PairVec &psrc);
-bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d);
+// A sweep's factor as the byte stream of the column solves (trsv_col.cu).
+struct TriStream {
+    std::vector<unsigned char> bytes;
+    std::vector<int> coff, cslab, head;   // per chunk: byte offset, first slab; slab headers
+    int diag = 0, nstage = 0;
+};
+void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<int> &pos, TriStream &out,
+                   std::vector<int> &tpos);
+// values = false: the schedule only (the values are kept elsewhere)
+bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d, bool values = true);
 void tri_free(TriDev &d);
 bpf_status tri_scatter(bpf_ctx *ctx, const TriDev &d, const double *fv);
 
@@ -107,6 +116,10 @@ struct bpf_prec {
     // pattern (0-based device copies) and factor values in pattern order
     int *rp = nullptr, *ci = nullptr, *diag = nullptr;
     double *fv = nullptr;
+    // ILU(0) data-flow factorization: the longest row, and the source entry of A per pattern entry
+    // (null: the same position)
+    int max_row = 0;
+    int *fsrc = nullptr;
     int *pp = nullptr, *pdst = nullptr, *psrc = nullptr;
     long long npairs = 0;
     bpf::TriDev lower;   // forward solve (L unit for ILU0; L for IC0)
@@ -134,6 +147,21 @@ struct bpf_prec {
     std::vector<int> perm_host;
     double *zbuf = nullptr;
     int zcols = 0;
+    // Where a factor entry goes in each sweep's storage, per pattern entry: its value's index (the
+    // level-sorted val, or the stream in units of the factor type), -1 nowhere, -2 - index its
+    // reciprocal (the level-sorted dinv, or the stream).
+    int *tpos[2] = {nullptr, nullptr};
+    // Column solves (trsv_col.cu): each sweep's factor as a byte stream in place of the level-sorted
+    // storage; pos0[r] / pos1[r] = forward / backward position of the block's row r, pos01[q] =
+    // forward position of the row at backward position q.
+    bool col = false;
+    struct ColStream {
+        unsigned char *bytes = nullptr;
+        int *coff = nullptr, *cslab = nullptr, *head = nullptr;
+        int nchunk = 0, nslab = 0, nstage = 0, diag = 0;
+        size_t len = 0;
+    } cs[2];
+    int *pos0 = nullptr, *pos01 = nullptr, *pos1 = nullptr;
     // Sync-free triangular solves: one ready word per factor row, 2e when the forward sweep of
     // launch e has produced the row and 2e + 1 after the backward sweep (monotone across
     // launches, so nothing is reset between them).
@@ -148,10 +176,22 @@ struct bpf_prec {
 
 namespace bpf {
 bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
-                      const std::vector<int> &ci, const std::vector<int> &diag, bpf_prec **out);
+                      const std::vector<int> &ci, const std::vector<int> &diag, int fdtype,
+                      const std::vector<int> &perm, bpf_prec **out);
 bpf_status csr_pattern_to_host(bpf_ctx *ctx, const bpf_csr_desc *A, std::vector<int> &rp,
                                std::vector<int> &ci, bool need_diag, std::vector<int> *diag);
 bpf_status factor_numeric(bpf_ctx *ctx, bpf_prec *P);
+// The whole numeric step from A's values (device, A's entry order): values in, factors in fv and
+// in the level-sorted storage of both sweeps.
+bpf_status prec_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals);
+// Column-per-CTA triangular solves (trsv_col.cu) of a preconditioner kept for them (P->col):
+// column-major blocks (Y may be X with the same leading dimension), or row-major ones.
+bool trsv_col_fits(const bpf_ctx *ctx, int n, int fdtype);
+int trsv_col_ring(const bpf_ctx *ctx, int n, int fdtype);
+bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, size_t ldx, double *Y, size_t ldy,
+                    const int *gate = nullptr);
+bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y,
+                             const int *gate = nullptr);
 bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X,
                                double *Y, const int *gate = nullptr);
 // Reordered preconditioners: make the factor-ordered scratch hold p columns (allocates when it

@@ -313,9 +313,8 @@ bpf_status bpf_rf_analyze(bpf_ctx *ctx, const bpf_csr_desc *A, int ordering, dou
         bpf_rf_destroy(rf);
         return s;
     };
-    bpf_status s = prec_setup(ctx, PREC_LU, n, Frp, Fci, Fdiag, &rf->lu);
+    bpf_status s = prec_setup(ctx, PREC_LU, n, Frp, Fci, Fdiag, BPF_F64, {}, &rf->lu);
     if (s != BPF_SUCCESS) return fail(s);
-    rf->lu->fdtype = BPF_F64;
     cudaError_t e = cudaMalloc((void **)&rf->Pd, sizeof(int) * std::max(n, 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&rf->Qd, sizeof(int) * std::max(n, 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&rf->amap, sizeof(int) * std::max(nnz, 1));

@@ -18,6 +18,7 @@
 
 #include "bpf_internal.cuh"
 #include "dense.cuh"
+#include "bulk.cuh"
 #include "small.cuh"
 
 namespace bpf {
@@ -28,46 +29,7 @@ __device__ __forceinline__ unsigned long long small_globaltimer_ns() {
     return t;
 }
 
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
 
-// --- mbarrier + bulk async copy (global -> shared) ---------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned parity) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// Bounded wait on a phase of an mbarrier (~2^21 polls); false on timeout.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity) {
-    for (long long it = 0; it < kSpinLimit; it++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (it > 64) __nanosleep(32);
-    }
-    return false;
-}
 
 // Inverse of an upper-triangular p x p matrix U (row stride ldu) into X (row stride ldx), both
 // in shared memory (or X in global memory).  Column c of X = U^{-1} is computed by back

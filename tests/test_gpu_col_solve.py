@@ -1,0 +1,127 @@
+"""Column-per-CTA triangular solves and the data-flow ILU(0) against the CPU oracle, at the sizes
+where their layouts change: one row, warp and chunk remainders, long rows that span several parts
+of a level, the last row count kept for the column solves and the first one past it, both factor
+types, blocks solved in place and blocks that overlap."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import oracle as O
+from conftest import spd_from
+
+pytestmark = pytest.mark.gpu
+
+FP64_ROWS = 24_831   # 227 KB - 1 KB less two 16 KB chunks, 8 bytes a row and one more
+
+
+@pytest.fixture(scope="module")
+def bpf():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import blockpowerflow_b200 as bpf
+
+    return bpf
+
+
+def _random(n, per_row, seed):
+    """Diagonally dominant, about per_row off-diagonal entries a row."""
+    rng = np.random.default_rng(seed)
+    k = per_row * n
+    A = sp.coo_matrix((rng.standard_normal(k), (rng.integers(0, n, k), rng.integers(0, n, k))), shape=(n, n)).tocsr()
+    A = A - sp.diags(A.diagonal())
+    return (A + sp.diags(1.0 + np.asarray(abs(A).sum(axis=1)).ravel())).tocsr()
+
+
+def _arrow(n):
+    """Dense first and last rows and columns: rows of n entries, single-row levels."""
+    A = sp.lil_matrix((n, n))
+    A.setdiag(4.0 * n)
+    A[0, :] = A[n - 1, :] = 1.0
+    A[:, 0] = A[:, n - 1] = 1.0
+    A.setdiag(4.0 * n)
+    return A.tocsr()
+
+
+def _block(X):
+    import torch
+
+    return torch.as_tensor(np.asfortranarray(X), device="cuda").t().contiguous().t()
+
+
+@pytest.mark.parametrize("dtype,rtol", [("float64", 1e-12), ("float32", 1e-4)])
+@pytest.mark.parametrize("n,per_row,p", [(1, 0, 1), (2, 1, 3), (31, 3, 2), (32, 3, 1), (33, 3, 5), (700, 40, 3),
+                                         (5000, 4, 17)])
+def test_ilu0_column_solve_sizes(bpf, n, per_row, p, dtype, rtol):
+    A = _random(n, per_row, n)
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), p, dtype)
+    F = O.ilu0(A)
+    np.testing.assert_allclose(P.P.nzVal.cpu().numpy(), F.data, rtol=1e-11, atol=1e-11 * np.abs(F.data).max())
+    X = np.random.default_rng(1).standard_normal((n, p))
+    Y = P.ldiv(_block(X)).cpu().numpy()
+    ref = O.prec_apply(1, F, X)
+    assert np.linalg.norm(Y - ref) <= rtol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("dtype,rtol", [("float64", 1e-12), ("float32", 1e-4)])
+@pytest.mark.parametrize("n", [200, 1500])
+def test_long_rows_span_several_parts(bpf, n, dtype, rtol):
+    A = _arrow(n)
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), 2, dtype)
+    X = np.random.default_rng(2).standard_normal((n, 2))
+    ref = O.prec_apply(1, O.ilu0(A), X)
+    Y = P.ldiv(_block(X)).cpu().numpy()
+    assert np.linalg.norm(Y - ref) <= rtol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n", [FP64_ROWS, FP64_ROWS + 1])
+def test_last_row_count_of_the_column_solve(bpf, n):
+    A = _random(n, 3, 7)
+    for p in (1, 20):
+        P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), p)
+        X = np.random.default_rng(3).standard_normal((n, p))
+        ref = O.prec_apply(1, O.ilu0(A), X)
+        Y = P.ldiv(_block(X)).cpu().numpy()
+        assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+def test_ic0_column_solve(bpf, case300):
+    A, _ = case300
+    S = spd_from(A)
+    for dtype, rtol in (("float64", 1e-12), ("float32", 1e-4)):
+        P = bpf.ic0(bpf.CuSparseMatrixCSR.from_scipy(S), 6, dtype)
+        X = np.random.default_rng(4).standard_normal((S.shape[0], 6))
+        ref = O.prec_apply(2, O.ic0(S), X)
+        Y = P.ldiv(_block(X)).cpu().numpy()
+        assert np.linalg.norm(Y - ref) <= rtol * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("ordering", ["natural", "AMD", "RCM"])
+def test_in_place_and_overlapping_blocks(bpf, ordering):
+    A = bpf.grid.synthetic_jacobian(200)
+    n = A.shape[0]
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), 4, ordering=ordering)
+    X = np.random.default_rng(5).standard_normal((n, 5))
+    ref = P.ldiv(_block(X)).cpu().numpy()
+    W = _block(X)
+    bpf.ldiv_(W, P, W)
+    np.testing.assert_array_equal(W.cpu().numpy(), ref)
+    W = _block(X)
+    bpf.ldiv_(W[:, 1:], P, W[:, :4])   # the output is the input shifted by a column
+    np.testing.assert_array_equal(W[:, 1:].cpu().numpy(), ref[:, :4])
+    W = _block(np.vstack([X, X]))
+    bpf.ldiv_(W[3:n + 3, :], P, W[:n, :])   # and by three rows
+    np.testing.assert_array_equal(W[3:n + 3, :].cpu().numpy(), ref)
+
+
+def test_zero_pivot_is_reported_and_the_next_factorization_runs(bpf):
+    pat = _random(300, 3, 9)
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(pat)
+    P = bpf.ilu0(Ad, 1)
+    vals = Ad.nzVal.clone()
+    vals[pat.indptr[17]:pat.indptr[18]] = 0.0   # a zero row keeps its pivot zero
+    with pytest.raises(bpf.SingularException):
+        P.refactor(vals)
+    P.refactor(Ad.nzVal)
+    np.testing.assert_allclose(P.P.nzVal.cpu().numpy(), O.ilu0(pat).data, rtol=1e-11)
