@@ -141,7 +141,8 @@ bpf_status csr_pattern_to_host(bpf_ctx *ctx, const bpf_csr_desc *A, std::vector<
 
 // Analyse a 0-based host pattern (sorted rows, diagonal present) and upload everything the
 // numeric factorization and the triangular solves need.  P->fv is allocated, not filled.
-// kind PREC_ILU0 / PREC_LU: unit L + U on the pattern; PREC_IC0: L and L' (lower part).
+// kind PREC_ILU0: unit L + U on the pattern; PREC_IC0: L and L' (lower part); PREC_LU: L + U without
+// stored update pairs (the patterns lu_setup does not take).
 bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
                       const std::vector<int> &ci, const std::vector<int> &diag, int fdtype,
                       const std::vector<int> &perm, bpf_prec **out) {
@@ -166,8 +167,8 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     }
     if (P->col) {
         const int nring = trsv_col_ring(ctx, n, fdtype);
-        tri_to_stream(lo, fdtype, nring, 0, pos0, cs[0], tpos[0]);
-        tri_to_stream(up, fdtype, nring, (int)cs[0].coff.size() - 1, pos1, cs[1], tpos[1]);
+        tri_to_stream(lo, fdtype, nring, 0, n, false, pos0, cs[0], tpos[0]);
+        tri_to_stream(up, fdtype, nring, (int)cs[0].coff.size() - 1, n, false, pos1, cs[1], tpos[1]);
         for (int q = 0; q < n; q++) pos01[q] = pos0[up.rows[q]];
         if (!perm.empty()) {   // positions of the block's rows: factor row i is row perm[i]
             std::vector<int> b0(n), b1(n);
@@ -187,10 +188,15 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     }
     std::vector<int> pp;
     PairVec pdst, psrc;
-    const char *env_pl = getenv("BPF_LU_PAIRLESS");
-    const bool force_pairless = kind == PREC_LU && env_pl && atoi(env_pl) != 0;
-    const bool pairs_ok = !force_pairless && build_pairs(n, rp.data(), ci.data(), diag.data(), ic, pp, pdst, psrc);
-    P->npairs = (long long)pdst.size();
+    std::vector<long long> goff;
+    PairVec gsrc;
+    for (int i = 0; i < n; i++) P->max_row = std::max(P->max_row, rp[i + 1] - rp[i]);
+    const bool pairs_ok = kind != PREC_LU && (kind != PREC_ILU0 || P->max_row > kGatherRow
+                                                  ? build_pairs(n, rp.data(), ci.data(), diag.data(), ic, pp, pdst, psrc)
+                                                  : true);
+    long long gathered = 0;
+    if (kind == PREC_ILU0) gathered = build_gather(n, rp, ci, diag, {}, goff, gsrc);
+    P->npairs = std::max((long long)pdst.size(), gathered);
     auto fail = [&](bpf_status s) {
         cudaStreamSynchronize(ctx->stream);
         bpf_prec_destroy(P);
@@ -200,7 +206,7 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
         return fail(set_error(ctx, BPF_ERR_NOT_SUPPORTED,
                               "factorization update pairs exceed 2^31 - 1 (pattern of %d entries too dense)", nnz));
     if (!pairs_ok) {
-        // the LU refactorization finds each L entry's updates by a search in its row instead
+        // this form of the LU refactorization finds each L entry's updates by a search in its row
         P->pairless = true;
         long long upd = 0;
         for (int i = 0; i < n; i++)
@@ -252,8 +258,12 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     }
     up_i(&P->tpos[0], tpos[0]);
     up_i(&P->tpos[1], tpos[1]);
-    if (kind == PREC_ILU0)
-        for (int i = 0; i < n; i++) P->max_row = std::max(P->max_row, rp[i + 1] - rp[i]);
+    up_i(&P->gsrc, gsrc);
+    if (e == cudaSuccess && !goff.empty()) {
+        e = cudaMalloc((void **)&P->goff, sizeof(long long) * goff.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(P->goff, goff.data(), sizeof(long long) * goff.size(), cudaMemcpyHostToDevice, ctx->stream);
+    }
     if (kind == PREC_LU && n > 0) {
         // column-step levels: step k depends on the steps j < k with L(k, j) != 0 (they update
         // row k) or U(j, k) != 0 (they update column k)
@@ -284,7 +294,7 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
         P->cl_max_level = mx;
         up_i(&P->cl_lev_ptr, lptr);
         up_i(&P->cl_ent, ent);
-        if (P->pairless) {
+        {
             std::vector<int> erow(ent.size());
             std::vector<int> rowof(nnz > 0 ? nnz : 1);
             for (int i = 0; i < n; i++)
@@ -700,6 +710,8 @@ bpf_status bpf_prec_destroy(bpf_prec *P) {
     cudaFree(P->perm);
     cudaFree(P->amap);
     cudaFree(P->fsrc);
+    cudaFree(P->goff);
+    cudaFree(P->gsrc);
     cudaFree(P->pos0);
     cudaFree(P->pos01);
     cudaFree(P->pos1);
@@ -712,6 +724,11 @@ bpf_status bpf_prec_destroy(bpf_prec *P) {
     }
     cudaFree(P->zbuf);
     cudaFree(P->sf_flags);
+    cudaFree(P->fend);
+    cudaFree(P->forder);
+    cudaFree(P->tail_S);
+    cudaFree(P->tail_F);
+    cudaFree(P->tail_inv);
     cudaFree(P->cl_lev_ptr);
     cudaFree(P->cl_ent);
     cudaFree(P->cl_row);

@@ -29,6 +29,7 @@
 #include <cstdlib>
 
 #include "bpf_internal.cuh"
+#include "pending.cuh"
 #include "prec.cuh"
 
 namespace bpf {
@@ -179,29 +180,18 @@ bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
             for (int k = rp[i]; k < rp[i + 1]; k++) pos[ci[k]] = -1;
         }
     };
-    // large patterns (the LU patterns of the refactorization) on several host threads, each with
-    // its own position array, taking blocks of 64 rows from a shared counter
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int nthreads = nnz >= 200000 ? (int)std::min(16u, std::max(1u, hw)) : 1;
+    // large patterns on several host threads, each with its own position array, taking blocks of 64 rows
+    // from a shared counter
     auto run = [&](int pass) {
         std::atomic<int> next(0);
-        auto work = [&]() {
+        run_threads(nnz >= 200000, [&]() {
             std::vector<int> pos(n, -1);
             for (;;) {
                 const int b = next.fetch_add(64);
                 if (b >= n) break;
                 rows(pass, b, std::min(n, b + 64), pos);
             }
-        };
-        std::vector<std::thread> pool;
-        try {
-            for (int t = 1; t < nthreads; t++) pool.emplace_back(work);
-        } catch (const std::system_error &) {
-            // fewer helpers than asked (a thread limit): the calling thread still takes every
-            // block the helpers do not
-        }
-        work();
-        for (auto &th : pool) th.join();
+        });
     };
     run(0);
     long long total = 0;
@@ -219,6 +209,44 @@ bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
     psrc.resize(pp[nnz]);
     run(1);
     return true;
+}
+
+long long build_gather(int nrows, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &diag,
+                       const std::vector<char> &skip, std::vector<long long> &goff, PairVec &gsrc) {
+    goff.assign(std::max(nrows, 1), -1);
+    long long total = 0;
+    for (int i = 0; i < nrows; i++) {
+        const int len = rp[i + 1] - rp[i];
+        if (len > kGatherRow || (!skip.empty() && skip[i])) continue;
+        goff[i] = total;
+        total += (long long)len * (diag[i] - rp[i]);
+    }
+    gsrc.resize(std::max<long long>(total, 1));
+    std::atomic<int> next(0);
+    std::atomic<long long> updates(0);
+    run_threads(total >= 400000, [&]() {
+        long long found = 0;
+        for (;;) {
+            const int b = next.fetch_add(256);
+            if (b >= nrows) break;
+            for (int i = b; i < std::min(nrows, b + 256); i++) {
+                if (goff[i] < 0) continue;
+                int *g = gsrc.data() + goff[i];
+                for (int e = rp[i]; e < diag[i]; e++) {   // merge the row's columns with U's row k
+                    int j = diag[ci[e]] + 1;
+                    const int end = rp[ci[e] + 1];
+                    for (int t = rp[i]; t < rp[i + 1]; t++, g++) {
+                        while (j < end && ci[j] < ci[t]) j++;
+                        const bool hit = j < end && ci[j] == ci[t];
+                        *g = hit ? j : -1;
+                        found += hit;
+                    }
+                }
+            }
+        }
+        updates += found;
+    });
+    return updates;
 }
 
 // ------------------------------------------------------------------------------------
@@ -299,36 +327,7 @@ bpf_status tri_scatter(bpf_ctx *ctx, const TriDev &d, const double *fv) {
     return BPF_SUCCESS;
 }
 
-// The storage of the two sweeps that a factor entry goes to (bpf_prec::tpos), CSR or stream.
-struct SweepStore {
-    const int *tpos[2];
-    double *val[2], *dinv[2];      // level-sorted storage, FP64 and FP32
-    float *valf[2], *dinvf[2];
-    unsigned char *stream[2];      // or the streams (column solves), of FP32 values if f32
-    int col, f32;
-};
-
-__device__ __forceinline__ void sweep_put(const SweepStore &s, int e, double x) {
-#pragma unroll
-    for (int w = 0; w < 2; w++) {
-        const int t = s.tpos[w] ? __ldg(s.tpos[w] + e) : -1;
-        if (t == -1) continue;
-        const double v = t >= 0 ? x : 1.0 / x;
-        const int k = t >= 0 ? t : -2 - t;
-        if (s.col) {
-            if (s.f32) reinterpret_cast<float *>(s.stream[w])[k] = (float)v;
-            else reinterpret_cast<double *>(s.stream[w])[k] = v;
-        } else if (t >= 0) {
-            s.val[w][k] = v;
-            s.valf[w][k] = (float)v;
-        } else {
-            s.dinv[w][k] = v;
-            s.dinvf[w][k] = (float)v;
-        }
-    }
-}
-
-static SweepStore sweep_store(const bpf_prec *P) {
+SweepStore sweep_store(const bpf_prec *P) {
     SweepStore s;
     const TriDev *t[2] = {&P->lower, &P->upper};
     for (int w = 0; w < 2; w++) {
@@ -446,175 +445,269 @@ __global__ void __launch_bounds__(256) factor_coop_kernel(FactorArgs a) {
     }
 }
 
-// ILU(0) as a data flow: a warp per row in level order, the row held in shared memory; a row
-// waits only for the values it reads, and a value is its own ready mark.
+// ILU(0) (and LU on a fill pattern) as a data flow: a warp per row in level order, the row held in
+// shared memory; a row waits only for the values it reads, which are their own ready marks
+// (pending.cuh).
 //
 // Bound: the chain of dependency levels.  A grid barrier per level cost 5-15 us a level; refactor()
 // of the 9,000-bus pattern took 231 us in natural order (14 levels), 427 us in minimum-degree order
 // (26), 4.7 ms in reverse Cuthill-McKee order (456), and takes 62, 94 and 1,285 us this way (70,000
-// buses: 381 -> 126 us).  Here
-// every factor value starts as a signalling-NaN bit pattern that no arithmetic can produce (results
-// of operations are quiet NaNs, and stores check), a reader polls the value itself until it is
-// something else, and a producer needs no fence: 64-bit accesses are single, and no value vouches for
-// another.  No deadlock: the unfinished row of smallest position reads finished rows only, and the
-// cooperative launch keeps its warp resident.  Polls are bounded by the context's wait limit.
-// The row's entries, its update pairs and the pivots of up to 32 L entries are fetched at once, so
-// a row costs one L2 round trip after its last input appears.  The finished row also goes straight
-// into the level-sorted storage of the sweeps (no separate scatter pass).
-constexpr unsigned long long kPending = 0x7FF4B0F5B0F5B0F5ull;   // signalling NaN
-
-__device__ __forceinline__ double not_pending(double v) {
-    return (unsigned long long)__double_as_longlong(v) == kPending ? __longlong_as_double(0x7FF8000000000000ll) : v;
-}
-
-// v = *p once it is not pending; false if the wait gave up.
-__device__ __forceinline__ bool poll_value(const double *p, double &v, long long lim, const DevStatus *ds) {
-    unsigned long long b;
-    long long it = 0;
-    while (true) {
-        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(b) : "l"(p) : "memory");
-        if (b != kPending) break;
-        if (++it > lim || ((it & 31) == 0 && ld_relaxed_i32(&ds->err) != 0)) return false;
-        __nanosleep(20);
-    }
-    v = __longlong_as_double((long long)b);
-    return true;
-}
-
+// buses: 381 -> 126 us).  No deadlock: the unfinished row of smallest position reads finished rows
+// only, and the cooperative launch keeps its warp resident.  Polls are bounded by the context's wait
+// limit.
+//
+// A row of up to 256 entries lives in the warp's registers (entry lane + 32 r), and each of its L
+// entries k comes with a list, over the row's entries, of the U entry of row k that updates it: the
+// step is a broadcast, a quotient and one FMA per register, with the coming entries' values already
+// loaded; only what is still pending is polled, all of a step at once, so a row's result follows its
+// last input by one L2 round trip and ~100 cycles per remaining entry.  (Rows in shared memory updated
+// through pair lists took ~700 cycles per entry: 22 levels of a 300-bus LU, 85-147 us.)  Longer rows
+// still go that way.  The finished row also goes straight into the storage of the sweeps (no separate
+// scatter pass).
 __global__ void fill_pending_kernel(size_t len, double *__restrict__ x) {
-    const double s = __longlong_as_double((long long)kPending);
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < len; e += (size_t)gridDim.x * blockDim.x)
-        reinterpret_cast<unsigned long long *>(x)[e] = (unsigned long long)__double_as_longlong(s);
+        x[e] = pending_value();
 }
 
 struct FactorDfArgs {
-    int n, max_row;
-    const int *rows, *rp, *ci, *diag, *pp, *pdst, *psrc;
-    const double *vals;   // A's values
-    const int *fsrc;      // source entry per pattern entry (null: the same position)
+    int n, max_row;          // rows to factor; longest row that goes through shared memory
+    const int *rows, *rp, *ci, *diag, *pp, *pdst, *psrc, *gsrc;
+    const long long *goff;
+    const double *vals;      // A's values
+    const int *fsrc;         // source entry per pattern entry (null: the same position; -1: zero)
     double *fv;
     SweepStore out;
     DevStatus *ds;
 };
 
+__device__ __forceinline__ double df_source(const FactorDfArgs &a, int e) {
+    const int src = a.fsrc ? __ldg(a.fsrc + e) : e;
+    return src < 0 ? 0.0 : __ldg(a.vals + src);
+}
+
+// Store of the row's entry at position e (index t of the row, nl of it before the diagonal).
+__device__ __forceinline__ void df_store(const FactorDfArgs &a, int i, int e, bool is_diag, double v) {
+    const double x = not_pending(v);
+    __stcg(a.fv + e, x);
+    if (is_diag && x == 0.0) {
+        if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = i;
+    }
+    sweep_put(a.out, e, x);
+}
+
+// A row of len <= 32 R entries in registers, nl of them before the diagonal; E entries' updates are
+// loaded at once, and the next E are under way.
+template <int R, int E>
+__device__ __forceinline__ bool df_row(const FactorDfArgs &a, int i, int rs, int len, int nl, const int *gs, int lane,
+                                       long long lim) {
+    double w[R], v[E][R];
+    int id[E][R], idn[E][R];
+    auto indices = [&](int eb, int (&x)[E][R]) {
+#pragma unroll
+        for (int u = 0; u < E; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int t = lane + 32 * r;
+                x[u][r] = eb + u < nl && t < len ? __ldg(gs + (size_t)(eb + u) * len + t) : -1;
+            }
+    };
+    auto values = [&](const int (&x)[E][R], double (&y)[E][R]) {
+#pragma unroll
+        for (int u = 0; u < E; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++) y[u][r] = x[u][r] >= 0 ? ld_value(a.fv + x[u][r]) : 0.0;
+    };
+    indices(0, id);
+    int dpos = 0;          // of L entry lane, + 32, ...: the pivot's position and its value
+    double piv = 1.0;
+    auto pivots = [&](int eb) {
+        if (eb + lane < nl) {
+            dpos = __ldg(a.diag + __ldg(a.ci + rs + eb + lane));
+            piv = ld_value(a.fv + dpos);
+        }
+    };
+    pivots(0);
+#pragma unroll
+    for (int r = 0; r < R; r++) w[r] = lane + 32 * r < len ? df_source(a, rs + lane + 32 * r) : 0.0;
+    values(id, v);
+    indices(E, idn);
+    for (int eb = 0; eb < nl; eb += E) {
+        if (eb > 0 && (eb & 31) == 0) pivots(eb);
+        double vn[E][R];
+        int idnn[E][R];
+        values(idn, vn);
+        indices(eb + 2 * E, idnn);
+#pragma unroll
+        for (int u = 0; u < E; u++) {
+            const int e = eb + u;
+            if (e < nl) {
+                double pv = __shfl_sync(0xffffffffu, piv, e & 31);
+                const int dp = __shfl_sync(0xffffffffu, dpos, e & 31);
+                for (long long it = 0;; it++) {
+                    bool pend = is_pending(pv);
+#pragma unroll
+                    for (int r = 0; r < R; r++) pend = pend || is_pending(v[u][r]);
+                    if (!__any_sync(0xffffffffu, pend)) break;
+                    bool ok = it <= lim;
+                    if ((it & 31) == 31) ok = ok && ld_relaxed_i32(&a.ds->err) == 0;
+                    if (!__all_sync(0xffffffffu, ok)) return false;
+                    if (is_pending(pv)) pv = ld_value(a.fv + dp);
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        if (is_pending(v[u][r])) v[u][r] = ld_value(a.fv + id[u][r]);
+                }
+                if (pv == 0.0 && lane == 0) {
+                    if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = __ldg(a.ci + rs + e);
+                }
+                double we = w[0];
+#pragma unroll
+                for (int r = 1; r < R; r++)
+                    if (e >> 5 == r) we = w[r];
+                const double lik = __shfl_sync(0xffffffffu, we, e & 31) / pv;
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    if (lane + 32 * r == e) w[r] = lik;
+                    if (id[u][r] >= 0) w[r] -= lik * v[u][r];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < E; u++)
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                v[u][r] = vn[u][r];
+                id[u][r] = idn[u][r];
+                idn[u][r] = idnn[u][r];
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int t = lane + 32 * r;
+        if (t < len) df_store(a, i, rs + t, t == nl, w[r]);
+    }
+    return true;
+}
+
+// Four update pairs of a lane: destination in the row, source position, and the source's value (to
+// be polled where it is still pending).
+struct PairBlock {
+    int d[4], s[4];
+    double v[4];
+    __device__ __forceinline__ void indices(const FactorDfArgs &a, int t0, int pend, int rs) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int t = t0 + 32 * c + (threadIdx.x & 31);
+            s[c] = -1;
+            d[c] = 0;
+            if (t < pend) {
+                d[c] = __ldg(a.pdst + t) - rs;
+                s[c] = __ldg(a.psrc + t);
+            }
+        }
+    }
+    __device__ __forceinline__ void values(const FactorDfArgs &a) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) v[c] = s[c] >= 0 ? ld_value(a.fv + s[c]) : 0.0;
+    }
+};
+
+// A row of any length in shared memory (w), updated through its pair lists.
+__device__ __noinline__ bool df_long_row(const FactorDfArgs &a, int i, double *w, long long lim) {
+    const int lane = threadIdx.x & 31;
+    const int rs = __ldg(a.rp + i), re = __ldg(a.rp + i + 1), di = __ldg(a.diag + i);
+    int p0 = __ldg(a.pp + rs);
+    const int pend = __ldg(a.pp + di);
+    // the row's update pairs in blocks of 128 (four a lane): the current block, the next one with its
+    // values under way, and the indices of the one after
+    int cb = p0;
+    PairBlock cur, nxt, idx;
+    cur.indices(a, cb, pend, rs);
+    nxt.indices(a, cb + 128, pend, rs);
+    idx.indices(a, cb + 256, pend, rs);
+    cur.values(a);
+    nxt.values(a);
+    bool ok = true;
+    for (int e = rs + lane; e < re; e += 32) w[e - rs] = df_source(a, e);
+    for (int eb = rs; eb < di; eb += 32) {
+        double piv = 1.0;
+        int p1 = 0;
+        if (eb + lane < di) {
+            const int k = __ldg(a.ci + eb + lane);
+            p1 = __ldg(a.pp + eb + lane + 1);
+            ok = ok && poll_value(a.fv + __ldg(a.diag + k), piv, lim, a.ds);
+            if (ok && piv == 0.0) {
+                if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = k;
+            }
+        }
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, ok)) return false;
+        const int cnt = min(32, di - eb);
+        for (int u = 0; u < cnt; u++) {
+            const double pv = __shfl_sync(0xffffffffu, piv, u);
+            const int p1u = __shfl_sync(0xffffffffu, p1, u);
+            const double lik = w[eb + u - rs] / pv;
+            __syncwarp();
+            if (lane == 0) w[eb + u - rs] = lik;
+            while (true) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int t = cb + 32 * c + lane;
+                    if (t >= p0 && t < p1u) {
+                        if (is_pending(cur.v[c])) ok = poll_value(a.fv + cur.s[c], cur.v[c], lim, a.ds) && ok;
+                        w[cur.d[c]] -= lik * cur.v[c];
+                    }
+                }
+                if (p1u <= cb + 128) break;
+                cb += 128;
+                cur = nxt;
+                nxt = idx;
+                nxt.values(a);
+                idx.indices(a, cb + 256, pend, rs);
+            }
+            p0 = p1u;
+            __syncwarp();
+        }
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    __syncwarp();
+    for (int e = rs + lane; e < re; e += 32) df_store(a, i, e, e == di, w[e - rs]);
+    __syncwarp();
+    return true;
+}
+
+// RMAX: rows of up to 32 RMAX entries (8: of any length); fewer registers leave more rows in flight.
+template <int RMAX>
 __global__ void __launch_bounds__(256) factor_df_kernel(FactorDfArgs a) {
     extern __shared__ double df_rows[];
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
-    double *w = df_rows + (size_t)(threadIdx.x >> 5) * a.max_row;
     const int gw = blockIdx.x * wpb + (threadIdx.x >> 5);
     const int nw = gridDim.x * wpb;
     const long long lim = a.ds->wait_limit > 0 ? a.ds->wait_limit : kSpinLimit;
-    bool ok = true;
     for (int q = gw; q < a.n; q += nw) {
         const int i = __ldg(a.rows + q);
-        const int rs = __ldg(a.rp + i), re = __ldg(a.rp + i + 1), di = __ldg(a.diag + i);
-        int p0 = __ldg(a.pp + rs);
-        const int pend = __ldg(a.pp + di);
-        int cb = p0, d = 0;
-        double v = 0.0;
-        for (int e = rs + lane; e < re; e += 32) w[e - rs] = __ldg(a.vals + (a.fsrc ? __ldg(a.fsrc + e) : e));
-        if (cb + lane < pend) {
-            d = __ldg(a.pdst + cb + lane) - rs;
-            ok = poll_value(a.fv + __ldg(a.psrc + cb + lane), v, lim, a.ds);
-        }
-        for (int eb = rs; eb < di; eb += 32) {
-            double piv = 1.0;
-            int p1 = 0;
-            if (eb + lane < di) {
-                const int k = __ldg(a.ci + eb + lane);
-                p1 = __ldg(a.pp + eb + lane + 1);
-                ok = ok && poll_value(a.fv + __ldg(a.diag + k), piv, lim, a.ds);
-                if (ok && piv == 0.0) {
-                    if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = k;
-                }
-            }
-            __syncwarp();
-            if (!__all_sync(0xffffffffu, ok)) break;
-            const int cnt = min(32, di - eb);
-            for (int u = 0; u < cnt; u++) {
-                const double pv = __shfl_sync(0xffffffffu, piv, u);
-                const int p1u = __shfl_sync(0xffffffffu, p1, u);
-                const double lik = w[eb + u - rs] / pv;
-                __syncwarp();
-                if (lane == 0) w[eb + u - rs] = lik;
-                while (true) {
-                    if (cb + lane >= p0 && cb + lane < p1u) w[d] -= lik * v;
-                    if (p1u <= cb + 32) break;
-                    cb += 32;
-                    if (cb + lane < pend) {
-                        d = __ldg(a.pdst + cb + lane) - rs;
-                        ok = ok && poll_value(a.fv + __ldg(a.psrc + cb + lane), v, lim, a.ds);
-                    }
-                }
-                p0 = p1u;
-                __syncwarp();
-            }
-        }
-        if (!__all_sync(0xffffffffu, ok)) {
-            if (!ok) atomicCAS(&a.ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
+        const int rs = __ldg(a.rp + i), len = __ldg(a.rp + i + 1) - rs, nl = __ldg(a.diag + i) - rs;
+        const long long go = __ldg(a.goff + i);
+        const int *gs = a.gsrc + go;
+        bool ok = true;
+        if (RMAX == 8 && go < 0) ok = df_long_row(a, i, df_rows + (size_t)(threadIdx.x >> 5) * a.max_row, lim);
+        else if (RMAX == 1 || len <= 32) ok = df_row<1, RMAX == 8 ? 8 : 4>(a, i, rs, len, nl, gs, lane, lim);
+        else if (RMAX == 2 || len <= 64) ok = df_row<2, 4>(a, i, rs, len, nl, gs, lane, lim);
+        else if (RMAX == 8 && len <= 128) ok = df_row<4, 2>(a, i, rs, len, nl, gs, lane, lim);
+        else if (RMAX == 8) ok = df_row<8, 2>(a, i, rs, len, nl, gs, lane, lim);
+        if (!ok) {   // uniform over the warp
+            if (lane == 0) atomicCAS(&a.ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
             return;
         }
-        __syncwarp();
-        for (int e = rs + lane; e < re; e += 32) {
-            const double x = not_pending(w[e - rs]);
-            __stcg(a.fv + e, x);
-            if (e == di && x == 0.0) {
-                if (atomicCAS(&a.ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) a.ds->aux = i;
-            }
-            sweep_put(a.out, e, x);
-        }
-        __syncwarp();
     }
 }
 
-// Right-looking LU on a fill pattern by column steps (the RF refactorization).  Level by
-// level, a warp per L entry e = (i, k) of the level's steps: l_ik = a_ik / u_kk, then the
-// entry's update pairs a_ij -= l_ik u_kj, added atomically (independent steps of one level may
+// Right-looking LU on a fill pattern by column steps, for patterns whose update pairs exceed
+// 2^31 - 1 even with a dense tail (lu.cu).  Level by level, a warp per L entry e = (i, k) of the
+// level's steps (row i from erow): l_ik = a_ik / u_kk, then every U entry (k, j), j > k, updates
+// (i, j), whose position is found by a binary search of column j in row i after e (the fill pattern is
+// closed under elimination, so it is there), added atomically (independent steps of one level may
 // update the same entry).  Every value a level reads was final before its barrier.
-__global__ void __launch_bounds__(256) lu_colstep_kernel(int nlev, const int *__restrict__ lev_ptr,
-                                                         const int *__restrict__ ent, const int *__restrict__ ci,
-                                                         const int *__restrict__ diag, const int *__restrict__ pp,
-                                                         const int *__restrict__ pdst, const int *__restrict__ psrc,
-                                                         double *fv, DevStatus *ds) {
-    __shared__ unsigned s_gen;
-    if (threadIdx.x == 0) s_gen = barrier_gen_start(ds);
-    __syncthreads();
-    unsigned gen = s_gen;
-    const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int l = 0; l < nlev; l++) {
-        const int q0 = __ldg(lev_ptr + l), q1 = __ldg(lev_ptr + l + 1);
-        for (int q = q0 + gw; q < q1; q += nw) {
-            const int e = __ldg(ent + q);
-            const int k = __ldg(ci + e);
-            double lik = 0.0;
-            if (lane == 0) {
-                const double piv = __ldcg(fv + __ldg(diag + k));
-                if (piv == 0.0) {
-                    if (atomicCAS(&ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) ds->aux = k;
-                } else {
-                    lik = __ldcg(fv + e) / piv;
-                }
-                fv[e] = lik;
-            }
-            lik = __shfl_sync(0xffffffffu, lik, 0);
-            const int t1 = __ldg(pp + e + 1);
-            if (lik != 0.0)
-                for (int t = __ldg(pp + e) + lane; t < t1; t += 32)
-                    atomicAdd(fv + __ldg(pdst + t), -lik * __ldcg(fv + __ldg(psrc + t)));
-        }
-        if (l + 1 < nlev) {
-            if (!grid_barrier(ds, gen)) return;
-        }
-    }
-}
-
-// The same column steps without stored update pairs: for the L entry e = (i, k) (row i from
-// erow), every U entry (k, j), j > k, updates (i, j), whose position is found by a binary search
-// of column j in row i after e (the fill pattern is closed under elimination, so it is there).
-// Used where the pairs would exceed 2^31 - 1 (the 70,000-bus minimum-degree LU).
 __global__ void __launch_bounds__(256) lu_colstep_search_kernel(int nlev, const int *__restrict__ lev_ptr,
                                                                 const int *__restrict__ ent,
                                                                 const int *__restrict__ erow,
@@ -720,7 +813,7 @@ static bpf_status coop_grid(bpf_ctx *ctx, K kernel, int threads, size_t smem, in
 }
 
 bpf_status factor_numeric(bpf_ctx *ctx, bpf_prec *P) {
-    if (P->kind == PREC_LU && P->cl_nlev > 0 && P->pairless) {
+    if (P->kind == PREC_LU && P->cl_nlev > 0) {
         int grid = 1;
         BPF_TRY(coop_grid(ctx, lu_colstep_search_kernel, 256, 0, std::max(1, ceil_div(P->cl_max_level, 8)), &grid));
         int nlev = P->cl_nlev;
@@ -733,25 +826,6 @@ bpf_status factor_numeric(bpf_ctx *ctx, bpf_prec *P) {
         // row i are cached re-reads)
         KScope ks(ctx, BPF_KC_FACTOR, 16.0 * P->nnz + 8.0 * (P->n + 1) + 28.0 * P->npairs, 2.0 * P->npairs);
         BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)lu_colstep_search_kernel, dim3(grid), dim3(256),
-                                                  args, 0, ctx->stream));
-        BPF_LAUNCHED(ctx);
-        return BPF_SUCCESS;
-    }
-    if (P->kind == PREC_LU && P->cl_nlev > 0) {
-        int grid = 1;
-        BPF_TRY(coop_grid(ctx, lu_colstep_kernel, 256, 0, std::max(1, ceil_div(P->cl_max_level, 8)), &grid));
-        int nlev = P->cl_nlev;
-        const int *lp = P->cl_lev_ptr, *en = P->cl_ent, *ci = P->ci, *dg = P->diag, *pp = P->pp,
-                  *pd = P->pdst, *ps = P->psrc;
-        double *fv = P->fv;
-        DevStatus *ds = ctx->dstat;
-        void *args[] = {&nlev, (void *)&lp, (void *)&en, (void *)&ci, (void *)&dg, (void *)&pp,
-                        (void *)&pd, (void *)&ps, &fv, &ds};
-        // Algorithmic bytes: the factor values read and written once, the entry list, and per
-        // update pair two indices, one value read and one atomically updated.
-        KScope ks(ctx, BPF_KC_FACTOR, 16.0 * P->nnz + 8.0 * (P->n + 1) + 24.0 * P->npairs,
-                  2.0 * P->npairs);
-        BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)lu_colstep_kernel, dim3(grid), dim3(256),
                                                   args, 0, ctx->stream));
         BPF_LAUNCHED(ctx);
         return BPF_SUCCESS;
@@ -1171,36 +1245,37 @@ bpf_status prec_load_values(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     return BPF_SUCCESS;
 }
 
-// Data-flow ILU(0): rows of up to max_row entries in shared memory, eight warps per CTA while
-// they fit (2,800 entries), else as many as do; longer rows use the level kernel.
-static bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const double *vals, bool *taken) {
+// Data-flow factorization.  Rows too long for gather lists go through shared memory, eight warps per
+// CTA while they fit (3,600 entries), else as many as do; longer rows are not taken.
+bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const int *order, int rows, const double *vals, bool *taken) {
     *taken = false;
     int wpb = 8;
-    const size_t row_bytes = sizeof(double) * (size_t)P->max_row;
+    const size_t row_bytes = P->max_row > kGatherRow ? sizeof(double) * (size_t)P->max_row : 0;
     while (wpb > 1 && wpb * row_bytes > (size_t)ctx->max_smem_optin) wpb >>= 1;
     if (wpb * row_bytes > (size_t)ctx->max_smem_optin) return BPF_SUCCESS;
+    *taken = true;
+    const int fb = std::max(1, std::min(ceil_div(P->nnz, 256), ctx->num_sms * 8));
+    fill_pending_kernel<<<fb, 256, 0, ctx->stream>>>((size_t)P->nnz, P->fv);   // rows not listed here too
+    BPF_LAUNCHED(ctx);
+    if (rows == 0) return BPF_SUCCESS;
     const size_t smem = wpb * row_bytes;
-    BPF_CUDA(ctx, cudaFuncSetAttribute(factor_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto kern = P->max_row <= 32 ? factor_df_kernel<1> : P->max_row <= 64 ? factor_df_kernel<2> : factor_df_kernel<8>;
+    BPF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int grid = 1;
-    BPF_TRY(coop_grid(ctx, factor_df_kernel, 32 * wpb, smem, ceil_div(P->n, wpb), &grid));
-    FactorDfArgs a{P->n, P->max_row, P->lower.rows, P->rp, P->ci, P->diag, P->pp, P->pdst, P->psrc, vals, P->fsrc,
-                   P->fv, sweep_store(P), ctx->dstat};
+    BPF_TRY(coop_grid(ctx, kern, 32 * wpb, smem, ceil_div(rows, wpb), &grid));
+    FactorDfArgs a{rows, P->max_row, order, P->rp, P->ci, P->diag, P->pp, P->pdst, P->psrc, P->gsrc, P->goff,
+                   vals, P->fsrc, P->fv, sweep_store(P), ctx->dstat};
     void *args[] = {&a};
     KScope ks(ctx, BPF_KC_FACTOR, 44.0 * P->nnz + 12.0 * (P->n + 1) + 8.0 * P->npairs, 2.0 * P->npairs);
-    const int fb = std::max(1, std::min(ceil_div(P->nnz, 256), ctx->num_sms * 8));
-    fill_pending_kernel<<<fb, 256, 0, ctx->stream>>>((size_t)P->nnz, P->fv);
+    BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(32 * wpb), args, smem, ctx->stream));
     BPF_LAUNCHED(ctx);
-    BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)factor_df_kernel, dim3(grid), dim3(32 * wpb), args, smem,
-                                              ctx->stream));
-    BPF_LAUNCHED(ctx);
-    *taken = true;
     return BPF_SUCCESS;
 }
 
 bpf_status prec_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     if (P->kind == PREC_ILU0 && P->n > 0) {
         bool taken = false;
-        BPF_TRY(factor_df(ctx, P, vals, &taken));
+        BPF_TRY(factor_df(ctx, P, P->lower.rows, P->n, vals, &taken));
         if (taken) return BPF_SUCCESS;
     }
     BPF_TRY(prec_load_values(ctx, P, vals));

@@ -1,7 +1,10 @@
 // Internal types of the preconditioner / triangular-factor machinery.
 #pragma once
 
+#include <algorithm>
 #include <memory>
+#include <system_error>
+#include <thread>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -16,6 +19,7 @@ struct TriHost {
     int nlev = 0;
     int max_level_rows = 0;
     bool unit = true;
+    bool keep_last = false;    // the last level's rows stay in their order (the LU's dense tail)
     std::vector<int> lev_ptr;  // nlev+1, positions into rows
     std::vector<int> rows;     // n, row id at each level-sorted position
     std::vector<int> rp;       // n+1, per level-sorted position
@@ -89,6 +93,26 @@ struct NoInitAlloc : std::allocator<T> {
 };
 using PairVec = std::vector<int, NoInitAlloc<int>>;
 
+// f() on up to 16 host threads (this one alone when small); f takes its work from a shared counter, so
+// fewer threads than asked do as well.
+template <typename F>
+void run_threads(bool large, const F &f) {
+    const unsigned hw = std::thread::hardware_concurrency();
+    const int nthreads = large ? (int)std::min(16u, std::max(1u, hw)) : 1;
+    std::vector<std::thread> pool;
+    try {
+        for (int t = 1; t < nthreads; t++) pool.emplace_back(f);
+    } catch (const std::system_error &) {
+        // a thread limit: the calling thread takes what the helpers do not
+    }
+    f();
+    for (auto &th : pool) th.join();
+}
+// Gather lists (bpf_prec::goff, gsrc) of the first `rows` rows but those `skip` marks (if not empty);
+// returns the number of updates.
+constexpr int kGatherRow = 256;
+long long build_gather(int rows, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &diag,
+                       const std::vector<char> &skip, std::vector<long long> &goff, PairVec &gsrc);
 // false (and empty outputs) when the pair count exceeds INT_MAX
 bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
                  std::vector<int> &pp, PairVec &pdst, PairVec &psrc);
@@ -98,8 +122,9 @@ struct TriStream {
     std::vector<int> coff, cslab, head;   // per chunk: byte offset, first slab; slab headers
     int diag = 0, nstage = 0;
 };
-void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<int> &pos, TriStream &out,
-                   std::vector<int> &tpos);
+// ntot: unknowns (rows from t.n on keep their positions); lu: long rows over a whole warp
+void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
+                   TriStream &out, std::vector<int> &tpos);
 // values = false: the schedule only (the values are kept elsewhere)
 bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d, bool values = true);
 void tri_free(TriDev &d);
@@ -116,25 +141,38 @@ struct bpf_prec {
     // pattern (0-based device copies) and factor values in pattern order
     int *rp = nullptr, *ci = nullptr, *diag = nullptr;
     double *fv = nullptr;
-    // ILU(0) data-flow factorization: the longest row, and the source entry of A per pattern entry
-    // (null: the same position)
+    // Data-flow factorization: the longest row, and the source entry of A per pattern entry (null: the
+    // same position; -1: fill, zero)
     int max_row = 0;
     int *fsrc = nullptr;
+    // Rows of up to kGatherRow entries: per L entry and entry of the row, the position of U's entry that
+    // updates it (-1: none), from goff[i] on (-1: a longer row, which goes by its update pairs).
+    long long *goff = nullptr;
+    int *gsrc = nullptr;
     int *pp = nullptr, *pdst = nullptr, *psrc = nullptr;
     long long npairs = 0;
     bpf::TriDev lower;   // forward solve (L unit for ILU0; L for IC0)
     bpf::TriDev upper;   // backward solve (U for ILU0; L' for IC0)
-    // LU on a fill pattern (the RF refactorization): right-looking column steps; step k (scale
-    // column k of L by 1 / u_kk, then apply its update pairs) waits for the steps that update
-    // row k or column k.  cl_lev_ptr / cl_ent: the L entries of each level's steps.
-    int cl_nlev = 0, cl_max_level = 0;
-    int *cl_lev_ptr = nullptr, *cl_ent = nullptr;
-    // Without stored update pairs (patterns whose pairs exceed 2^31 - 1, or BPF_LU_PAIRLESS=1):
-    // each L entry's updates are found by a search in its row; cl_row = the row of each listed
-    // entry.  npairs then counts the updates.
+    // LU on a fill pattern (the RF refactorization, lu.cu): rows and columns from tail_s on, tail_m of
+    // them padded to tail_mp, are a dense block: tail_S receives the Schur complement, tail_F holds
+    // the off-diagonal 64 x 64 tiles of its factors, tail_inv the inverted diagonal ones (L, then U).
+    // fend[i]: end of row i's entries before column tail_s.
+    // forder: the rows in the order of the factorization, nshort rows a warp takes, then nlong front
+    // rows a CTA takes (long rows, and what depends on them), then the tail;
+    // cta_nmax / cta_wmax: most entries to eliminate, longest storage of a CTA's row.
+    int tail_s = 0, tail_m = 0, tail_mp = 0, nshort = 0, nlong = 0, cta_nmax = 0, cta_wmax = 0;
+    long long cta_pairs = 0;
+    int *forder = nullptr;
+    int *fend = nullptr;
+    double *tail_S = nullptr, *tail_F = nullptr, *tail_inv = nullptr;
+    // LU whose front still has more than 2^31 - 1 update pairs (or BPF_LU_PAIRLESS=1): right-looking
+    // column steps that find an entry's updates by a search in its row.  Step k (scale column k of L by
+    // 1 / u_kk, then apply its updates) waits for the steps that update row k or column k;
+    // cl_lev_ptr / cl_ent / cl_row: the L entries of each level's steps and their rows.
     bool pairless = false;
-    int *cl_row = nullptr;
-    // LU solves in push form (right-looking): per level of each sweep, the factor entries whose
+    int cl_nlev = 0, cl_max_level = 0;
+    int *cl_lev_ptr = nullptr, *cl_ent = nullptr, *cl_row = nullptr;
+    // and its solves in push form (right-looking): per level of each sweep, the factor entries whose
     // source row became final at that level, as (source row, target row, position in fv).
     int ps_nlev[2] = {0, 0}, ps_max_level = 0;
     int *ps_ptr[2] = {nullptr, nullptr}, *ps_src[2] = {nullptr, nullptr},
@@ -184,6 +222,15 @@ bpf_status factor_numeric(bpf_ctx *ctx, bpf_prec *P);
 // The whole numeric step from A's values (device, A's entry order): values in, factors in fv and
 // in the level-sorted storage of both sweeps.
 bpf_status prec_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals);
+// Data-flow factorization of the listed rows (order: device, dependencies first) from A's values;
+// *taken = false when a row does not fit in shared memory.
+bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const int *order, int rows, const double *vals, bool *taken);
+// LU with a dense tail (lu.cu).
+bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::vector<int> &ci,
+                    const std::vector<int> &diag, const std::vector<int> &fsrc, const std::vector<int> &rowP,
+                    const std::vector<int> &colQ, bool *fits, bpf_prec **out);
+bpf_status lu_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals);
+bpf_status lu_solve(bpf_ctx *ctx, const bpf_prec *P, int nrhs, double *X, int ldx);   // in place
 // Column-per-CTA triangular solves (trsv_col.cu) of a preconditioner kept for them (P->col):
 // column-major blocks (Y may be X with the same leading dimension), or row-major ones.
 bool trsv_col_fits(const bpf_ctx *ctx, int n, int fdtype);
@@ -204,4 +251,37 @@ bpf_status bj_setup(bpf_ctx *ctx, bpf_prec *P);
 bpf_status bj_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y);
 // Y = U^{-1} L^{-1} Y in place (row-major n x p, p <= 256) for an LU factor with push lists.
 bpf_status lu_solve_push_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, double *Y);
+}  // namespace bpf
+
+namespace bpf {
+// The storage of the two sweeps that a factor entry goes to (bpf_prec::tpos), CSR or stream.
+struct SweepStore {
+    const int *tpos[2];
+    double *val[2], *dinv[2];      // level-sorted storage, FP64 and FP32
+    float *valf[2], *dinvf[2];
+    unsigned char *stream[2];      // or the streams (column solves), of FP32 values if f32
+    int col, f32;
+};
+
+__device__ __forceinline__ void sweep_put(const SweepStore &s, int e, double x) {
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+        const int t = s.tpos[w] ? __ldg(s.tpos[w] + e) : -1;
+        if (t == -1) continue;
+        const double v = t >= 0 ? x : 1.0 / x;
+        const int k = t >= 0 ? t : -2 - t;
+        if (s.col) {
+            if (s.f32) reinterpret_cast<float *>(s.stream[w])[k] = (float)v;
+            else reinterpret_cast<double *>(s.stream[w])[k] = v;
+        } else if (t >= 0) {
+            s.val[w][k] = v;
+            s.valf[w][k] = (float)v;
+        } else {
+            s.dinv[w][k] = v;
+            s.dinvf[w][k] = (float)v;
+        }
+    }
+}
+
+SweepStore sweep_store(const bpf_prec *P);
 }  // namespace bpf

@@ -11,12 +11,12 @@
 //      threshold 1.0 as the reference passes to csrluFactorHost (:148);
 //   3. the structural L + U pattern of A_hat = A(P, q) in CSR, and the map from A's entries
 //      into it.
-// Device side: the numeric factorization is the same level-scheduled cooperative kernel as
-// ILU(0), run on the L + U pattern (no fill is dropped, so it is the exact LU with the fixed
-// pivot order), and the solve is one cooperative launch of both triangular sweeps with the
-// row permutation P fused into the layout conversion on the way in and Q on the way out.
+// Device side: lu.cu (sparse front as a data flow, dense tail on the FP64 tensor pipe), with the
+// row permutation P on the way in and Q on the way out; patterns whose front has more than 2^31 - 1
+// update pairs run by column steps and push-form solves (prec.cu).
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <queue>
 #include <set>
@@ -184,8 +184,9 @@ struct bpf_rf {
     int *amap = nullptr;              // A entry -> L+U position
     bpf_prec *lu = nullptr;           // pattern, schedules and factor of the (uniform) matrix
     bool uniform = true;              // all batch replicas hold the same values
-    // per-replica factor values (batch mode after rf_batch_refactor with distinct columns)
-    std::vector<double *> rep_lval, rep_uval, rep_dinv;
+    // per-replica copies of the arrays the solves read (batch mode after rf_batch_refactor with
+    // distinct columns), in solve_arrays' order
+    std::vector<std::vector<void *>> reps;
 };
 
 namespace bpf {
@@ -193,6 +194,7 @@ namespace bpf {
 static bpf_status rf_factor_values(bpf_rf *rf, const double *vals) {
     bpf_ctx *ctx = rf->ctx;
     bpf_prec *P = rf->lu;
+    if (!P->pairless) return lu_factor(ctx, P, vals);
     BPF_CUDA(ctx, cudaMemsetAsync(P->fv, 0, sizeof(double) * P->nnz, ctx->stream));
     if (rf->nnzA > 0) {
         int blocks = std::min(ceil_div(rf->nnzA, 256), ctx->num_sms * 8);
@@ -205,13 +207,31 @@ static bpf_status rf_factor_values(bpf_rf *rf, const double *vals) {
     return BPF_SUCCESS;
 }
 
+// The arrays of a factor that its solves read, with their sizes in bytes.
+struct SolveArray {
+    void **ptr;
+    size_t bytes;
+};
+static std::vector<SolveArray> solve_arrays(bpf_prec *P) {
+    std::vector<SolveArray> v;
+    if (P->col)
+        for (auto &c : P->cs) v.push_back({(void **)&c.bytes, c.len});
+    else
+        for (TriDev *t : {&P->lower, &P->upper}) {
+            v.push_back({(void **)&t->val, sizeof(double) * t->nnz});
+            if (!t->unit) v.push_back({(void **)&t->dinv, sizeof(double) * t->n});
+        }
+    if (P->tail_mp > 0) {
+        v.push_back({(void **)&P->tail_F, sizeof(double) * (size_t)P->tail_mp * P->tail_mp});
+        v.push_back({(void **)&P->tail_inv, sizeof(double) * 2 * (size_t)P->tail_mp * 64});
+    }
+    return v;
+}
+
 static void rf_free_replicas(bpf_rf *rf) {
-    for (double *p : rf->rep_lval) cudaFree(p);
-    for (double *p : rf->rep_uval) cudaFree(p);
-    for (double *p : rf->rep_dinv) cudaFree(p);
-    rf->rep_lval.clear();
-    rf->rep_uval.clear();
-    rf->rep_dinv.clear();
+    for (auto &r : rf->reps)
+        for (void *p : r) cudaFree(p);
+    rf->reps.clear();
 }
 
 }  // namespace bpf
@@ -313,7 +333,15 @@ bpf_status bpf_rf_analyze(bpf_ctx *ctx, const bpf_csr_desc *A, int ordering, dou
         bpf_rf_destroy(rf);
         return s;
     };
-    bpf_status s = prec_setup(ctx, PREC_LU, n, Frp, Fci, Fdiag, BPF_F64, {}, &rf->lu);
+    const char *env_pl = getenv("BPF_LU_PAIRLESS");
+    bool fits = !(env_pl && atoi(env_pl) != 0);
+    bpf_status s = BPF_SUCCESS;
+    if (fits) {
+        std::vector<int> fsrc(Fci.size(), -1);
+        for (int k = 0; k < nnz; k++) fsrc[amap[k]] = k;
+        s = lu_setup(ctx, n, Frp, Fci, Fdiag, fsrc, rf->P, rf->Q, &fits, &rf->lu);
+    }
+    if (s == BPF_SUCCESS && !fits) s = prec_setup(ctx, PREC_LU, n, Frp, Fci, Fdiag, BPF_F64, {}, &rf->lu);
     if (s != BPF_SUCCESS) return fail(s);
     cudaError_t e = cudaMalloc((void **)&rf->Pd, sizeof(int) * std::max(n, 1));
     if (e == cudaSuccess) e = cudaMalloc((void **)&rf->Qd, sizeof(int) * std::max(n, 1));
@@ -347,25 +375,16 @@ bpf_status bpf_rf_refactor_batch(bpf_rf *rf, const double *vals, int ld) {
     if (rf->batch == 1) return bpf_rf_refactor(rf, vals);
     rf_free_replicas(rf);
     rf->uniform = false;
-    bpf_prec *P = rf->lu;
-    const int n = rf->n;
+    const std::vector<SolveArray> arrays = solve_arrays(rf->lu);
     for (int r = 0; r < rf->batch; r++) {
         BPF_TRY(rf_factor_values(rf, vals + (size_t)r * ld));
-        double *lv = nullptr, *uv = nullptr, *dv = nullptr;
-        BPF_CUDA(ctx, cudaMalloc((void **)&lv, sizeof(double) * std::max(P->lower.nnz, 1)));
-        rf->rep_lval.push_back(lv);
-        BPF_CUDA(ctx, cudaMalloc((void **)&uv, sizeof(double) * std::max(P->upper.nnz, 1)));
-        rf->rep_uval.push_back(uv);
-        BPF_CUDA(ctx, cudaMalloc((void **)&dv, sizeof(double) * std::max(n, 1)));
-        rf->rep_dinv.push_back(dv);
-        if (P->lower.nnz)
-            BPF_CUDA(ctx, cudaMemcpyAsync(lv, P->lower.val, sizeof(double) * P->lower.nnz,
-                                          cudaMemcpyDeviceToDevice, ctx->stream));
-        if (P->upper.nnz)
-            BPF_CUDA(ctx, cudaMemcpyAsync(uv, P->upper.val, sizeof(double) * P->upper.nnz,
-                                          cudaMemcpyDeviceToDevice, ctx->stream));
-        BPF_CUDA(ctx, cudaMemcpyAsync(dv, P->upper.dinv, sizeof(double) * n, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
+        rf->reps.emplace_back();
+        for (const SolveArray &a : arrays) {
+            void *p = nullptr;
+            BPF_CUDA(ctx, cudaMalloc(&p, std::max<size_t>(a.bytes, 16)));
+            rf->reps.back().push_back(p);
+            if (a.bytes) BPF_CUDA(ctx, cudaMemcpyAsync(p, *a.ptr, a.bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        }
     }
     return check_dev_status(ctx, "rf_refactor_batch");
 }
@@ -379,6 +398,7 @@ bpf_status bpf_rf_solve(bpf_rf *rf, int nrhs, double *X, int ldx) {
     if (rf->batch > 1 && nrhs != rf->batch)
         return set_error(ctx, BPF_ERR_DIMENSION, "batch mode solves exactly batchsize=%d columns", rf->batch);
     if (n == 0 || nrhs == 0) return BPF_SUCCESS;
+    if (rf->uniform && !rf->lu->pairless) return lu_solve(ctx, rf->lu, nrhs, X, ldx);
     const int chunk = 256;
     bpf_status s;
     double *buf = (double *)ws_get(ctx, WS_A, sizeof(double) * (size_t)n * std::min(nrhs, chunk), &s);
@@ -401,27 +421,25 @@ bpf_status bpf_rf_solve(bpf_rf *rf, int nrhs, double *X, int ldx) {
         for (int c0 = 0; c0 < nrhs; c0 += chunk) {
             int pc = std::min(chunk, nrhs - c0);
             BPF_TRY(conv_in(c0, pc));
-            if (rf->lu->ps_nlev[0] + rf->lu->ps_nlev[1] > 0)
-                BPF_TRY(lu_solve_push_rowmajor(ctx, rf->lu, pc, buf));
-            else
-                BPF_TRY(prec_apply_rowmajor(ctx, rf->lu, pc, buf, buf));
+            BPF_TRY(lu_solve_push_rowmajor(ctx, rf->lu, pc, buf));
             BPF_TRY(conv_out(c0, pc));
         }
         return BPF_SUCCESS;
     }
     // distinct replicas: column r with replica r's factors
     bpf_prec *P = rf->lu;
-    double *lv0 = P->lower.val, *uv0 = P->upper.val, *dv0 = P->upper.dinv;
+    std::vector<SolveArray> arrays = solve_arrays(P);
     for (int r = 0; r < nrhs; r++) {
-        P->lower.val = rf->rep_lval[r];
-        P->upper.val = rf->rep_uval[r];
-        P->upper.dinv = rf->rep_dinv[r];
-        bpf_status st = conv_in(r, 1);
-        if (st == BPF_SUCCESS) st = prec_apply_rowmajor(ctx, P, 1, buf, buf);
-        if (st == BPF_SUCCESS) st = conv_out(r, 1);
-        P->lower.val = lv0;
-        P->upper.val = uv0;
-        P->upper.dinv = dv0;
+        for (size_t k = 0; k < arrays.size(); k++) std::swap(*arrays[k].ptr, rf->reps[r][k]);
+        bpf_status st;
+        if (P->pairless) {
+            st = conv_in(r, 1);
+            if (st == BPF_SUCCESS) st = prec_apply_rowmajor(ctx, P, 1, buf, buf);
+            if (st == BPF_SUCCESS) st = conv_out(r, 1);
+        } else {
+            st = lu_solve(ctx, P, 1, X + (size_t)r * ldx, ldx);
+        }
+        for (size_t k = 0; k < arrays.size(); k++) std::swap(*arrays[k].ptr, rf->reps[r][k]);
         if (st != BPF_SUCCESS) return st;
     }
     return BPF_SUCCESS;

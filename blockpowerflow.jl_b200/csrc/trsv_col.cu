@@ -20,6 +20,8 @@
 //    four 16-bit columns in one 8-byte load and its values in 16-byte loads, and a padding entry
 //    is a zero times the unknown after the last, which is zero: no branch or predicate between the
 //    barrier and the result (with them a slab took ~1,000 cycles).
+//  * An LU's long rows (more than kWideRow entries) are slabs of their own, a row's entries over the
+//    32 lanes and a warp sum at the end.
 //  * Slab g goes to warp g mod nw, levels notwithstanding: a warp fetches its next slab's
 //    entries, if they have arrived, then passes the level barriers that separate it from the last,
 //    so in a long chain of narrow levels the fetches of the coming levels overlap the current one.
@@ -49,6 +51,7 @@
 namespace bpf {
 
 constexpr int kChunk = 16384;      // bytes of a chunk, at most
+constexpr int kWideRow = 16;       // entries past which an LU's row takes a whole warp
 constexpr int kColWarps = 23;      // computing warps, at most
 constexpr int kChunkRing = 6;      // chunks in flight, at most (as many as fit beside the column)
 
@@ -89,6 +92,8 @@ struct ColGroup<float> {
         c[3] = y >> 16;
     }
 };
+__device__ __forceinline__ double warp_total(double v) { return warp_sum(v); }
+__device__ __forceinline__ float warp_total(float v) { return warp_sumf(v); }
 // Unknown i of the column at shared address y.
 __device__ __forceinline__ void col_get(unsigned y, unsigned i, double &v) {
     asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(y + 8 * i));
@@ -107,12 +112,16 @@ struct ColArgs {
     int n, nring;
     const unsigned char *stream[2];
     const int *coff[2], *cslab[2];   // per chunk: byte offset, first slab
-    // per slab: first position | rows << 16 | groups of entries << 22 | last part << 27; offset of
+    // per slab: first position | rows << 16 | groups of entries << 22 | last part << 27 | one row over
+    // all lanes << 28; offset of
     // its entries in the ring | slot << 20 | parity of the slot's phase << 24; stage; chunk (of both
     // sweeps)
     const int4 *head[2];
     int nchunk[2], nslab[2], nstage[2], diag[2];
     const int *pos0, *pos01, *pos1;
+    // the LU's dense tail: unknowns s.. of both sweeps, nb tiles of 64 (0: none)
+    int s, nb;
+    const double *F, *Linv, *Uinv;
 };
 
 // Counters of the ring, relaxed: `ready` only tells that a slot's mbarrier phase is over (its own wait
@@ -160,7 +169,7 @@ __device__ __forceinline__ void col_produce(const ColArgs &a, unsigned char *rin
             const unsigned bytes = (unsigned)(__ldg(a.coff[w] + k + 1) - o);
             st_relaxed_cta(r.done + islot, 0u);
             mbar_expect_tx(r.full + islot, bytes);
-            bulk_g2s(ring + (size_t)islot * kChunk, a.stream[w] + o, bytes, r.full + islot);
+            if (bytes > 0) bulk_g2s(ring + (size_t)islot * kChunk, a.stream[w] + o, bytes, r.full + islot);
             if (++islot == a.nring) islot = 0;
             if (++issued >= a.nring && issued < total) need = slabs(issued - a.nring);
             moved = true;
@@ -214,9 +223,10 @@ __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstag
             if (ng > 0) e.load(ch, lane);
         }
         seen = h.w;
-        if (lane < rows) {
-            TF acc;
-            col_get(y, q + lane, acc);
+        const bool wide = (h.x >> 28) & 1;
+        if (wide || lane < rows) {
+            TF acc = (TF)0;
+            if (!wide || lane == 0) col_get(y, q + lane, acc);
             for (int j = 0; j < ng; j++) {
                 TF v[4];
 #pragma unroll
@@ -226,12 +236,13 @@ __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstag
                 for (int u = 0; u < 4; u++) acc -= e.a[u] * v[u];
                 e = en;
             }
-            if (diag && (h.x >> 27)) {
+            if (wide) acc = warp_total(acc);
+            if (diag && ((h.x >> 27) & 1)) {
                 TF dv;
                 col_get(ch + ng * ColGroup<TF>::bytes, lane, dv);
                 acc *= dv;
             }
-            col_put(y, q + lane, acc);
+            if (!wide || lane == 0) col_put(y, q + lane, acc);
         }
         __syncwarp();
         if (lane == 0) red_relaxed_cta(r.done + slot, 1u);
@@ -239,6 +250,51 @@ __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstag
     // every warp passes every barrier, whatever its waits brought
     for (; passed < nstage; passed++) col_barrier(32 * nw);
     return ok;
+}
+
+// y[0..64) of a dense tail in shared memory, at address y: U^{-1} L^{-1} y by 64-wide block steps.  A
+// warp takes four rows at a time, two columns a lane; z: 64 values of scratch.
+__device__ __forceinline__ void col_tail(const ColArgs &a, unsigned y, double *z, int nw) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t ld = (size_t)a.nb * 64;
+    // sums over 64 columns of rows r (< r1) of A (row stride lda) times x (shared): f(r, sum)
+    auto rows = [&](const double *A, size_t lda, int r0, int r1, unsigned x, auto f) {
+        double x0, x1;
+        col_get(x, 2 * lane, x0);
+        col_get(x, 2 * lane + 1, x1);
+        for (int r = r0 + 4 * warp; r < r1; r += 4 * nw) {
+            double2 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = __ldg(reinterpret_cast<const double2 *>(A + (size_t)(r + u) * lda) + lane);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const double s = warp_sum(v[u].x * x0 + v[u].y * x1);
+                if (lane == 0) f(r + u, s);
+            }
+        }
+    };
+    const unsigned zs = smem_u32(z);
+#pragma unroll 1
+    for (int sweep = 0; sweep < 2; sweep++)
+#pragma unroll 1
+        for (int bi = 0; bi < a.nb; bi++) {
+            const int b = sweep == 0 ? bi : a.nb - 1 - bi;
+            rows((sweep == 0 ? a.Linv : a.Uinv) + (size_t)b * 4096, 64, 0, 64, y + 512 * b,
+                 [&](int r, double v) { col_put(zs, r, v); });
+            col_barrier(32 * nw);
+            if (threadIdx.x < 64) {
+                double v;
+                col_get(zs, threadIdx.x, v);
+                col_put(y, 64 * b + threadIdx.x, v);
+            }
+            rows(a.F + (size_t)b * 64, ld, sweep == 0 ? 64 * (b + 1) : 0, sweep == 0 ? 64 * a.nb : 64 * b, zs,
+                 [&](int r, double v) {
+                     double o;
+                     col_get(y, r, o);
+                     col_put(y, r, o - v);
+                 });
+            col_barrier(32 * nw);
+        }
 }
 
 template <typename TF>
@@ -268,7 +324,7 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, c
     const unsigned rbase = smem_u32(ring), y = rbase + a.nring * kChunk;
     X += blockIdx.x * ldx;
     Y += blockIdx.x * ldy;
-    if (tid == 0) col_put(y, n, (TF)0);
+    for (int i = n + tid; i <= max(n, a.s + 64 * a.nb); i += nt) col_put(y, i, (TF)0);
     for (int i0 = tid; i0 < n; i0 += 8 * nt) {   // eight loads in flight
         int at[8];
         double v[8];
@@ -284,6 +340,11 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, c
     }
     col_barrier(nt);
     bool ok = col_sweep<TF>(a.head[0], a.nslab[0], a.nstage[0], a.diag[0] != 0, y, rbase, r, nw, true);
+    if constexpr (std::is_same<TF, double>::value)
+        if (a.nb > 0) {
+            __shared__ double z[64];
+            col_tail(a, y + 8 * a.s, z, nw);
+        }
     for (int i0 = tid; i0 < n; i0 += 8 * nt) {   // forward results in backward positions, through Y
         int at[8];
 #pragma unroll
@@ -304,6 +365,7 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, c
         for (int u = 0; u < 8; u++)
             if (i0 + u * nt < n) col_put(y, i0 + u * nt, (TF)v[u]);
     }
+    for (int i = n + tid; i <= a.s + 64 * a.nb; i += nt) col_put(y, i, (TF)0);   // (the tail's padding)
     col_barrier(nt);
     ok = col_sweep<TF>(a.head[1], a.nslab[1], a.nstage[1], a.diag[1] != 0, y, rbase, r, nw, ok);
     if (!ok) atomicCAS(&ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
@@ -322,7 +384,7 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, c
 
 // Chunks that fit in shared memory beside the column (1 KB left for the kernel's own variables).
 int trsv_col_ring(const bpf_ctx *ctx, int n, int fdtype) {
-    const long long left = (long long)ctx->max_smem_optin - 1024 - (n + 1ll) * (fdtype == BPF_F32 ? 4 : 8);
+    const long long left = (long long)ctx->max_smem_optin - 1024 - 512 - (n + 1ll) * (fdtype == BPF_F32 ? 4 : 8);
     return left <= 0 ? 0 : (int)std::min<long long>(kChunkRing, left / kChunk);
 }
 // Whether a factor of n rows is kept for the column solves: the column and two chunks fit.
@@ -336,7 +398,12 @@ bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, siz
     ColArgs a;
     a.n = P->n;
     a.nring = trsv_col_ring(ctx, P->n, P->fdtype);
-    const size_t smem = (size_t)a.nring * kChunk + ((size_t)P->n + 1) * es;
+    a.s = P->tail_s;
+    a.nb = P->tail_mp / 64;
+    a.F = P->tail_F;
+    a.Linv = P->tail_inv;
+    a.Uinv = P->tail_inv + (size_t)P->tail_mp * 64;
+    const size_t smem = (size_t)a.nring * kChunk + (std::max(P->n, a.s + P->tail_mp) + 1) * es;
     double fb = 0.0;
     for (int w = 0; w < 2; w++) {
         a.stream[w] = P->cs[w].bytes;
@@ -355,7 +422,8 @@ bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, siz
     // Computing warps for about two average levels, up to kColWarps: more of them only make the barriers of
     // a long chain of narrow levels wider.  One more warp brings the chunks.
     const int per_level = P->n / std::max(1, std::min(P->lower.nlev, P->upper.nlev));
-    const int threads = 32 * (1 + std::min(kColWarps, std::max(4, ceil_div(2 * per_level, 32))));
+    // (the dense tail of an LU takes 16 at least).
+    const int threads = 32 * (1 + std::min(kColWarps, std::max(a.nb > 0 ? 16 : 4, ceil_div(2 * per_level, 32))));
     KScope ks(ctx, BPF_KC_TRSV, fb + 12.0 * P->n + 16.0 * (double)P->n * p,
               2.0 * ((double)P->lower.nnz + P->upper.nnz + P->n) * p);
     auto kern = f32 ? trsv_col_kernel<float> : trsv_col_kernel<double>;
@@ -381,13 +449,14 @@ bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const doubl
 // ... follow); pos[i] = position of row i; tpos[k] = value index (in units of the factor type) of
 // pattern entry k in the stream (-2 - index: its reciprocal's).  nring: slots of the ring; chunk0:
 // chunks of the sweep before.
-void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<int> &pos, TriStream &out,
-                   std::vector<int> &tpos) {
+void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
+                   TriStream &out, std::vector<int> &tpos) {
+    const int wide_row = lu ? kWideRow : 2147483647;
     const size_t es = fdtype == BPF_F32 ? sizeof(float) : sizeof(double);
     const int n = t.n;
     std::vector<int> ord(n);
     for (int q = 0; q < n; q++) ord[q] = q;
-    for (int l = 0; l < t.nlev; l++)
+    for (int l = 0; l < t.nlev - (t.keep_last ? 1 : 0); l++)
         std::stable_sort(ord.begin() + t.lev_ptr[l], ord.begin() + t.lev_ptr[l + 1],
                          [&](int x, int y) { return t.rp[x + 1] - t.rp[x] > t.rp[y + 1] - t.rp[y]; });
     TriHost s = t;
@@ -401,13 +470,14 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<in
         if (!t.unit) s.dmap[q] = t.dmap[o];
     }
     t = std::move(s);
-    pos.resize(n);
+    pos.resize(ntot);
+    for (int i = n; i < ntot; i++) pos[i] = i;
     for (int q = 0; q < n; q++) pos[t.rows[q]] = q;
 
     // a slab part: positions q0.. (rows of them), its entries j0.. in ng groups, whether it is the
-    // rows' last part, its stage
+    // rows' last part, its stage, whether one row takes all lanes
     struct Part {
-        int q0, rows, j0, ng, last, stage;
+        int q0, rows, j0, ng, last, stage, wide;
     };
     const size_t gb = 256 + 128 * es;
     auto part_bytes = [&](int ng) { return ng * gb + (t.unit ? 0 : 32 * es); };
@@ -427,17 +497,18 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<in
         for (int k = 0; k < ns; k++) {
             const Part &d = cur[k];
             const int c = chunk0 + (int)out.coff.size() - 1, slot = c % nring;
-            for (int v : {d.q0 | (d.rows << 16) | (d.ng << 22) | (d.last << 27),
+            for (int v : {d.q0 | (d.rows << 16) | (d.ng << 22) | (d.last << 27) | (d.wide << 28),
                           (slot * kChunk + (int)off) | (slot << 20) | (((c / nring) & 1) << 24), d.stage, c})
                 out.head.push_back(v);
             for (int g = 0; g < d.ng; g++) {
                 unsigned short *c16 = reinterpret_cast<unsigned short *>(ch + off + g * gb);
-                std::fill(c16, c16 + 128, (unsigned short)n);   // padding: the zero after the last unknown
+                std::fill(c16, c16 + 128, (unsigned short)ntot);   // padding: the zero after the last unknown
                 const size_t vbase = (at + off + g * gb + 256) / es;
-                for (int r = 0; r < d.rows; r++)
+                for (int r = 0; r < (d.wide ? 32 : d.rows); r++)
                     for (int u = 0; u < 4; u++) {
-                        const int e = t.rp[d.q0 + r] + d.j0 + 4 * g + u;
-                        if (e >= t.rp[d.q0 + r + 1]) break;
+                        const int row = d.wide ? d.q0 : d.q0 + r;
+                        const int e = t.rp[row] + d.j0 + (d.wide ? 128 * g + 4 * r + u : 4 * g + u);
+                        if (e >= t.rp[row + 1]) break;
                         c16[4 * r + u] = (unsigned short)pos[t.ci[e]];
                         tpos[t.map[e]] = (int)(vbase + (fdtype == BPF_F32 ? 4 * r + u : 64 * (u / 2) + 2 * r + u % 2));
                     }
@@ -460,14 +531,20 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, std::vector<in
     for (int l = 0; l < t.nlev; l++) {
         int rest = 0;   // further parts the widest slab needs (each a stage of its own)
         for (int pass = 0; pass <= rest; pass++, stage++) {
-            for (int q0 = t.lev_ptr[l]; q0 < t.lev_ptr[l + 1]; q0 += 32) {
-                const int rows = std::min(t.lev_ptr[l + 1] - q0, 32);
-                const int ng = (t.rp[q0 + 1] - t.rp[q0] + 3) / 4;   // of the longest row (sorted)
+            for (int q0 = t.lev_ptr[l], rows; q0 < t.lev_ptr[l + 1]; q0 += rows) {
+                const int wide = t.rp[q0 + 1] - t.rp[q0] > wide_row;
+                int w = 0;
+                for (rows = 0; rows < (wide ? 1 : 32) && q0 + rows < t.lev_ptr[l + 1]; rows++) {
+                    const int len = t.rp[q0 + rows + 1] - t.rp[q0 + rows];
+                    if (!wide && len > wide_row) break;
+                    w = std::max(w, len);
+                }
+                const int ng = wide ? (w + 127) / 128 : (w + 3) / 4;
                 const int parts = std::max(1, (ng + gmax - 1) / gmax);
                 rest = std::max(rest, parts - 1);
                 if (pass >= parts) continue;
                 const int g0 = pass * gmax;
-                add(Part{q0, rows, 4 * g0, std::min(gmax, ng - g0), pass == parts - 1 ? 1 : 0, stage});
+                add(Part{q0, rows, (wide ? 128 : 4) * g0, std::min(gmax, ng - g0), pass == parts - 1 ? 1 : 0, stage, wide});
             }
         }
     }
