@@ -89,6 +89,7 @@ SIGNATURES = {
     "bpf_ctx_kernel_time": (_I, [_P, _I, C.POINTER(_D), C.POINTER(C.c_longlong),
                                  C.POINTER(_D), C.POINTER(_D)]),
     "bpf_spmm": (_I, [_P, C.POINTER(CsrDesc), _I, _D, _P, _I, _D, _P, _I]),
+    "bpf_block_to_host": (_I, [_P, _I, _I, _P, _I, _P, _I]),
     "bpf_householder": (_I, [_P, _I, _I, _P, _I, _P, _I]),
     "bpf_householder_lapack": (_I, [_P, _I, _I, _P, _I, _P, _I, _P, _I]),
     "bpf_ilu0_create": (_I, [_P, C.POINTER(CsrDesc), _I, _I, C.POINTER(_P)]),

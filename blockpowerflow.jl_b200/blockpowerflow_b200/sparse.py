@@ -93,6 +93,18 @@ def ld(X) -> int:
     return max(1, X.stride(1) if p > 1 else n)
 
 
+def to_host(X, negate: bool = False) -> np.ndarray:
+    """A 2-D device block (or its negative) as a host array, in Fortran order if X is column-major."""
+    if X.dim() != 2 or (X.stride(0) != 1 and X.shape[0] > 1) or ld(X) < X.shape[0]:
+        S = X.cpu().numpy()
+        return np.negative(S, out=S) if negate else S
+    n, p = X.shape
+    out = np.empty((p, n)).T
+    ctx = _lib.context(X.device.index)
+    _lib.check(_lib.load().bpf_block_to_host(ctx, n, p, X.data_ptr(), ld(X), out.ctypes.data, int(negate)), ctx)
+    return out
+
+
 def mul(A: CuSparseMatrixCSR, X, alpha: float = 1.0, beta: float = 0.0, Y=None):
     """mul!(Y, A, X, alpha, beta) on the device (CSR SpMM)."""
     Xc = colmajor(X)

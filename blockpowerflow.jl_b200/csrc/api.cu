@@ -425,6 +425,9 @@ bpf_status bpf_ctx_destroy(bpf_ctx *ctx) {
         if (ctx->ev_b[i]) cudaEventDestroy(ctx->ev_b[i]);
     }
     if (ctx->hstream) cudaStreamDestroy(ctx->hstream);
+    for (cudaEvent_t ev : ctx->ev_stage)
+        if (ev) cudaEventDestroy(ev);
+    if (ctx->stage) cudaFreeHost(ctx->stage);
     for (int s = 0; s < WS_COUNT; s++)
         if (ctx->ws[s]) cudaFree(ctx->ws[s]);
     cudaFree(ctx->dstat);

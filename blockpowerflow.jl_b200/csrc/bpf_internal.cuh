@@ -91,6 +91,9 @@ struct bpf_ctx {
     std::vector<TimedLaunch> timed;
     bpf::DevStatus *dstat = nullptr;   // device
     bpf::DevStatus *hstat = nullptr;   // pinned host mirror
+    // pinned slots of bpf_block_to_host (32 MB, made on first use) and their events
+    double *stage = nullptr;
+    cudaEvent_t ev_stage[4] = {nullptr, nullptr, nullptr, nullptr};
     void *ws[bpf::WS_COUNT] = {};
     size_t ws_bytes[bpf::WS_COUNT] = {};
 };

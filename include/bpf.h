@@ -214,6 +214,12 @@ BPF_API bpf_status bpf_mlp_param_copy(bpf_mlp *mlp, int which, int grad, float *
 BPF_API bpf_status bpf_mlp_basis(bpf_mlp *mlp, int rank, unsigned long long seed, double *Z,
                                  int ldz);
 
+/* host (n x p, column-major, ld n; pageable or pinned) = X (device, ldx), or its negative: large
+ * blocks through pinned pieces and several host threads.  No counterpart in the reference (Array(X));
+ * the Newton caller brings its sensitivities back with it.  Waits for the context's stream. */
+BPF_API bpf_status bpf_block_to_host(bpf_ctx *ctx, int n, int p, const double *X, int ldx, double *host,
+                                     int negate);
+
 /* ---- sparse x dense block -------------------------------------------------------------- */
 /* Y = alpha*A*X + beta*Y: mul!(W, A, P) of src/block_gmres.jl:299 (CSR SpMM). */
 BPF_API bpf_status bpf_spmm(bpf_ctx *ctx, const bpf_csr_desc *A, int p, double alpha,

@@ -138,3 +138,20 @@ def test_dump_ingest_and_the_benchmark_solve(bpf, tmp_path):
     assert st2.niter <= 50 and np.isfinite(rn2)
     if st2.solved:
         assert rn2 <= 1e-9, rn2
+
+
+@pytest.mark.parametrize("n,p,ldx", [(1, 1, 1), (7, 3, 7), (5, 4, 9), (1 << 18, 1, 1 << 18), (40_000, 70, 40_000),
+                                     (40_001, 70, 40_003), (1_100_000, 2, 1_100_000), (1_100_000, 2, 1_100_001)])
+@pytest.mark.parametrize("negate", [False, True])
+def test_block_to_host(n, p, ldx, negate):
+    """Blocks below and above the staged size, contiguous or not, columns longer than a piece."""
+    import torch
+
+    from blockpowerflow_b200.sparse import to_host
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    X = torch.randn(p, ldx, dtype=torch.float64, device="cuda").t()[:n]
+    H = to_host(X, negate)
+    assert H.shape == (n, p) and (H.flags.f_contiguous or p == 1 or n == 1)
+    np.testing.assert_array_equal(H, -X.cpu().numpy() if negate else X.cpu().numpy())
