@@ -89,6 +89,7 @@ struct bpf_ctx {
     size_t event_next = 0;
     struct TimedLaunch { int kc; cudaEvent_t a, b; double bytes, flops; };
     std::vector<TimedLaunch> timed;
+    int arnoldi_epoch = 0;             // launches of arnoldi_step (its skip decision is kept by epoch)
     bpf::DevStatus *dstat = nullptr;   // device
     bpf::DevStatus *hstat = nullptr;   // pinned host mirror
     // pinned slots of bpf_block_to_host (32 MB, made on first use) and their events
@@ -231,12 +232,12 @@ __device__ __forceinline__ bool grid_barrier(DevStatus *ds, unsigned &gen) {
             long long it = 0;
             const long long lim = ds->wait_limit > 0 ? ds->wait_limit : kSpinLimit;
             while (ld_acquire_u32(&ds->bar_gen) == g) {
-                if (++it > lim || ld_relaxed_i32(&ds->err) != 0) {
+                if (++it > lim || ((it & 15) == 0 && ld_relaxed_i32(&ds->err) != 0)) {
                     ok = 0;
                     atomicCAS(&ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
                     break;
                 }
-                __nanosleep(64);
+                if (it > 32) __nanosleep(64);   // most barriers are over within a few polls
             }
         }
         gen = g + 1;

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "arnoldi.cuh"
 #include "bpf_internal.cuh"
 #include "dense.cuh"
 #include "prec.cuh"
@@ -340,10 +341,24 @@ static bpf_status block_gmres_impl(bpf_ctx *ctx, const bpf_csr_desc *A, int p, c
         printf("%5s  %5s  %7s  %5s\n", "pass", "k", "‖Rₖ‖", "timer");
         printf("%5d  %5d  %7.1e  %.2fs\n", 0, 0, hs.rnorm, now_s() - t0);
     }
+    // the Hessenberg update of iteration kk, on the second stream when overlapped
+    auto hessenberg = [&](int kk, const double *Cm) -> bpf_status {
+        if (!overlap) return launch_hess(ctx, p, kk, g.Rblk, g.HY, tau_cur, g.Z, Cm, st, hist, scr);
+        BPF_CUDA(ctx, cudaEventRecord(ctx->ev_a[kk & 1], ctx->stream));
+        BPF_CUDA(ctx, cudaStreamWaitEvent(ctx->hstream, ctx->ev_a[kk & 1], 0));
+        StreamSwap sw(ctx, ctx->hstream);
+        BPF_TRY(launch_hess(ctx, p, kk, g.Rblk, g.HY, tau_cur, g.Z, Cm, st, hist, scr));
+        BPF_CUDA(ctx, cudaEventRecord(ctx->ev_b[kk & 1], ctx->hstream));
+        last_hess = kk;
+        return BPF_SUCCESS;
+    };
     int npass = 0, iter = 0, inner_itmax = itmax;
     bool solved = hs.solved != 0, tired = iter >= itmax, overtimed = false;
     int printed = 1;
-    const int chunk = restart ? memory : 16;
+    // narrow blocks without a deflation basis: the orthogonalization of an iteration in one launch
+    const bool one_launch = dfl.r == 0 && arnoldi_ok(ctx, n, p);
+    // iterations between looks at the stopping test: those past the stop are launches for nothing
+    const int chunk = std::min(restart ? memory : 16, one_launch ? 8 : 16);
     std::vector<double> hbuf;
 
     while (!(solved || tired || overtimed)) {
@@ -376,7 +391,9 @@ static bpf_status block_gmres_impl(bpf_ctx *ctx, const bpf_csr_desc *A, int p, c
             // allocation (and no implicit synchronisation) happens between launches.
             double *Psi2buf = (double *)ws_get(ctx, WS_I32, sizeof(double) * pp * kend, &s);
             if (!Psi2buf) return s;
-            if (!ws_get(ctx, WS_PARTIAL, sizeof(double) * pp * ((size_t)ctx->num_sms * 4 + kend + 1), &s))
+            if (!ws_get(ctx, WS_PARTIAL,
+                        sizeof(double) * std::max(pp * ((size_t)ctx->num_sms * 4 + kend + 1),
+                                                  one_launch ? arnoldi_partials(ctx, n, p, kend) : 0), &s))
                 return s;
             for (int kk = k + 1; kk <= kend; kk++) {
                 const int jj = kk - 1;
@@ -395,6 +412,15 @@ static bpf_status block_gmres_impl(bpf_ctx *ctx, const bpf_csr_desc *A, int p, c
                     Qk = Qm;
                 }
                 double *Psi = g.Rblk + rblk_pos(0, jj) * pp;                     // :301-313
+                double *Cm = Cpar[kk & 1];
+                // Cpar[kk & 1] was last read by the Hessenberg update of iteration kk - 2
+                if (overlap && kk >= 3)
+                    BPF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_b[kk & 1], 0));
+                if (one_launch) {
+                    BPF_TRY(arnoldi_step(ctx, n, p, kk, g.V, np, Qk, Vn, Psi, Psi2buf, Cm, st));
+                    BPF_TRY(hessenberg(kk, Cm));
+                    continue;
+                }
                 double *Ek = dfl.r > 0 ? dfl.E + (size_t)jj * pp : nullptr;
                 if (Ek) {   // against Q_C first (GCRO): E_k = Q_C^T W, W -= Q_C E_k
                     BPF_TRY(gram(ctx, n, p, 1, dfl.Qp, 0, Qk, Ek, 1.0, false, st));
@@ -408,10 +434,6 @@ static bpf_status block_gmres_impl(bpf_ctx *ctx, const bpf_csr_desc *A, int p, c
                 }
                 BPF_TRY(gram(ctx, n, p, kk, g.V, np, Qk, Psi, 1.0, true, st, nullptr, Psi2buf));
                 BPF_TRY(tsmm(ctx, n, p, kk, g.V, np, Psi2buf, pp, -1.0, Qk, 1.0, Qk, st));
-                double *Cm = Cpar[kk & 1];
-                // Cpar[kk & 1] was last read by the Hessenberg update of iteration kk - 2
-                if (overlap && kk >= 3)
-                    BPF_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->ev_b[kk & 1], 0));
                 BPF_TRY(cholqr(ctx, n, p, Qk, Vn, Cm, Tq, st, nullptr, &st->qr_shift,
                                &st->qr_reorth, kk));                         // :316
                 // Ill-conditioned block (Cholesky lost > 8 digits): its Q may carry amplified
@@ -425,16 +447,7 @@ static bpf_status block_gmres_impl(bpf_ctx *ctx, const bpf_csr_desc *A, int p, c
                     BPF_TRY(cholqr(ctx, n, p, Qk, Vn, C2, Tq, st, rg, &st->qr_shift2, nullptr, kk));
                     BPF_TRY(reorth_fold(ctx, p, kk, Psi, Psi2buf, Cm, C2, Cm, fold_scr, st, rg));
                 }
-                if (overlap) {
-                    BPF_CUDA(ctx, cudaEventRecord(ctx->ev_a[kk & 1], ctx->stream));
-                    BPF_CUDA(ctx, cudaStreamWaitEvent(ctx->hstream, ctx->ev_a[kk & 1], 0));
-                    StreamSwap sw(ctx, ctx->hstream);
-                    BPF_TRY(launch_hess(ctx, p, kk, g.Rblk, g.HY, tau_cur, g.Z, Cm, st, hist, scr));
-                    BPF_CUDA(ctx, cudaEventRecord(ctx->ev_b[kk & 1], ctx->hstream));
-                    last_hess = kk;
-                } else {
-                    BPF_TRY(launch_hess(ctx, p, kk, g.Rblk, g.HY, tau_cur, g.Z, Cm, st, hist, scr));
-                }
+                BPF_TRY(hessenberg(kk, Cm));
             }
             k = kend;
             BPF_TRY(join());

@@ -1,0 +1,65 @@
+"""block_gmres with the orthogonalization in one launch, at the edges of its tiles and groups.
+
+The basis is checked through what it must give: the CPU oracle's iteration count, and a solution whose
+true residual ||B - A X|| agrees with the solver's own estimate.  The estimate is exact in exact
+arithmetic; with an orthonormal basis to a few eps the two differ by k eps kappa ||B||, far below the
+tolerance of 1e-2 of the stopping bound at rtol 1e-8.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def bpf():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import blockpowerflow_b200 as bpf
+
+    return bpf
+
+
+def _solve(bpf, A, B, **kw):
+    import torch
+
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    N = bpf.ilu0(Ad, B.shape[1])
+    X, st = bpf.block_gmres(Ad, torch.as_tensor(B, device="cuda"), N=N, ldiv=True, atol=0.0, rtol=1e-8,
+                            history=True, **kw)
+    return X.cpu().numpy(), st
+
+
+# column counts at the edges of the 8-wide tiles; rows: a short last slab, one slab, and more
+# rows than SMs x 16 (slabs of 24 rows); 33 columns go by the kernels for wider blocks
+@pytest.mark.parametrize("nbus,p", [(20, 1), (40, 7), (300, 8), (300, 9), (300, 16), (301, 17), (300, 24),
+                                    (300, 25), (300, 31), (300, 32), (300, 33), (1400, 5), (1700, 32)])
+def test_edges(bpf, nbus, p):
+    A = bpf.grid.synthetic_jacobian(nbus, seed=nbus)
+    B = np.random.default_rng(p).standard_normal((A.shape[0], p))
+    X, st = _solve(bpf, A, B, memory=60)
+    _, so = O.block_gmres(A, B, N=(1, O.ilu0(A)), memory=60, atol=0.0, rtol=1e-8, history=True)
+    assert st.solved and abs(st.niter - so.niter) <= 1
+    nb = np.linalg.norm(B)
+    assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= 1e-2 * 1e-8 * nb
+
+
+def test_more_blocks_than_a_group(bpf):
+    """80 blocks of 32 columns: products go in groups of 64 blocks.  Unpreconditioned and not converged:
+    estimate and true residual differ by rounding, at most 10 k eps ||A|| ||X|| + 10 k eps ||B||."""
+    import torch
+
+    A = bpf.grid.synthetic_jacobian(1700, seed=3)
+    p, k = 32, 80
+    B = np.random.default_rng(3).standard_normal((A.shape[0], p))
+    X, st = bpf.block_gmres(bpf.CuSparseMatrixCSR.from_scipy(A), torch.as_tensor(B, device="cuda"), memory=k, itmax=k,
+                            atol=0.0, rtol=1e-14, history=True)
+    X = X.cpu().numpy()
+    assert st.niter == k
+    bound = 10 * k * 2.0**-52 * (np.sqrt((A.multiply(A)).sum()) * np.linalg.norm(X) + np.linalg.norm(B))
+    assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= bound
+    assert bound < 0.1 * st.residuals[-1]
