@@ -518,6 +518,11 @@ const char *bpf_solve_status_string(int status) {
     }
 }
 
+static bool blocks_disjoint(int n, int p, const double *X, int ldx, const double *Y, int ldy) {
+    const double *xe = X + (size_t)(p - 1) * ldx + n, *ye = Y + (size_t)(p - 1) * ldy + n;
+    return xe <= Y || ye <= X;
+}
+
 bpf_status bpf_spmm(bpf_ctx *ctx, const bpf_csr_desc *A, int p, double alpha, const double *X,
                     int ldx, double beta, double *Y, int ldy) {
     if (!ctx) return BPF_ERR_INVALID_VALUE;
@@ -528,22 +533,11 @@ bpf_status bpf_spmm(bpf_ctx *ctx, const bpf_csr_desc *A, int p, double alpha, co
     if (ldx < std::max(1, n) || ldy < std::max(1, n))
         return set_error(ctx, BPF_ERR_DIMENSION, "bpf_spmm: leading dimension < n");
     if (n == 0 || p == 0) return BPF_SUCCESS;
-    bpf_status st;
-    const int chunk = 256;
-    size_t cols = std::min(p, chunk);
-    double *xr = (double *)ws_get(ctx, WS_A, sizeof(double) * (size_t)n * cols, &st);
-    if (!xr) return st;
-    double *yr = (double *)ws_get(ctx, WS_B, sizeof(double) * (size_t)n * cols, &st);
-    if (!yr) return st;
-    for (int c0 = 0; c0 < p; c0 += chunk) {
-        int pc = std::min(chunk, p - c0);
-        BPF_TRY(colmajor_to_rowmajor(ctx, n, pc, X + (size_t)c0 * ldx, ldx, xr));
-        if (beta != 0.0) BPF_TRY(colmajor_to_rowmajor(ctx, n, pc, Y + (size_t)c0 * ldy, ldy, yr));
-        BPF_TRY(spmm_rowmajor(ctx, n, A->nnz, A->rowptr, A->colind, (const double *)A->vals, A->index_base,
-                              pc, alpha, xr, beta, yr, nullptr));
-        BPF_TRY(rowmajor_to_colmajor(ctx, n, pc, yr, Y + (size_t)c0 * ldy, ldy));
-    }
-    return BPF_SUCCESS;
+    const BlockOverlap ov = blocks_disjoint(n, p, X, ldx, Y, ldy) ? BlockOverlap::kNone
+                            : X == Y && ldx == ldy                ? BlockOverlap::kSame
+                                                                  : BlockOverlap::kPart;
+    return spmm_colmajor(ctx, n, A->nnz, A->rowptr, A->colind, (const double *)A->vals, A->index_base, p, alpha, X, ldx,
+                         beta, Y, ldy, ov);
 }
 
 static bpf_status prec_create(bpf_ctx *ctx, const bpf_csr_desc *A, int nrhs, int fdtype,
@@ -644,11 +638,6 @@ bpf_status bpf_prec_refactor(bpf_prec *P, const double *vals) {
     }
     BPF_TRY(prec_factor(ctx, P, vals));
     return check_dev_status(ctx, P->kind == PREC_IC0 ? "ic0 refactor" : "ilu0 refactor");
-}
-
-static bool blocks_disjoint(int n, int p, const double *X, int ldx, const double *Y, int ldy) {
-    const double *xe = X + (size_t)(p - 1) * ldx + n, *ye = Y + (size_t)(p - 1) * ldy + n;
-    return xe <= Y || ye <= X;
 }
 
 bpf_status bpf_prec_apply(bpf_prec *P, int p, const double *X, int ldx, double *Y, int ldy) {

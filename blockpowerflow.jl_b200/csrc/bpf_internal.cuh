@@ -267,6 +267,11 @@ bpf_status rowmajor_to_colmajor(bpf_ctx *ctx, int n, int p, const double *src, d
 bpf_status spmm_rowmajor(bpf_ctx *ctx, int n, long long nnz, const int *rp, const int *ci,
                          const double *av, int base, int p, double alpha, const double *X,
                          double beta, double *Y, const double *B, const int *gate = nullptr);
+// Y = alpha*A*X + beta*Y on column-major blocks.  Blocks that share memory are read before they are
+// written: a column group at a time if X and Y are the same block, 256 columns at a time otherwise.
+enum class BlockOverlap { kNone, kSame, kPart };
+bpf_status spmm_colmajor(bpf_ctx *ctx, int n, long long nnz, const int *rp, const int *ci, const double *av, int base,
+                         int p, double alpha, const double *X, int ldx, double beta, double *Y, int ldy, BlockOverlap ov);
 // Same with an FP32 input block (mixed-precision path): Y = A*X.
 bpf_status spmm_rowmajor_f32x(bpf_ctx *ctx, int n, long long nnz, const int *rp, const int *ci,
                               const double *av, int base, int p, const float *X, double *Y,

@@ -218,6 +218,187 @@ bpf_status spmm_rowmajor_f32x(bpf_ctx *ctx, int n, long long nnz, const int *rp,
 }
 
 // ------------------------------------------------------------------------------------
+// The product on column-major blocks (bpf_spmm)
+// ------------------------------------------------------------------------------------
+// Few columns, or a small product: straight from the columns, a thread per row holding CPT of them.
+// A gathered value costs a 32-byte sector, but there is one launch and no copy of X.  Eight entries'
+// loads in flight a thread; products and summation order as spmm_rm_kernel.
+template <int CPT>
+__global__ void __launch_bounds__(128)
+spmm_cm_kernel(int n, const int *__restrict__ rp, const int *__restrict__ ci, const double *__restrict__ av, int base,
+               int p, double alpha, const double *__restrict__ X, int ldx, double beta, double *__restrict__ Y, int ldy) {
+    const int row = blockIdx.x * 128 + threadIdx.x;
+    if (row >= n) return;
+    const int rs = __ldg(rp + row) - base, re = __ldg(rp + row + 1) - base;
+    for (int c0 = blockIdx.y * CPT; c0 < p; c0 += gridDim.y * CPT) {
+        const double *Xc = X + (size_t)c0 * ldx;
+        const int pc = min(CPT, p - c0);
+        double acc[CPT];
+#pragma unroll
+        for (int j = 0; j < CPT; j++) acc[j] = 0.0;
+        for (int k = rs; k < re; k += 8) {
+            int c[8];
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                c[u] = k + u < re ? __ldg(ci + k + u) - base : 0;
+                v[u] = k + u < re ? __ldg(av + k + u) : 0.0;
+            }
+            double x[8][CPT];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int j = 0; j < CPT; j++) x[u][j] = k + u < re && j < pc ? __ldg(Xc + (size_t)j * ldx + c[u]) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int j = 0; j < CPT; j++)
+                    if (k + u < re) acc[j] += v[u] * x[u][j];
+        }
+#pragma unroll
+        for (int j = 0; j < CPT; j++)
+            if (j < pc) {
+                double *y = Y + (size_t)(c0 + j) * ldy + row;
+                double v = alpha * acc[j];
+                if (beta != 0.0) v += beta * *y;
+                *y = v;
+            }
+    }
+}
+
+// X (column-major) into panels of W columns: panel q holds n rows of w doubles (the last panel's rows may be
+// narrower; w even, a pad column is zero).  64 rows of one panel a CTA.
+template <int W>
+__global__ void __launch_bounds__(256)
+cm_to_panels_kernel(int n, int p, const double *__restrict__ src, int ld, double *__restrict__ dst) {
+    constexpr int R = 64;
+    __shared__ double tile[W][R + 1];
+    const int r0 = blockIdx.x * R, c0 = blockIdx.y * W;
+    const int pc = min(W, p - c0), w = (pc + 1) & ~1, nr = min(R, n - r0);
+    const int x = threadIdx.x % R;
+#pragma unroll
+    for (int q = 0; q < W * R / 256; q++) {
+        const int c = threadIdx.x / R + 256 / R * q;
+        if (c < w) tile[c][x] = c < pc && x < nr ? src[(size_t)(c0 + c) * ld + r0 + x] : 0.0;
+    }
+    __syncthreads();
+    double *d = dst + (size_t)c0 * n + (size_t)r0 * w;
+    if (w == W)
+        for (int e = threadIdx.x; e < nr * W; e += 256) d[e] = tile[e % W][e / W];
+    else
+        for (int e = threadIdx.x; e < nr * w; e += 256) d[e] = tile[e % w][e / w];
+}
+
+// Y = alpha A X + beta Y from panels of X, Y column-major: G lanes a row, two columns a lane, so an entry
+// gathers one contiguous row of the panel; the CTA's tile of Y turns in shared memory.  Summation order as
+// spmm_rm_kernel.  Bound: the gathers from L2 (1 GB at 70000 buses x 128 columns, 6-7 TB/s); many warps with
+// few loads each carry them best: 32 registers and 64 warps an SM 165 us, eight loads in flight a lane at 48-64
+// registers 190-230 us, entries staged in shared memory 230 us.
+template <int G>
+__global__ void __launch_bounds__(256)
+spmm_panel_kernel(int n, const int *__restrict__ rp, const int *__restrict__ ci, const double *__restrict__ av, int base,
+                  int p, double alpha, const double *__restrict__ XP, double beta, double *__restrict__ Y, int ldy) {
+    constexpr int NG = 256 / G, ROWS = NG > 32 ? NG : 32, W = 2 * G;
+    __shared__ double tile[W][ROWS + 1];
+    const int lane = threadIdx.x & 31, gl = lane % G, grp = threadIdx.x / G;
+    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (lane / G * G);
+    const int r0 = blockIdx.x * ROWS, c0 = blockIdx.y * W;
+    const int pc = min(W, p - c0), w2 = (pc + 1) / 2;
+    const double2 *Xp = reinterpret_cast<const double2 *>(XP + (size_t)c0 * n) + min(gl, w2 - 1);
+#pragma unroll 1
+    for (int lr = grp; lr < ROWS; lr += NG) {
+        const int row = r0 + lr;
+        double2 acc = make_double2(0.0, 0.0);
+        if (row < n) {
+            const int rs = __ldg(rp + row) - base, re = __ldg(rp + row + 1) - base;
+            for (int kb = rs; kb < re; kb += G) {
+                const int k = kb + gl;
+                int c = 0;
+                double a = 0.0;
+                if (k < re) {
+                    c = __ldg(ci + k) - base;
+                    a = __ldg(av + k);
+                }
+                const int cnt = min(G, re - kb);
+#pragma unroll 8
+                for (int t = 0; t < cnt; t++) {
+                    const int ct = __shfl_sync(gmask, c, t, G);
+                    const double at = __shfl_sync(gmask, a, t, G);
+                    const double2 v = __ldg(Xp + (size_t)ct * w2);
+                    acc.x += at * v.x;
+                    acc.y += at * v.y;
+                }
+            }
+        }
+        tile[2 * gl][lr] = acc.x;
+        tile[2 * gl + 1][lr] = acc.y;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < pc * ROWS; e += 256) {
+        const int c = e / ROWS, lr = e % ROWS;
+        if (r0 + lr < n) {
+            double *y = Y + (size_t)(c0 + c) * ldy + r0 + lr;
+            double v = alpha * tile[c][lr];
+            if (beta != 0.0) v += beta * *y;
+            *y = v;
+        }
+    }
+}
+
+// X into panels, then the product.
+template <int G>
+static bpf_status launch_spmm_panel(bpf_ctx *ctx, int n, long long nnz, const int *rp, const int *ci, const double *av,
+                                    int base, int p, double alpha, const double *X, int ldx, double *xp, double beta,
+                                    double *Y, int ldy) {
+    constexpr int W = 2 * G, ROWS = 256 / G > 32 ? 256 / G : 32;
+    cm_to_panels_kernel<W><<<dim3(ceil_div(n, 64), ceil_div(p, W)), 256, 0, ctx->stream>>>(n, p, X, ldx, xp);
+    BPF_LAUNCHED(ctx);
+    const double np = (double)n * p;
+    KScope ks(ctx, BPF_KC_SPMM, 12.0 * nnz + 4.0 * (n + 1) + 16.0 * np + (beta != 0.0 ? 8.0 * np : 0.0), 2.0 * nnz * p);
+    spmm_panel_kernel<G><<<dim3(ceil_div(n, ROWS), ceil_div(p, W)), 256, 0, ctx->stream>>>(n, rp, ci, av, base, p, alpha,
+                                                                                         xp, beta, Y, ldy);
+    BPF_LAUNCHED(ctx);
+    return BPF_SUCCESS;
+}
+
+bpf_status spmm_colmajor(bpf_ctx *ctx, int n, long long nnz, const int *rp, const int *ci, const double *av, int base,
+                         int p, double alpha, const double *X, int ldx, double beta, double *Y, int ldy, BlockOverlap ov) {
+    if (n == 0 || p == 0) return BPF_SUCCESS;
+    // Straight from the columns while its 32 bytes a gathered value cost less than the panels' copy and
+    // second launch.  Direct / panels, cold caches: 300 buses x 16 8.3 / 17.6 us, 9000 x 16 (1.9 M products)
+    // 16.4 / 17.4, 30000 x 5 (2.0 M) 20.4 / 19.5, 9000 x 33 (4.0 M) 24.6 / 25, 9000 x 64 38.9 / 27; one to four
+    // columns fill only a quarter of a panel row's sectors: 70000 x 3 22.6, x 8 43 / 32.
+    if (ov == BlockOverlap::kNone && (p <= 4 || (double)nnz * p <= 2e6)) {
+        const double np = (double)n * p;
+        KScope ks(ctx, BPF_KC_SPMM, 12.0 * nnz + 4.0 * (n + 1) + 16.0 * np + (beta != 0.0 ? 8.0 * np : 0.0), 2.0 * nnz * p);
+        // more columns a thread share its row's entries; fewer where threads are few
+        const int cpt = p == 1 ? 1 : p <= 2 || np < 32768 ? 2 : 4;
+        const auto kern = cpt == 1 ? spmm_cm_kernel<1> : cpt == 2 ? spmm_cm_kernel<2> : spmm_cm_kernel<4>;
+        kern<<<dim3(ceil_div(n, 128), std::min(ceil_div(p, cpt), 65535)), 128, 0, ctx->stream>>>(n, rp, ci, av, base, p, alpha,
+                                                                                                X, ldx, beta, Y, ldy);
+        BPF_LAUNCHED(ctx);
+        return BPF_SUCCESS;
+    }
+    const int chunk = 256;
+    bpf_status st;
+    double *xp = (double *)ws_get(ctx, WS_A, sizeof(double) * (size_t)n * ((std::min(p, chunk) + 1) & ~1), &st);
+    if (!xp) return st;
+    for (int c0 = 0; c0 < p; c0 += chunk) {
+        const int pc = std::min(chunk, p - c0);
+        // Panels of 64 columns (a warp a row) move the most bytes an instruction: 70000 buses x 128 columns 211
+        // us against 222 in panels of 32, 30000 x 128 90 against 97; less than a wave of such CTAs (9000 x 64)
+        // 31.7 against 27.3.  Narrower blocks take as many lanes a row as they fill.
+        const bool wave = (long long)ceil_div(n, 32) * ceil_div(pc, 64) >= 8LL * ctx->num_sms;
+        const auto launch = pc <= 8             ? launch_spmm_panel<4>
+                            : pc <= 16          ? launch_spmm_panel<8>
+                            : pc <= 32 || !wave ? launch_spmm_panel<16>
+                                                : launch_spmm_panel<32>;
+        BPF_TRY(launch(ctx, n, nnz, rp, ci, av, base, pc, alpha, X + (size_t)c0 * ldx, ldx, xp, beta, Y + (size_t)c0 * ldy, ldy));
+    }
+    return BPF_SUCCESS;
+}
+
+// ------------------------------------------------------------------------------------
 // layout conversions (32x32 tiles through shared memory)
 // ------------------------------------------------------------------------------------
 __global__ void cm_to_rm_kernel(int n, int p, const double *__restrict__ src, int ld,
