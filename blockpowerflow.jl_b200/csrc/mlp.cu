@@ -49,9 +49,11 @@ struct bpf_mlp {
     // activations and gradients of one batch (P = 128 samples)
     __nv_bfloat16 *Ub = nullptr, *Utb = nullptr, *A1b = nullptr, *A1tb = nullptr, *A2b = nullptr,
                   *A2tb = nullptr, *dYb = nullptr, *dYtb = nullptr, *dZb = nullptr, *dZtb = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr, *dA = nullptr;
+    float *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr;
+    int yslices = 1;          // K slices of the output product
+    float *colp = nullptr;    // hidden bias gradients, summed by 8 samples: 2 x 16 x H
+    double *norms = nullptr;  // parts of the squared column norms of B and X
     float *bn = nullptr;      // per-sample ||b||
-    float *tn = nullptr;      // per-sample ||t||^2
     double *loss = nullptr;   // device scalar
     int *err = nullptr;       // tensor-core pipeline error word
 };
@@ -61,141 +63,203 @@ namespace bpf {
 // ---------------------------------------------------------------------------------------
 // elementwise kernels
 // ---------------------------------------------------------------------------------------
-__global__ void col_norms_kernel(int n, int p, const double *__restrict__ B, int ldb, float *__restrict__ out) {
-    const int j = blockIdx.x;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double v = B[(size_t)j * ldb + i];
-        s += v * v;
+// Columns are summed in kNormParts parts (one CTA each: 64 CTAs, one a column, took 36 us for 9 MB), which the
+// reader adds in order: part[which][s][j], which 0: B, 1: X.
+constexpr int kNormParts = 8;
+__global__ void __launch_bounds__(256)
+col_norms_kernel(int n, const double *__restrict__ B, int ldb, const double *__restrict__ X, int ldx,
+                 double *__restrict__ part) {
+    const int j = blockIdx.x, s = blockIdx.y;
+    const double *V = blockIdx.z ? X + (size_t)j * ldx : B + (size_t)j * ldb;
+    const int len = (n + kNormParts - 1) / kNormParts, i1 = min(n, (s + 1) * len);
+    double t = 0.0;
+#pragma unroll 8
+    for (int i = s * len + threadIdx.x; i < i1; i += 256) {
+        const double v = __ldg(V + i);
+        t += v * v;
     }
-    __shared__ double red[32];
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __shared__ double red[8];
+    t = warp_sum(t);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) out[j] = (float)sqrt(t);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) t += red[w];
+        part[(blockIdx.z * kNormParts + s) * kMlpBatch + j] = t;
     }
+}
+
+__device__ __forceinline__ double norm_total(const double *part, int which, int j) {
+    double t = 0.0;
+#pragma unroll
+    for (int s = 0; s < kNormParts; s++) t += part[(which * kNormParts + s) * kMlpBatch + j];
+    return t;
 }
 
 // U[j][i] = b_ij / ||b_j|| (sample-major, BF16) and its transpose Ut[i][j]; zero padding for
-// i >= n and j >= p.
-__global__ void prep_input_kernel(int n, int np, int p, const double *__restrict__ B, int ldb,
-                                  const float *__restrict__ bn, __nv_bfloat16 *__restrict__ U,
-                                  __nv_bfloat16 *__restrict__ Ut) {
-    const size_t total = (size_t)np * kMlpBatch;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(e / np), i = (int)(e % np);
+// i >= n and j >= p.  A CTA turns a 64 x 64 tile in shared memory (straight from the columns the
+// transposed 2-byte stores were 23 us).  The first row of tiles stores ||b_j||.
+__global__ void __launch_bounds__(256)
+prep_input_kernel(int n, int np, int p, const double *__restrict__ B, int ldb, const double *__restrict__ part,
+                  float *__restrict__ bn, __nv_bfloat16 *__restrict__ U, __nv_bfloat16 *__restrict__ Ut) {
+    __shared__ float s_bn[64];
+    __shared__ __nv_bfloat16 tile[64][66];   // [i][j]
+    const int i0 = blockIdx.x * 64, j0 = blockIdx.y * 64, x = threadIdx.x & 63;
+    if (threadIdx.x < 64) {
+        const int j = j0 + x;
+        const float nb = j < p ? (float)sqrt(norm_total(part, 0, j)) : 0.f;
+        s_bn[x] = nb;
+        if (blockIdx.x == 0 && j < p) bn[j] = nb;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int jj = threadIdx.x >> 6; jj < 64; jj += 4) {
+        const int j = j0 + jj, i = i0 + x;
+        const float nb = s_bn[jj];
         float v = 0.f;
-        if (j < p && i < n) {
-            const float nb = bn[j];
-            v = nb > 0.f ? (float)(B[(size_t)j * ldb + i] / (double)nb) : 0.f;
-        }
+        if (j < p && i < n && nb > 0.f) v = (float)(B[(size_t)j * ldb + i] / (double)nb);
         const __nv_bfloat16 h = __float2bfloat16_rn(v);
         U[(size_t)j * np + i] = h;
-        Ut[(size_t)i * kMlpBatch + j] = h;
+        tile[x][jj] = h;
     }
+    __syncthreads();
+#pragma unroll 4
+    for (int ii = threadIdx.x >> 6; ii < 64; ii += 4) Ut[(size_t)(i0 + ii) * kMlpBatch + j0 + x] = tile[ii][x];
 }
 
-// Z (P x H) += bias; A = lrelu(Z) as BF16, sample-major and transposed; rows j >= p zero.
-__global__ void bias_act_kernel(int H, int p, float *__restrict__ Z, const float *__restrict__ bias,
-                                __nv_bfloat16 *__restrict__ A, __nv_bfloat16 *__restrict__ At) {
-    const int total = kMlpBatch * H;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const int j = e / H, c = e % H;
-        float z = 0.f, a = 0.f;
-        if (j < p) {
-            z = Z[e] + bias[c];
-            a = z > 0.f ? z : kLeak * z;
-        }
-        Z[e] = z;
-        const __nv_bfloat16 h = __float2bfloat16_rn(a);
-        A[e] = h;
-        At[(size_t)c * kMlpBatch + j] = h;
+// Sum of the K slices' products at element e: the last, which may be a short one, then the others in order.
+__device__ __forceinline__ float slices_total(const float *__restrict__ part, int splits, size_t slice, size_t e) {
+    float t = __ldcg(part + (splits - 1) * slice + e);
+#pragma unroll 16
+    for (int s = 0; s < splits - 1; s++) t += __ldcg(part + s * slice + e);
+    return t;
+}
+
+// Z (P x H) = the slices' sum + bias; A = lrelu(Z) as BF16, sample-major and transposed; rows j >= p
+// zero.  32 features x 8 samples a CTA.
+__global__ void __launch_bounds__(256)
+bias_act_kernel(int H, int p, const float *__restrict__ part, int splits, float *__restrict__ Z,
+                const float *__restrict__ bias, __nv_bfloat16 *__restrict__ A, __nv_bfloat16 *__restrict__ At) {
+    __shared__ __nv_bfloat16 tile[32][10];
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31), j0 = blockIdx.y * 8, jj = threadIdx.x >> 5, j = j0 + jj;
+    const size_t e = (size_t)j * H + c;
+    float z = 0.f, a = 0.f;
+    if (j < p) {
+        z = slices_total(part, splits, (size_t)kMlpBatch * H, e) + bias[c];
+        a = z > 0.f ? z : kLeak * z;
     }
+    Z[e] = z;
+    const __nv_bfloat16 h = __float2bfloat16_rn(a);
+    A[e] = h;
+    tile[threadIdx.x & 31][jj] = h;
+    __syncthreads();
+    At[(size_t)(blockIdx.x * 32 + threadIdx.x / 8) * kMlpBatch + j0 + threadIdx.x % 8] = tile[threadIdx.x / 8][threadIdx.x % 8];
 }
 
 // y = Y + b3 (normalized output); forward only: X[i, j] = s ||b_j|| y_ji.
-__global__ void output_kernel(int n, int np, int p, const float *__restrict__ Y, const float *__restrict__ b3,
+__global__ void output_kernel(int n, int np, int p, const float *__restrict__ Y, int splits, const float *__restrict__ b3,
                               const float *__restrict__ bn, double scale, double *__restrict__ X, int ldx) {
     const size_t total = (size_t)p * n;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int j = (int)(e / n), i = (int)(e % n);
-        X[(size_t)j * ldx + i] = scale * (double)bn[j] * (double)(Y[(size_t)j * np + i] + b3[i]);
+        X[(size_t)j * ldx + i] = scale * (double)bn[j] * (double)(slices_total(Y, splits, (size_t)kMlpBatch * np, (size_t)j * np + i) + b3[i]);
     }
 }
 
-// tn[j] = ||t_j||^2 with t_j = x_j / (s ||b_j||)
-__global__ void target_norms_kernel(int n, const double *__restrict__ X, int ldx, const float *__restrict__ bn,
-                                    double scale, float *__restrict__ tn) {
-    const int j = blockIdx.x;
-    const double f = bn[j] > 0.f ? 1.0 / (scale * (double)bn[j]) : 0.0;
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double t = X[(size_t)j * ldx + i] * f;
-        s += t * t;
+// dY = 2 w_j (y - t), w_j = 1 / (p ||t_j||^2), t_j = x_j / (s ||b_j||); BF16 sample-major and transposed
+// (rows j >= p zero); the loss sum_j w_j ||y_j - t_j||^2 into *loss (atomic; cleared by the caller); the
+// output bias' gradient db3[i] = sum_j dY[j][i].  A CTA takes 32 rows and all samples, so that the
+// transposed tile and the sums over the samples stay in it (element by element, with the FP32 gradient
+// written and summed by another kernel: 47 us).
+__global__ void __launch_bounds__(256)
+loss_grad_kernel(int n, int np, int p, const float *__restrict__ Y, int splits, const float *__restrict__ b3,
+                 const double *__restrict__ X, int ldx, const float *__restrict__ bn, const double *__restrict__ part,
+                 double scale, __nv_bfloat16 *__restrict__ dY, __nv_bfloat16 *__restrict__ dYt, float *__restrict__ db3,
+                 double *loss) {
+    __shared__ double s_w[kMlpBatch], s_f[kMlpBatch];
+    __shared__ __nv_bfloat16 tile[32][kMlpBatch + 2];   // [i][j]
+    __shared__ float s_db[8][32];
+    const int i0 = blockIdx.x * 32, x = threadIdx.x & 31, i = i0 + x, jq = threadIdx.x >> 5;
+    if (threadIdx.x < kMlpBatch) {
+        const int j = threadIdx.x;
+        double w = 0.0, f = 0.0;
+        if (j < p && bn[j] > 0.f) {
+            f = scale * (double)bn[j];
+            const float tn = (float)(norm_total(part, 1, j) / (f * f));
+            w = tn > 0.f ? 1.0 / ((double)p * (double)tn) : 0.0;
+        }
+        s_w[j] = w;
+        s_f[j] = f;
     }
-    __shared__ double red[32];
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        t = warp_sum(t);
-        if (threadIdx.x == 0) tn[j] = (float)t;
-    }
-}
-
-// dY = 2 w_j (y - t), w_j = 1 / (p ||t_j||^2); BF16 sample-major and transposed; the loss
-// sum_j w_j ||y_j - t_j||^2 into *loss (atomic; cleared by the caller); rows j >= p zero.
-// Y and dYf may be the same buffer (each element is read before it is overwritten).
-__global__ void loss_grad_kernel(int n, int np, int p, const float *Y, const float *__restrict__ b3,
-                                 const double *__restrict__ X, int ldx, const float *__restrict__ bn,
-                                 const float *__restrict__ tn, double scale, __nv_bfloat16 *__restrict__ dY,
-                                 __nv_bfloat16 *__restrict__ dYt, float *dYf, double *loss) {
-    const size_t total = (size_t)np * kMlpBatch;
     double ls = 0.0;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(e / np), i = (int)(e % np);
+    float db = 0.f;
+    const float bias = b3[i];
+#pragma unroll 4
+    for (int j = jq; j < kMlpBatch; j += 8) {
         float g = 0.f;
         if (j < p && i < n) {
-            const double w = tn[j] > 0.f ? 1.0 / ((double)p * (double)tn[j]) : 0.0;
-            const double t = bn[j] > 0.f ? X[(size_t)j * ldx + i] / (scale * (double)bn[j]) : 0.0;
-            const double d = (double)(Y[e] + b3[i]) - t;
+            const double w = s_w[j], t = s_f[j] > 0.0 ? X[(size_t)j * ldx + i] / s_f[j] : 0.0;
+            const double d = (double)(slices_total(Y, splits, (size_t)kMlpBatch * np, (size_t)j * np + i) + bias) - t;
             ls += w * d * d;
             g = (float)(2.0 * w * d);
         }
-        dYf[e] = g;
+        db += g;
         const __nv_bfloat16 h = __float2bfloat16_rn(g);
-        dY[e] = h;
-        dYt[(size_t)i * kMlpBatch + j] = h;
+        dY[(size_t)j * np + i] = h;
+        tile[x][j] = h;
+    }
+    s_db[jq][x] = db;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        float t = 0.f;
+        for (int w = 0; w < 8; w++) t += s_db[w][x];
+        db3[i] = t;
+    }
+    for (int e = threadIdx.x; e < 32 * kMlpBatch / 2; e += 256) {
+        const int ii = e / (kMlpBatch / 2), j = 2 * (e % (kMlpBatch / 2));
+        __nv_bfloat162 h;
+        h.x = tile[ii][j];
+        h.y = tile[ii][j + 1];
+        *reinterpret_cast<__nv_bfloat162 *>(dYt + (size_t)(i0 + ii) * kMlpBatch + j) = h;
     }
     ls = warp_sum(ls);
     if ((threadIdx.x & 31) == 0 && ls != 0.0) atomicAdd(loss, ls);
 }
 
-// db[c] = sum_j G[j][c] over the batch (G: P x width, FP32)
-__global__ void col_sum_kernel(int width, const float *__restrict__ G, float *__restrict__ db) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < width; c += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int j = 0; j < kMlpBatch; j++) s += G[(size_t)j * width + c];
-        db[c] = s;
+// dZ = (the slices' sum) * lrelu'(Z) as BF16, sample-major and transposed, and its sums over each 8
+// samples: colp[j / 8][c].  32 features x 8 samples a CTA.
+__global__ void __launch_bounds__(256)
+act_back_kernel(int H, const float *__restrict__ Z, const float *__restrict__ part, int splits,
+                __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZt, float *__restrict__ colp) {
+    __shared__ __nv_bfloat16 tile[32][10];
+    __shared__ float s_sum[8][32];
+    const int c = blockIdx.x * 32 + (threadIdx.x & 31), j0 = blockIdx.y * 8, jj = threadIdx.x >> 5;
+    const size_t e = (size_t)(j0 + jj) * H + c;
+    const float g = slices_total(part, splits, (size_t)kMlpBatch * H, e) * (Z[e] > 0.f ? 1.f : kLeak);
+    const __nv_bfloat16 h = __float2bfloat16_rn(g);
+    dZ[e] = h;
+    tile[threadIdx.x & 31][jj] = h;
+    s_sum[jj][threadIdx.x & 31] = g;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        float t = 0.f;
+        for (int w = 0; w < 8; w++) t += s_sum[w][threadIdx.x];
+        colp[(size_t)blockIdx.y * H + c] = t;
     }
+    dZt[(size_t)(blockIdx.x * 32 + threadIdx.x / 8) * kMlpBatch + j0 + threadIdx.x % 8] = tile[threadIdx.x / 8][threadIdx.x % 8];
 }
 
-// dZ = dA * lrelu'(Z) (FP32 in dA, in place) and BF16 sample-major / transposed copies
-__global__ void act_back_kernel(int H, const float *__restrict__ Z, float *__restrict__ dA,
-                                __nv_bfloat16 *__restrict__ dZ, __nv_bfloat16 *__restrict__ dZt) {
-    const int total = kMlpBatch * H;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const int j = e / H, c = e % H;
-        const float g = dA[e] * (Z[e] > 0.f ? 1.f : kLeak);
-        dA[e] = g;
-        const __nv_bfloat16 h = __float2bfloat16_rn(g);
-        dZ[e] = h;
-        dZt[(size_t)c * kMlpBatch + j] = h;
-    }
+// The hidden biases' gradients from act_back_kernel's sums.
+__global__ void bias_grad_kernel(int H, const float *__restrict__ colp1, const float *__restrict__ colp2,
+                                 float *__restrict__ db1, float *__restrict__ db2) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2 * H) return;
+    const float *colp = e < H ? colp1 : colp2;
+    const int c = e < H ? e : e - H;
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < kMlpBatch / 8; q++) t += colp[(size_t)q * H + c];
+    (e < H ? db1 : db2)[c] = t;
 }
 
 // Adam on an FP32 master with bias correction.
@@ -239,55 +303,70 @@ static bpf_status mlp_refresh_bf16(bpf_mlp *m) {
     return BPF_SUCCESS;
 }
 
-// Forward pass of a batch of p <= 128 samples into m->Y (normalized outputs, without b3).
-static bpf_status mlp_forward_core(bpf_mlp *m, int p, const double *B, int ldb) {
+// Products of the K slices of a P x H result (kTcPartial) in the workspace.
+static bpf_status mlp_partial(bpf_mlp *m, int K, const void *A, const void *B, TcProduct *out) {
     bpf_ctx *ctx = m->ctx;
-    const int H = m->H, np = m->np, P = kMlpBatch;
-    col_norms_kernel<<<p, 256, 0, ctx->stream>>>(m->n, p, B, ldb, m->bn);
-    BPF_LAUNCHED(ctx);
-    prep_input_kernel<<<grid_for(ctx, (size_t)np * P), 256, 0, ctx->stream>>>(m->n, np, p, B, ldb, m->bn, m->Ub, m->Utb);
-    BPF_LAUNCHED(ctx);
-    BPF_TRY(tc_gemm_bf16_tn(ctx, P, H, np, m->Ub, np, m->W1b, np, m->Z1, H, false, m->err));
-    bias_act_kernel<<<grid_for(ctx, (size_t)P * H), 256, 0, ctx->stream>>>(H, p, m->Z1, m->b1.w, m->A1b, m->A1tb);
-    BPF_LAUNCHED(ctx);
-    BPF_TRY(tc_gemm_bf16_tn(ctx, P, H, H, m->A1b, H, m->W2b, H, m->Z2, H, false, m->err));
-    bias_act_kernel<<<grid_for(ctx, (size_t)P * H), 256, 0, ctx->stream>>>(H, p, m->Z2, m->b2.w, m->A2b, m->A2tb);
-    BPF_LAUNCHED(ctx);
-    BPF_TRY(tc_gemm_bf16_tn(ctx, P, np, H, m->A2b, H, m->W3b, H, m->Y, np, false, m->err));
+    TcProduct q = tc_product(ctx, kMlpBatch, m->H, K, A, K, B, K, nullptr, m->H);
+    bpf_status s;
+    q.D = (float *)ws_get(ctx, WS_PARTIAL, sizeof(float) * q.splits * q.slice, &s);
+    if (!q.D) return s;
+    q.mode = kTcPartial;
+    *out = q;
     return BPF_SUCCESS;
 }
 
-// Loss and gradients of a batch (into the params' g buffers); *loss_dev = L.
+// Forward pass of a batch of p <= 128 samples into m->Y (normalized outputs, without b3, as the products of
+// m->yslices K slices).  X (nullable): its
+// columns' norms are taken along.
+static bpf_status mlp_forward_core(bpf_mlp *m, int p, const double *B, int ldb, const double *X, int ldx) {
+    bpf_ctx *ctx = m->ctx;
+    const int H = m->H, np = m->np, P = kMlpBatch;
+    const dim3 act(H / 32, P / 8);
+    TcProduct q;
+    col_norms_kernel<<<dim3(p, kNormParts, X ? 2 : 1), 256, 0, ctx->stream>>>(m->n, B, ldb, X, ldx, m->norms);
+    BPF_LAUNCHED(ctx);
+    prep_input_kernel<<<dim3(np / 64, P / 64), 256, 0, ctx->stream>>>(m->n, np, p, B, ldb, m->norms, m->bn, m->Ub, m->Utb);
+    BPF_LAUNCHED(ctx);
+    BPF_TRY(mlp_partial(m, np, m->Ub, m->W1b, &q));
+    BPF_TRY(tc_gemm_group(ctx, q, nullptr, m->err));
+    bias_act_kernel<<<act, 256, 0, ctx->stream>>>(H, p, q.D, q.splits, m->Z1, m->b1.w, m->A1b, m->A1tb);
+    BPF_LAUNCHED(ctx);
+    BPF_TRY(mlp_partial(m, H, m->A1b, m->W2b, &q));
+    BPF_TRY(tc_gemm_group(ctx, q, nullptr, m->err));
+    bias_act_kernel<<<act, 256, 0, ctx->stream>>>(H, p, q.D, q.splits, m->Z2, m->b2.w, m->A2b, m->A2tb);
+    BPF_LAUNCHED(ctx);
+    q = tc_product(ctx, P, np, H, m->A2b, H, m->W3b, H, m->Y, np);
+    q.mode = kTcPartial;
+    return tc_gemm_group(ctx, q, nullptr, m->err);
+}
+
+// Loss and gradients of a batch (into the params' g buffers); *loss_dev = L.  The products that only a
+// weight's gradient needs run beside those of the chain.
 static bpf_status mlp_backward_core(bpf_mlp *m, int p, const double *X, int ldx) {
     bpf_ctx *ctx = m->ctx;
     const int H = m->H, np = m->np, P = kMlpBatch;
-    target_norms_kernel<<<p, 256, 0, ctx->stream>>>(m->n, X, ldx, m->bn, m->scale, m->tn);
-    BPF_LAUNCHED(ctx);
+    const dim3 act(H / 32, P / 8);
+    TcProduct q;
     BPF_CUDA(ctx, cudaMemsetAsync(m->loss, 0, sizeof(double), ctx->stream));
-    // dY (FP32 kept in Y's storage after use: the loss kernel reads Y[e] before writing dYf[e])
-    loss_grad_kernel<<<grid_for(ctx, (size_t)np * P), 256, 0, ctx->stream>>>(
-        m->n, np, p, m->Y, m->b3.w, X, ldx, m->bn, m->tn, m->scale, m->dYb, m->dYtb, m->Y, m->loss);
+    loss_grad_kernel<<<np / 32, 256, 0, ctx->stream>>>(m->n, np, p, m->Y, m->yslices, m->b3.w, X, ldx, m->bn, m->norms, m->scale,
+                                                       m->dYb, m->dYtb, m->b3.g, m->loss);
     BPF_LAUNCHED(ctx);
-    col_sum_kernel<<<grid_for(ctx, np), 256, 0, ctx->stream>>>(np, m->Y, m->b3.g);
+    // dA2 [P x H] = dY W3, dW3 [np x H] = dY^T A2
+    const TcProduct dW3 = tc_product(ctx, np, H, P, m->dYtb, P, m->A2tb, P, m->W3.g, H, 1);
+    BPF_TRY(mlp_partial(m, np, m->dYb, m->W3tb, &q));
+    BPF_TRY(tc_gemm_group(ctx, q, &dW3, m->err));
+    act_back_kernel<<<act, 256, 0, ctx->stream>>>(H, m->Z2, q.D, q.splits, m->dZb, m->dZtb, m->colp + 16 * (size_t)H);
     BPF_LAUNCHED(ctx);
-    // dW3 [np x H] = dY^T A2
-    BPF_TRY(tc_gemm_bf16_tn(ctx, np, H, P, m->dYtb, P, m->A2tb, P, m->W3.g, H, false, m->err));
-    // dA2 [P x H] = dY W3
-    BPF_TRY(tc_gemm_bf16_tn(ctx, P, H, np, m->dYb, np, m->W3tb, np, m->dA, H, false, m->err));
-    act_back_kernel<<<grid_for(ctx, (size_t)P * H), 256, 0, ctx->stream>>>(H, m->Z2, m->dA, m->dZb, m->dZtb);
-    BPF_LAUNCHED(ctx);
-    col_sum_kernel<<<grid_for(ctx, H), 256, 0, ctx->stream>>>(H, m->dA, m->b2.g);
-    BPF_LAUNCHED(ctx);
-    // dW2 [H x H] = dZ2^T A1
-    BPF_TRY(tc_gemm_bf16_tn(ctx, H, H, P, m->dZtb, P, m->A1tb, P, m->W2.g, H, false, m->err));
-    // dA1 [P x H] = dZ2 W2
-    BPF_TRY(tc_gemm_bf16_tn(ctx, P, H, H, m->dZb, H, m->W2tb, H, m->dA, H, false, m->err));
-    act_back_kernel<<<grid_for(ctx, (size_t)P * H), 256, 0, ctx->stream>>>(H, m->Z1, m->dA, m->dZb, m->dZtb);
-    BPF_LAUNCHED(ctx);
-    col_sum_kernel<<<grid_for(ctx, H), 256, 0, ctx->stream>>>(H, m->dA, m->b1.g);
+    // dA1 [P x H] = dZ2 W2, dW2 [H x H] = dZ2^T A1
+    const TcProduct dW2 = tc_product(ctx, H, H, P, m->dZtb, P, m->A1tb, P, m->W2.g, H, 1);
+    BPF_TRY(mlp_partial(m, H, m->dZb, m->W2tb, &q));
+    BPF_TRY(tc_gemm_group(ctx, q, &dW2, m->err));
+    act_back_kernel<<<act, 256, 0, ctx->stream>>>(H, m->Z1, q.D, q.splits, m->dZb, m->dZtb, m->colp);
     BPF_LAUNCHED(ctx);
     // dW1 [H x np] = dZ1^T U
-    BPF_TRY(tc_gemm_bf16_tn(ctx, H, np, P, m->dZtb, P, m->Utb, P, m->W1.g, np, false, m->err));
+    BPF_TRY(tc_gemm_group(ctx, tc_product(ctx, H, np, P, m->dZtb, P, m->Utb, P, m->W1.g, np, 1), nullptr, m->err));
+    bias_grad_kernel<<<ceil_div(2 * H, 256), 256, 0, ctx->stream>>>(H, m->colp, m->colp + 16 * (size_t)H, m->b1.g, m->b2.g);
+    BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;
 }
 
@@ -317,8 +396,8 @@ bpf_status bpf_mlp_destroy(bpf_mlp *m) {
     for (void *q : {(void *)m->W1b, (void *)m->W2b, (void *)m->W2tb, (void *)m->W3b, (void *)m->W3tb,
                     (void *)m->Ub, (void *)m->Utb, (void *)m->A1b, (void *)m->A1tb, (void *)m->A2b,
                     (void *)m->A2tb, (void *)m->dYb, (void *)m->dYtb, (void *)m->dZb, (void *)m->dZtb,
-                    (void *)m->Z1, (void *)m->Z2, (void *)m->Y, (void *)m->dA, (void *)m->bn,
-                    (void *)m->tn, (void *)m->loss, (void *)m->err})
+                    (void *)m->Z1, (void *)m->Z2, (void *)m->Y, (void *)m->colp, (void *)m->norms, (void *)m->bn,
+                    (void *)m->loss, (void *)m->err})
         cudaFree(q);
     delete m;
     return BPF_SUCCESS;
@@ -371,10 +450,11 @@ bpf_status bpf_mlp_create(bpf_ctx *ctx, int n, int hidden, unsigned long long se
     fa((void **)&m->dZtb, 2 * (size_t)P * H);
     fa((void **)&m->Z1, 4 * (size_t)P * H);
     fa((void **)&m->Z2, 4 * (size_t)P * H);
-    fa((void **)&m->Y, 4 * (size_t)P * np);
-    fa((void **)&m->dA, 4 * (size_t)P * H);
+    m->yslices = tc_product(ctx, P, np, H, nullptr, H, nullptr, H, nullptr, np).splits;
+    fa((void **)&m->Y, 4 * (size_t)P * np * m->yslices);
+    fa((void **)&m->colp, 4 * 2 * 16 * (size_t)H);
+    fa((void **)&m->norms, 8 * 2 * bpf::kNormParts * P);
     fa((void **)&m->bn, 4 * P);
-    fa((void **)&m->tn, 4 * P);
     fa((void **)&m->loss, sizeof(double));
     fa((void **)&m->err, sizeof(int) * 4);
     if (e != cudaSuccess) {
@@ -422,9 +502,9 @@ bpf_status bpf_mlp_forward(bpf_mlp *m, int p, const double *B, int ldb, double *
     BPF_CUDA(ctx, cudaMemsetAsync(m->err, 0, sizeof(int), ctx->stream));
     for (int j0 = 0; j0 < p; j0 += kMlpBatch) {
         const int pb = std::min(kMlpBatch, p - j0);
-        BPF_TRY(mlp_forward_core(m, pb, B + (size_t)j0 * ldb, ldb));
+        BPF_TRY(mlp_forward_core(m, pb, B + (size_t)j0 * ldb, ldb, nullptr, 0));
         output_kernel<<<grid_for(ctx, (size_t)pb * m->n), 256, 0, ctx->stream>>>(
-            m->n, m->np, pb, m->Y, m->b3.w, m->bn, m->scale, X + (size_t)j0 * ldx, ldx);
+            m->n, m->np, pb, m->Y, m->yslices, m->b3.w, m->bn, m->scale, X + (size_t)j0 * ldx, ldx);
         BPF_LAUNCHED(ctx);
     }
     return mlp_check_err(m);
@@ -438,7 +518,7 @@ bpf_status bpf_mlp_gradients(bpf_mlp *m, int p, const double *B, int ldb, const 
         return set_error(ctx, BPF_ERR_INVALID_VALUE, "mlp_gradients: 1 <= p <= %d", kMlpBatch);
     if (ldb < m->n || ldx < m->n) return set_error(ctx, BPF_ERR_DIMENSION, "mlp_gradients: leading dimension < n");
     BPF_CUDA(ctx, cudaMemsetAsync(m->err, 0, sizeof(int), ctx->stream));
-    BPF_TRY(mlp_forward_core(m, p, B, ldb));
+    BPF_TRY(mlp_forward_core(m, p, B, ldb, X, ldx));
     BPF_TRY(mlp_backward_core(m, p, X, ldx));
     if (loss) BPF_CUDA(ctx, cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     return mlp_check_err(m);

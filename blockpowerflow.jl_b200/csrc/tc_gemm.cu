@@ -6,11 +6,18 @@
 //  * operands reach shared memory by 16-byte cp.async in the canonical no-swizzle K-major
 //    UMMA layout -- 8-row x 16-byte core matrices, 128 contiguous bytes each; the two core
 //    matrices of one K = 16 instruction 128 bytes apart (leading byte offset), successive
-//    8-row groups 1024 bytes apart (stride byte offset) -- in a 4-stage ring of 64-wide K tiles;
+//    8-row groups 1024 bytes apart (stride byte offset) -- in a 3-stage ring of 64-wide K tiles
+//    (97 KB: two CTAs an SM, three where K is 128);
 //  * one thread issues the four tcgen05.mma (kind::f16, M = N = 128, K = 16) of a stage and
 //    commits them to the stage's mbarrier, which the ring waits on before overwriting it;
 //  * the accumulator lives in 128 TMEM columns; the epilogue reads it with tcgen05.ld
-//    (each warp its 32 lanes = 32 rows) and stores, or atomically adds for split-K.
+//    (each warp its 32 lanes = 32 rows), turns it in shared memory so that a row's 32 columns
+//    are one 128-byte store, and stores it -- to D, to the K slice's own partial block (the
+//    reader sums those), or atomically added to D (the public split-K form).
+//  * a launch takes up to two products, so that one with few tiles runs beside a large one.
+// A thread storing its own row, one 4-byte word at a time, wrote sectors piecemeal: the 17024 x
+// 512 weight gradient (35 MB out) took 63-72 us, as did 54 K slices adding to a 128 x 512
+// block atomically (47-55 us).
 // Every wait is bounded: on timeout the kernel records an error word, stops issuing, waits
 // (bounded) for its own MMAs, frees its TMEM and returns.
 //
@@ -32,10 +39,10 @@ namespace bpf {
 
 namespace {
 
-constexpr int kTM = 128, kTN = 128, kTK = 64, kStages = 4;
+constexpr int kTM = 128, kTN = 128, kTK = 64, kStages = 3;
 constexpr int kTileBytes = kTM * kTK * 2;                  // 16 KB per operand tile
 constexpr int kStageBytes = 2 * kTileBytes;                // A + B
-constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + 1024;   // + alignment slack
+constexpr int kEpiLd = 36;                                 // floats a row of the epilogue's tile
 
 __device__ __forceinline__ unsigned su32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -102,10 +109,13 @@ __device__ __forceinline__ void load_tile(unsigned dst, const __nv_bfloat16 *src
     }
 }
 
-__global__ void __launch_bounds__(128, 1)
-tc_gemm_bf16_tn_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, int lda,
-                       const __nv_bfloat16 *__restrict__ B, int ldb, float *__restrict__ D, int ldd,
-                       int k_per_slice, int mode, int *err) {
+__global__ void __launch_bounds__(128)
+tc_gemm_bf16_tn_kernel(TcGroup grp, int *err) {
+    const TcProduct &q = grp.q[blockIdx.x >= grp.second ? 1 : 0];
+    const int id = blockIdx.x >= grp.second ? blockIdx.x - grp.second : blockIdx.x;
+    const int M = q.M, N = q.N, K = q.K, lda = q.lda, ldb = q.ldb, ldd = q.ldd, mode = q.mode;
+    const __nv_bfloat16 *A = (const __nv_bfloat16 *)q.A, *B = (const __nv_bfloat16 *)q.B;
+    const int z = id / (q.mt * q.nt), mn = id - z * q.mt * q.nt;
     extern __shared__ __align__(1024) unsigned char tsm[];
     __shared__ __align__(8) uint64_t bar[kStages];
     __shared__ uint32_t s_tmem;
@@ -113,9 +123,10 @@ tc_gemm_bf16_tn_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
     __shared__ int s_issued;   // stages whose MMAs were committed
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const unsigned base = (su32(tsm) + 1023u) & ~1023u;
-    const int m0 = blockIdx.x * kTM, n0 = blockIdx.y * kTN;
-    const int kb = blockIdx.z * k_per_slice;
-    const int ke = min(K, kb + k_per_slice);
+    const int m0 = (mn % q.mt) * kTM, n0 = (mn / q.mt) * kTN;
+    const int kb = z * q.kps;
+    const int ke = min(K, kb + q.kps);
+    float *D = q.D + (mode == kTcPartial ? (size_t)z * q.slice : 0);
     const int nk = ke > kb ? (ke - kb) / kTK : 0;
     if (tid == 0) {
         s_fail = 0;
@@ -189,7 +200,8 @@ tc_gemm_bf16_tn_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
         if (tid == 0) atomicCAS(err, 0, 1);
     } else if (nk > 0) {
         // epilogue: warp w owns TMEM lanes (rows) 32w .. 32w+31
-        const int row = m0 + warp * 32 + lane;
+        float *et = reinterpret_cast<float *>(tsm + (base - su32(tsm))) + warp * 32 * kEpiLd;   // the ring is idle
+        const bool vec = ((ldd | N) & 3) == 0 && ((uintptr_t)D & 15) == 0;
 #pragma unroll 1
         for (int c0 = 0; c0 < kTN; c0 += 32) {
             uint32_t v[32];
@@ -204,14 +216,29 @@ tc_gemm_bf16_tn_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
                   "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < M) {
-                float *drow = D + (size_t)row * ldd + n0 + c0;
+            __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    if (n0 + c0 + j >= N) break;
-                    const float x = __uint_as_float(v[j]);
-                    if (mode == 0) drow[j] = x;
-                    else atomicAdd(drow + j, x);
+            for (int j = 0; j < 32; j += 4)
+                *reinterpret_cast<float4 *>(et + lane * kEpiLd + j) =
+                    make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
+                                __uint_as_float(v[j + 3]));
+            __syncwarp();
+            if (vec && mode != kTcAdd) {
+#pragma unroll
+                for (int r = lane >> 3; r < 32; r += 4) {
+                    const int row = m0 + warp * 32 + r, col = n0 + c0 + 4 * (lane & 7);
+                    if (row < M && col < N)
+                        *reinterpret_cast<float4 *>(D + (size_t)row * ldd + col) =
+                            *reinterpret_cast<const float4 *>(et + r * kEpiLd + 4 * (lane & 7));
+                }
+            } else if (n0 + c0 + lane < N) {
+                for (int r = 0; r < 32; r++) {
+                    const int row = m0 + warp * 32 + r;
+                    if (row >= M) break;
+                    float *d = D + (size_t)row * ldd + n0 + c0 + lane;
+                    const float x = et[r * kEpiLd + lane];
+                    if (mode == kTcAdd) atomicAdd(d, x);
+                    else *d = x;
                 }
             }
         }
@@ -222,31 +249,66 @@ tc_gemm_bf16_tn_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTN) : "memory");
 }
 
+TcProduct tc_product(const bpf_ctx *ctx, int M, int N, int K, const void *A, int lda, const void *B, int ldb, float *D,
+                     int ldd, int splits) {
+    TcProduct q{};
+    q.M = M;
+    q.N = N;
+    q.K = K;
+    q.A = A;
+    q.lda = lda;
+    q.B = B;
+    q.ldb = ldb;
+    q.D = D;
+    q.ldd = ldd;
+    q.mt = ceil_div(M, kTM);
+    q.nt = ceil_div(N, kTN);
+    if (splits <= 0) {   // enough K slices for two CTAs an SM, >= 4 tiles each
+        const int want = std::max(1, (2 * ctx->num_sms) / std::max(1, q.mt * q.nt));
+        splits = std::max(1, std::min(want, K / (4 * kTK)));
+    }
+    q.kps = ceil_div(ceil_div(K, splits), kTK) * kTK;
+    q.splits = ceil_div(K, q.kps);
+    q.slice = (size_t)M * ldd;
+    return q;
+}
+
+bpf_status tc_gemm_group(bpf_ctx *ctx, const TcProduct &a, const TcProduct *b, int *err_dev) {
+    TcGroup g;
+    g.q[0] = a;
+    g.q[1] = b ? *b : a;
+    g.second = a.mt * a.nt * a.splits;
+    int grid = g.second, tiles = 0;
+    double bytes = 0.0, flops = 0.0;
+    for (int i = 0; i < (b ? 2 : 1); i++) {
+        const TcProduct &q = g.q[i];
+        if (q.K % kTK || q.lda % 8 || q.ldb % 8 || ((uintptr_t)q.A & 15) || ((uintptr_t)q.B & 15))
+            return set_error(ctx, BPF_ERR_INVALID_VALUE,
+                             "tensor-core GEMM: K (%d) must be a multiple of 64, leading dimensions of 8, "
+                             "bases 16-byte aligned", q.K);
+        if (i) grid += q.mt * q.nt * q.splits;
+        tiles = std::max(tiles, std::min(q.K, q.kps) / kTK);
+        bytes += 2.0 * ((double)q.M * q.K + (double)q.N * q.K) + 4.0 * q.M * q.N;
+        flops += 2.0 * (double)q.M * q.N * q.K;
+    }
+    // a short K needs no more stages than it has tiles (the ring does not wrap), and more CTAs fit; two at
+    // least, which leaves three CTAs an SM within its 512 TMEM columns
+    const int smem = std::max(2, std::min(tiles, kStages)) * kStageBytes + 1024;
+    BPF_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_bf16_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    KScope ks(ctx, BPF_KC_MLP, bytes, flops);
+    tc_gemm_bf16_tn_kernel<<<grid, 128, smem, ctx->stream>>>(g, err_dev);
+    BPF_LAUNCHED(ctx);
+    return BPF_SUCCESS;
+}
+
 bpf_status tc_gemm_bf16_tn(bpf_ctx *ctx, int M, int N, int K, const void *A, int lda, const void *B,
                            int ldb, float *D, int ldd, bool accumulate, int *err_dev, int splits) {
     if (M <= 0 || N <= 0 || K <= 0) return BPF_SUCCESS;
-    if (K % kTK || lda % 8 || ldb % 8 || ((uintptr_t)A & 15) || ((uintptr_t)B & 15))
-        return set_error(ctx, BPF_ERR_INVALID_VALUE,
-                         "tensor-core GEMM: K (%d) must be a multiple of 64, leading dimensions of 8, "
-                         "bases 16-byte aligned", K);
-    const int mt = ceil_div(M, kTM), nt = ceil_div(N, kTN);
-    if (splits <= 0) {   // enough K slices to fill the SMs (one CTA per SM), >= 4 tiles each
-        const int want = std::max(1, (2 * ctx->num_sms) / std::max(1, mt * nt));
-        splits = std::max(1, std::min(want, K / (4 * kTK)));
-    }
-    int kps = ceil_div(ceil_div(K, splits), kTK) * kTK;
-    splits = ceil_div(K, kps);
-    const int mode = (accumulate || splits > 1) ? 1 : 0;
-    if (!accumulate && splits > 1)
+    TcProduct q = tc_product(ctx, M, N, K, A, lda, B, ldb, D, ldd, splits);
+    q.mode = (accumulate || q.splits > 1) ? kTcAdd : kTcStore;
+    if (!accumulate && q.splits > 1)
         BPF_CUDA(ctx, cudaMemsetAsync(D, 0, sizeof(float) * (size_t)ldd * M, ctx->stream));
-    BPF_CUDA(ctx, cudaFuncSetAttribute(tc_gemm_bf16_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kSmemBytes));
-    KScope ks(ctx, BPF_KC_MLP, 2.0 * ((double)M * K + (double)N * K) + 4.0 * M * N,
-              2.0 * (double)M * N * K);
-    tc_gemm_bf16_tn_kernel<<<dim3(mt, nt, splits), 128, kSmemBytes, ctx->stream>>>(
-        M, N, K, (const __nv_bfloat16 *)A, lda, (const __nv_bfloat16 *)B, ldb, D, ldd, kps, mode, err_dev);
-    BPF_LAUNCHED(ctx);
-    return BPF_SUCCESS;
+    return tc_gemm_group(ctx, q, nullptr, err_dev);
 }
 
 }  // namespace bpf
