@@ -1,4 +1,4 @@
-// One block-Arnoldi orthogonalization in one launch (blocks of up to 32 columns).
+// One block-Arnoldi orthogonalization in one launch (blocks of up to 64 columns).
 //
 // Reference: src/block_gmres.jl:301-316 (block Gram-Schmidt against the basis, QR of the new block).
 //
@@ -18,12 +18,14 @@
 // Same algorithm and decisions as gram / tsmm / cholqr / reorth_fold (dense.cu, small.cu); the sums are
 // grouped differently, so results agree to rounding.
 //
-// Measured, a whole solve per iteration, kernel by kernel -> one launch: 300 buses 8 columns 418 -> 119 us,
-// 24 columns 560 -> 189; 1500 buses 16 columns 599 -> 173; 9000 buses 8 columns 1981 -> 410 (long basis), 32
-// columns 1436 -> 742; 70000 buses 8 columns 2258 -> 1057.  With few columns now bound by the latency of a
-// product's 100 to 200 basis blocks a warp at a time, with 32 by HBM and the tensor pipe in turn (13 TFLOP/s).
-// Loads one step ahead and as pairs of columns, coefficients in shared memory, the update's order reversed and
-// four lanes an element of a sum took 9000 buses 8 columns from 547 to 410 us, 32 columns from 926 to 742.
+// Measured, a whole solve per iteration, kernel by kernel -> one launch: 300 buses 8 columns 418 -> 114 us,
+// 24 columns 560 -> 174; 1500 buses 16 columns 599 -> 162; 3000 buses 64 columns 671 -> 514; 9000 buses 8 columns
+// 1981 -> 408 (long basis), 32 columns 1436 -> 687, 48 columns 1411 -> 963, 64 columns 1393 -> 1233 (the
+// projections there are gram and tsmm, qr_only); 70000 buses 8 columns 2258 -> 1030.  With few columns now bound by
+// the latency of a product's 100 to 200 basis blocks, with 32 by HBM and the tensor pipe in turn (14 TFLOP/s).
+// What counted, 9000 buses: loads one step ahead as pairs of columns, coefficients in shared memory, the update's
+// order reversed and four lanes an element of a sum, 8 columns 547 -> 410 us and 32 columns 926 -> 742; the
+// factorization in registers and R^{-1} applied on the tensor pipe, 32 columns 742 -> 687.
 #include <algorithm>
 
 #include "arnoldi.cuh"
@@ -46,6 +48,7 @@ struct ArnoldiArgs {
     SolveState *st;
     int *snap;           // the grid's decision to skip, by epoch
     int epoch;
+    int qr_only;
     DevStatus *ds;
 };
 
@@ -59,20 +62,35 @@ __device__ __forceinline__ void arn_dmma(double &d0, double &d1, double a, doubl
 
 // Blocks of coefficients that one step of the update takes.
 __host__ __device__ constexpr int arn_step(int nt) { return nt == 1 ? 4 : nt == 2 ? 3 : nt == 3 ? 2 : 1; }
+// Warps that share a row of tiles of W^T W.
+__host__ __device__ constexpr int arn_parts(int nt) { return kArnoldiWarps / nt; }
+// Doubles for partial results of warps (arn_parts x PT^2, or kArnoldiWarps x 8 PT) and two steps' coefficients.
 __host__ __device__ constexpr int arn_buf(int nt) {
-    const int pt = 8 * nt, warps = kArnoldiWarps * pt * pt, coef = 2 * arn_step(nt) * pt * (pt + 2);
+    const int pt = 8 * nt, coef = 2 * arn_step(nt) * pt * (pt + 2);
+    const int warps = arn_parts(nt) * pt * pt > kArnoldiWarps * 8 * pt ? arn_parts(nt) * pt * pt : kArnoldiWarps * 8 * pt;
     return warps > coef ? warps : coef;
+}
+// The Cholesky's matrix g and buf are not needed at the same time: they share memory.
+__host__ __device__ constexpr int arn_area(int nt) {
+    const int g = 8 * nt * (8 * nt + 1), bf = arn_buf(nt);
+    return ((g > bf ? g : bf) + 1) & ~1;
 }
 
 // The shared-memory pieces of a CTA.
 template <int NT>
 struct ArnoldiSmem {
     static constexpr int PT = 8 * NT, LW = PT + 4, LG = PT + 1;
-    double *w;      // rows x LW: the CTA's rows of the block
-    double *buf;    // arn_buf(NT): partial results of warps (kArnoldiWarps x PT^2 or 8 PT), or two steps' coefficients
-    double *g, *x, *r, *t;   // PT x LG: Gram matrix / R^{-T}, inverse, accumulated R, scratch
-    double *dref, *rs;
+    double *w;        // rows x LW: the CTA's rows of the block
+    double *buf;      // arn_buf(NT)
+    double *g;        // PT x LG: pivot rows, then R^{-1} (in buf's memory)
+    double *r, *t;    // PT x LG: accumulated R, scratch
+    double *rs;
 };
+
+__device__ __forceinline__ void cp_async16(double *dst, const double *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 
 // Two adjacent values of a row at column c (zero beyond p): one 16-byte load where rows are 16-byte aligned.
 template <bool EVEN>
@@ -87,15 +105,18 @@ __device__ __forceinline__ double2 arn_load2(const double *row, int c, int p, bo
     return v;
 }
 
-// Partial sums of V_j^T W over the CTA's rows, j < nb: part[j].  A warp per j; the next 4 U rows of V (of
-// this j or the warp's next) are on their way while these are multiplied.  Lane (g, t4) takes columns 16 mp
-// + 2 g + {0, 1} of row t4 as one load: the two are the same row of two tiles' A fragments.
+// Partial sums of V_j^T W over the CTA's rows, j < nb: part[j].  A warp per j (from 33 columns two, each half
+// of the product's rows); the next 4 U rows of V (of this j or the warp's next) are on their way while these are
+// multiplied.  Lane (g, t4) takes columns 16 mp + 2 g + {0, 1} of row t4 as one load: the two are the same row
+// of two tiles' A fragments.
 template <int NT, bool EVEN>
 __device__ __forceinline__ void arn_gram(const ArnoldiArgs &a, const ArnoldiSmem<NT> &s, int r0, const double *A, int nb,
                                          double *part) {
-    constexpr int LW = ArnoldiSmem<NT>::LW, U = NT == 1 ? 10 : NT == 2 ? 8 : 4, MP = (NT + 1) / 2;
+    constexpr int LW = ArnoldiSmem<NT>::LW, U = NT == 1 ? 10 : NT == 2 ? 8 : NT <= 4 ? 4 : 2;
+    constexpr int MH = NT > 4 ? 2 : 1, MP = (NT + 2 * MH - 1) / (2 * MH);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, p = a.p;
     const size_t pp = (size_t)p * p;
+    nb *= MH;   // j MH + half
     if (warp >= nb) return;
     double acc[2 * MP][NT][2];
 #pragma unroll
@@ -103,14 +124,15 @@ __device__ __forceinline__ void arn_gram(const ArnoldiArgs &a, const ArnoldiSmem
 #pragma unroll
         for (int ni = 0; ni < NT; ni++) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
     double2 cur[U][MP], nxt[U][MP];
+    const int c0 = 16 * MP * (warp % MH);   // kArnoldiWarps is a multiple of MH: a warp keeps its half
     auto load = [&](double2 (&v)[U][MP], int j, int k0) {
-        const double *Aj = A + (size_t)j * a.strideV;
+        const double *Aj = A + (size_t)(j / MH) * a.strideV;
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int lr = k0 + 4 * u, r = r0 + lr + t4;
             const bool ok = lr < a.rows && r < a.n;
 #pragma unroll
-            for (int mp = 0; mp < MP; mp++) v[u][mp] = arn_load2<EVEN>(Aj + (size_t)r * p, 16 * mp + 2 * g, p, ok);
+            for (int mp = 0; mp < MP; mp++) v[u][mp] = arn_load2<EVEN>(Aj + (size_t)r * p, c0 + 16 * mp + 2 * g, p, ok);
         }
     };
     load(cur, warp, 0);
@@ -142,8 +164,8 @@ __device__ __forceinline__ void arn_gram(const ArnoldiArgs &a, const ArnoldiSmem
                 for (int ni = 0; ni < NT; ni++)
 #pragma unroll
                     for (int i = 0; i < 2; i++) {
-                        const int row = 16 * (mi / 2) + 2 * g + (mi & 1), col = 8 * ni + 2 * t4 + i;
-                        if (row < p && col < p) part[j * pp + (size_t)row * p + col] = acc[mi][ni][i];
+                        const int row = c0 + 16 * (mi / 2) + 2 * g + (mi & 1), col = 8 * ni + 2 * t4 + i;
+                        if (row < p && col < p) part[(j / MH) * pp + (size_t)row * p + col] = acc[mi][ni][i];
                         acc[mi][ni][i] = 0.0;
                     }
         }
@@ -179,7 +201,7 @@ __device__ __forceinline__ void arn_update(const ArnoldiArgs &a, const ArnoldiSm
 #pragma unroll
                 for (int ni = 0; ni < NT; ni++) acc[q][ni][0] = acc[q][ni][1] = 0.0;
             double2 cur[JB][2][NT], nxt[JB][2][NT];
-            double sv[ES];
+            double sv[NT > 4 ? 1 : ES];
             auto load = [&](double2 (&v)[JB][2][NT], int j0) {   // blocks j0 .. j0 + JB - 1, those below 0 as zeros
 #pragma unroll
                 for (int jb = 0; jb < JB; jb++)
@@ -192,28 +214,43 @@ __device__ __forceinline__ void arn_update(const ArnoldiArgs &a, const ArnoldiSm
                         for (int kk = 0; kk < NT; kk++) v[jb][q][kk] = arn_load2<EVEN>(row, 8 * kk + 2 * t4, p, ok);
                     }
             };
-            auto load_s = [&](int j0) {
+            auto load_s = [&](int j0, double *b) {
+                if constexpr (NT > 4 && !EVEN) {
+                    for (int e = threadIdx.x; e < (int)pp; e += 256)
+                        b[(e / p) * LS + e % p] = __ldcg(S + j0 * (long long)pp + e);
+                } else if constexpr (NT > 4) {   // one block a step: straight to shared memory, not by L1
+                    for (int e = 2 * threadIdx.x; e < (int)pp; e += 512)
+                        cp_async16(b + (e / p) * LS + e % p, S + j0 * (long long)pp + e);
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                } else {
 #pragma unroll
-                for (int u = 0; u < ES; u++) {
-                    const int e = threadIdx.x + 256 * u, jb = e / (int)pp;
-                    sv[u] = jb < JB && j0 + jb >= 0 ? __ldcg(S + j0 * (long long)pp + e) : 0.0;
+                    for (int u = 0; u < ES; u++) {
+                        const int e = threadIdx.x + 256 * u, jb = e / (int)pp;
+                        sv[u] = jb < JB && j0 + jb >= 0 ? __ldcg(S + j0 * (long long)pp + e) : 0.0;
+                    }
                 }
             };
+            if (NT > 4) __syncthreads();   // the zeros are there
             load(cur, a.k - JB);
-            load_s(a.k - JB);
+            load_s(a.k - JB, sb);
             for (int j0 = a.k - JB, step = 0; j0 > -JB; j0 -= JB, step ^= 1) {
                 double *b = sb + step * JB * PT * LS;
-                __syncthreads();   // the readers of the step before last are done (and, first, the zeros are there)
+                if constexpr (NT > 4) {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                    __syncthreads();   // this step's coefficients; the other buffer's readers are done
+                } else {
+                    __syncthreads();   // the readers of the step before last are done (and, first, the zeros are there)
 #pragma unroll
-                for (int u = 0; u < ES; u++) {
-                    const int e = threadIdx.x + 256 * u, jb = e / (int)pp, x = e - jb * (int)pp;
-                    if (jb < JB) b[jb * PT * LS + (x / p) * LS + x % p] = sv[u];
+                    for (int u = 0; u < ES; u++) {
+                        const int e = threadIdx.x + 256 * u, jb = e / (int)pp, x = e - jb * (int)pp;
+                        if (jb < JB) b[jb * PT * LS + (x / p) * LS + x % p] = sv[u];
+                    }
                 }
                 if (j0 > 0) {
                     load(nxt, j0 - JB);
-                    load_s(j0 - JB);
+                    load_s(j0 - JB, sb + (step ^ 1) * JB * PT * LS);
                 }
-                __syncthreads();
+                if (NT <= 4) __syncthreads();
 #pragma unroll
                 for (int jb = 0; jb < JB; jb++)
 #pragma unroll
@@ -259,24 +296,25 @@ __device__ __forceinline__ void arn_update(const ArnoldiArgs &a, const ArnoldiSm
         for (int j = share; j < a.k; j += split) {
             const double *row = a.V + (size_t)j * a.strideV + (size_t)r * p, *Sj = S + j * pp;
             double2 av[NT];
-            double bv[2 * NT][NT];
 #pragma unroll
-            for (int kk = 0; kk < NT; kk++) {
-                av[kk] = arn_load2<EVEN>(row, 8 * kk + 2 * t4, p, r < a.n);
+            for (int kk = 0; kk < NT; kk++) av[kk] = arn_load2<EVEN>(row, 8 * kk + 2 * t4, p, r < a.n);
+            constexpr int HB = NT <= 4 ? 2 * NT : 2;   // k-steps whose coefficients are in flight
 #pragma unroll
-                for (int h = 0; h < 2; h++)
+            for (int k0 = 0; k0 < 2 * NT; k0 += HB) {
+                double bv[HB][NT];
+#pragma unroll
+                for (int h = 0; h < HB; h++)
 #pragma unroll
                     for (int ni = 0; ni < NT; ni++) {
-                        const int c = 8 * kk + 2 * t4 + h;
-                        bv[2 * kk + h][ni] = c < p && 8 * ni + g < p ? __ldcg(Sj + (size_t)c * p + 8 * ni + g) : 0.0;
+                        const int c = 8 * ((k0 + h) / 2) + 2 * t4 + (h & 1);
+                        bv[h][ni] = c < p && 8 * ni + g < p ? __ldcg(Sj + (size_t)c * p + 8 * ni + g) : 0.0;
                     }
+#pragma unroll
+                for (int h = 0; h < HB; h++)
+#pragma unroll
+                    for (int ni = 0; ni < NT; ni++)
+                        arn_dmma(acc[ni][0], acc[ni][1], h & 1 ? av[(k0 + h) / 2].y : av[(k0 + h) / 2].x, bv[h][ni]);
             }
-#pragma unroll
-            for (int kk = 0; kk < NT; kk++)
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-#pragma unroll
-                    for (int ni = 0; ni < NT; ni++) arn_dmma(acc[ni][0], acc[ni][1], h ? av[kk].y : av[kk].x, bv[2 * kk + h][ni]);
         }
 #pragma unroll
         for (int ni = 0; ni < NT; ni++)
@@ -344,6 +382,29 @@ __device__ __forceinline__ bool arn_project(const ArnoldiArgs &a, const ArnoldiS
     return true;
 }
 
+// r <- t r, both PT x PT upper triangular (no barrier at the end): a row of tiles a warp.
+template <int NT>
+__device__ __forceinline__ void arn_mul_r(const double *t, double *r) {
+    constexpr int LG = 8 * NT + 1;
+    const int lane = threadIdx.x & 31, mi = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    double acc[NT][2];
+#pragma unroll
+    for (int ni = 0; ni < NT; ni++) acc[ni][0] = acc[ni][1] = 0.0;
+    if (mi < NT) {
+        for (int ks = 2 * mi; ks < 2 * NT; ks++) {
+            const double v = t[(8 * mi + g) * LG + 4 * ks + t4];
+#pragma unroll
+            for (int ni = 0; ni < NT; ni++) arn_dmma(acc[ni][0], acc[ni][1], v, r[(4 * ks + t4) * LG + 8 * ni + g]);
+        }
+    }
+    __syncthreads();
+    if (mi < NT)
+#pragma unroll
+        for (int ni = 0; ni < NT; ni++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) r[(8 * mi + g) * LG + 8 * ni + 2 * t4 + i] = acc[ni][i];
+}
+
 // One pass of Cholesky-QR on the CTAs' rows: s.r <- R s.r (first: R).  0: done; 1: a barrier gave up; 2:
 // breakdown.  shift / ill: set when the pass needed the shift / lost more than eight digits.
 template <int NT>
@@ -352,35 +413,40 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
     constexpr int PT = ArnoldiSmem<NT>::PT, LW = ArnoldiSmem<NT>::LW, LG = ArnoldiSmem<NT>::LG;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, p = a.p, tid = threadIdx.x;
     const size_t pp = (size_t)p * p;
-    // W^T W of the CTA's rows: the rows over the warps, their results added in order
+    // W^T W of the CTA's rows: a row of tiles a warp, the rows of W in arn_parts, whose sums are added in order
     {
-        double acc[NT][NT][2];
+        constexpr int PARTS = arn_parts(NT);
+        const int mi = warp % NT, q = warp / NT;
+        if (q < PARTS) {
+            double acc[NT][2];
 #pragma unroll
-        for (int mi = 0; mi < NT; mi++)
+            for (int ni = 0; ni < NT; ni++) acc[ni][0] = acc[ni][1] = 0.0;
+#pragma unroll 2
+            for (int k0 = 4 * q; k0 < a.rows; k0 += 4 * PARTS) {
+                double v[NT];
 #pragma unroll
-            for (int ni = 0; ni < NT; ni++) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-        for (int k0 = 4 * warp; k0 < a.rows; k0 += 4 * kArnoldiWarps) {
-            double v[NT];
+                for (int ni = 0; ni < NT; ni++) v[ni] = s.w[(k0 + t4) * LW + 8 * ni + g];
+                const double m = s.w[(k0 + t4) * LW + 8 * mi + g];
 #pragma unroll
-            for (int ni = 0; ni < NT; ni++) v[ni] = s.w[(k0 + t4) * LW + 8 * ni + g];
-#pragma unroll
-            for (int mi = 0; mi < NT; mi++)
-#pragma unroll
-                for (int ni = 0; ni < NT; ni++) arn_dmma(acc[mi][ni][0], acc[mi][ni][1], v[mi], v[ni]);
-        }
-#pragma unroll
-        for (int mi = 0; mi < NT; mi++)
+                for (int ni = 0; ni < NT; ni++) arn_dmma(acc[ni][0], acc[ni][1], m, v[ni]);
+            }
 #pragma unroll
             for (int ni = 0; ni < NT; ni++)
 #pragma unroll
-                for (int i = 0; i < 2; i++)
-                    s.buf[(size_t)warp * PT * PT + (8 * mi + g) * PT + 8 * ni + 2 * t4 + i] = acc[mi][ni][i];
-        __syncthreads();
-        for (int e = tid; e < p * p; e += 256) {
-            double v = 0.0;
+                for (int i = 0; i < 2; i++) {
+                    const int row = 8 * mi + g, col = 8 * ni + 2 * t4 + i;
+                    if (PARTS > 1) s.buf[q * PT * PT + row * PT + col] = acc[ni][i];
+                    else if (row < p && col < p) a.part[blockIdx.x * pp + (size_t)row * p + col] = acc[ni][i];
+                }
+        }
+        if (PARTS > 1) {
+            __syncthreads();
+            for (int e = tid; e < p * p; e += 256) {
+                double v = 0.0;
 #pragma unroll
-            for (int q = 0; q < kArnoldiWarps; q++) v += s.buf[(size_t)q * PT * PT + (e / p) * PT + e % p];
-            a.part[blockIdx.x * pp + e] = v;
+                for (int u = 0; u < PARTS; u++) v += s.buf[u * PT * PT + (e / p) * PT + e % p];
+                a.part[blockIdx.x * pp + e] = v;
+            }
         }
     }
     if (!grid_barrier(a.ds, gen)) return 1;
@@ -399,30 +465,53 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
     for (int i = 0; i < p; i++) trace += s.t[i * LG + i];
     int fail = 0;
     bool illcond = false;
+    // Elimination on [G | I] with unscaled pivot rows, G = Lt D Lt^T, X = Lt^{-1}: G's upper triangle and X's lower
+    // one share a matrix of which a thread keeps rows a16 + 16 u and columns b16 + 16 v in registers; a step needs
+    // the pivot row only (its G part divided by the pivot are the factors), which its owners pass on: one barrier a
+    // step (some 200 cycles; with the matrices in shared memory a step of 64 columns took about 1 us).
+    constexpr int TT = (PT + 15) / 16;
+    const int a16 = tid >> 4, b16 = tid & 15;
+    double M[TT][TT];
+    double *prow = s.g;   // two pivot rows of PT
     for (int attempt = 0; attempt < 2; attempt++) {
         const double shift = attempt == 0 ? 0.0
                                           : 11.0 * ((double)a.n * p + (double)p * (p + 1)) * 1.1102230246251565e-16 * trace;
-        for (int e = tid; e < p * p; e += 256) {
-            const int i = e / p, j = e % p;
-            s.g[i * LG + j] = s.t[i * LG + j] + (i == j ? shift : 0.0);
-            s.x[i * LG + j] = i == j ? 1.0 : 0.0;
-        }
+#pragma unroll
+        for (int u = 0; u < TT; u++)
+#pragma unroll
+            for (int v = 0; v < TT; v++) {
+                const int i = a16 + 16 * u, c = b16 + 16 * v;
+                M[u][v] = i < p && c < p && c >= i ? s.t[i * LG + c] + (i == c ? shift : 0.0) : 0.0;
+                if (i == 0 && c < PT) prow[c] = M[u][v];
+            }
         __syncthreads();
         fail = 0;
-        // elimination on [G | I] with unscaled pivot rows: G = Lt D Lt^T, X = Lt^{-1}
         for (int j = 0; j < p; j++) {
-            const double d = s.g[j * LG + j], ref = s.t[j * LG + j] + shift;
+            const double *row = prow + (j & 1) * PT;
+            const double d = row[j], ref = s.t[j * LG + j] + shift;
             if (attempt == 0 && !(d >= 1e-8 * ref)) illcond = true;
             if (!(d > 1e-13 * ref) || !(d > 0.0)) {
                 fail = 1;
                 break;
             }
             const double dinv = 1.0 / d;
-            for (int e = tid; e < (p - j - 1) * p; e += 256) {
-                const int i = j + 1 + e / p, c = e % p;
-                const double f = s.g[j * LG + i] * dinv;
-                if (c >= i) s.g[i * LG + c] -= f * s.g[j * LG + c];
-                else if (c <= j) s.x[i * LG + c] -= f * s.x[j * LG + c];
+            double rv[TT];
+#pragma unroll
+            for (int v = 0; v < TT; v++) {
+                const int c = b16 + 16 * v;
+                rv[v] = c == j ? 1.0 : c < p ? row[c] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < TT; u++) {
+                const int i = a16 + 16 * u;
+                if (i <= j || i >= p) continue;
+                const double f = row[i] * dinv;
+#pragma unroll
+                for (int v = 0; v < TT; v++) {
+                    const int c = b16 + 16 * v;
+                    if (c >= i || c <= j) M[u][v] -= f * rv[v];
+                    if (i == j + 1 && c < PT) prow[((j + 1) & 1) * PT + c] = M[u][v];
+                }
             }
             __syncthreads();
         }
@@ -432,47 +521,46 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
     }
     if (ill) *ill = fail != 0 || illcond || shifted;
     if (fail) return 2;
-    for (int i = tid; i < p; i += 256) s.rs[i] = 1.0 / sqrt(s.g[i * LG + i]);
+#pragma unroll
+    for (int u = 0; u < TT; u++)
+        if (a16 == b16 && a16 + 16 * u < p) s.rs[a16 + 16 * u] = 1.0 / sqrt(M[u][u]);
     __syncthreads();
-    // t = R, g = R^{-1}; then r = R r
-    for (int e = tid; e < p * p; e += 256) {
-        const int i = e / p, j = e % p;
-        s.t[i * LG + j] = j >= i ? s.g[i * LG + j] * s.rs[i] : 0.0;
-    }
+    // t = R, g = R^{-1} (zero below the diagonal and beyond p); then r = R r
+#pragma unroll
+    for (int u = 0; u < TT; u++)
+#pragma unroll
+        for (int v = 0; v < TT; v++) {
+            const int i = a16 + 16 * u, c = b16 + 16 * v;
+            if (i >= PT || c >= PT) continue;
+            const bool in = i < p && c < p;
+            const double rs = in ? s.rs[i] : 0.0;
+            s.t[i * LG + c] = in && c >= i ? M[u][v] * rs : 0.0;
+            s.g[c * LG + i] = in && c <= i ? (c == i ? 1.0 : M[u][v]) * rs : 0.0;
+        }
     __syncthreads();
-    for (int e = tid; e < p * p; e += 256) {
-        const int i = e / p, j = e % p;
-        s.g[i * LG + j] = i <= j ? s.x[j * LG + i] * s.rs[j] : 0.0;
-    }
     if (first) {
-        for (int e = tid; e < p * p; e += 256) s.r[(e / p) * LG + e % p] = s.t[(e / p) * LG + e % p];
+        for (int e = tid; e < PT * PT; e += 256) s.r[(e / PT) * LG + e % PT] = s.t[(e / PT) * LG + e % PT];
     } else {
-        double v[4];   // p^2 <= 1024
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = tid + 256 * u, i = e / p, j = e % p;
-            v[u] = 0.0;
-            if (e < p * p)
-                for (int c = i; c <= j; c++) v[u] += s.t[i * LG + c] * s.r[c * LG + j];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = tid + 256 * u;
-            if (e < p * p) s.r[(e / p) * LG + e % p] = v[u];
-        }
+        arn_mul_r<NT>(s.t, s.r);
     }
     __syncthreads();
-    // W <- W R^{-1}, 256 / p rows at a time
-    const int per = 256 / p;
-    for (int b = 0; b < a.rows; b += per) {
-        const int row = b + tid / p, c = tid % p;
-        const bool ok = tid < per * p && row < a.rows;
-        double v = 0.0;
-        if (ok)
-            for (int i = 0; i <= c; i++) v += s.w[row * LW + i] * s.g[i * LG + c];
-        __syncthreads();
-        if (ok) s.w[row * LW + c] = v;
+    // W <- W R^{-1}, a warp's row tiles in place
+    for (int t = warp; t < a.rows / 8; t += kArnoldiWarps) {
+        double acc[NT][2];
+#pragma unroll
+        for (int ni = 0; ni < NT; ni++) acc[ni][0] = acc[ni][1] = 0.0;
+#pragma unroll
+        for (int ks = 0; ks < 2 * NT; ks++) {
+            const double v = s.w[(8 * t + g) * LW + 4 * ks + t4];
+#pragma unroll
+            for (int ni = 0; ni < NT; ni++)
+                if (ks < 2 * (ni + 1)) arn_dmma(acc[ni][0], acc[ni][1], v, s.g[(4 * ks + t4) * LG + 8 * ni + g]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int ni = 0; ni < NT; ni++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) s.w[(8 * t + g) * LW + 8 * ni + 2 * t4 + i] = acc[ni][i];
     }
     __syncthreads();
     return 0;
@@ -509,10 +597,8 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
     unsigned gen = s_gen;
     ArnoldiSmem<NT> s;
     s.w = sm;
-    s.buf = s.w + a.rows * LW;
-    s.g = s.buf + arn_buf(NT);
-    s.x = s.g + PT * LG;
-    s.r = s.x + PT * LG;
+    s.buf = s.g = s.w + a.rows * LW;
+    s.r = s.g + arn_area(NT);
     s.t = s.r + PT * LG;
     s.rs = s.t + PT * LG;
     const int r0 = blockIdx.x * a.rows, p = a.p;
@@ -521,8 +607,13 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
         s.w[row * LW + c] = r0 + row < a.n && c < p ? a.Q[(size_t)(r0 + row) * p + c] : 0.0;
     }
     __syncthreads();
-    if (!arn_project<NT, EVEN>(a, s, r0, a.Psi, nullptr, gen, s_off != 0, true)) return;
-    if (!arn_project<NT, EVEN>(a, s, r0, a.Psi2, a.Psi, gen, false, false)) return;
+    if (a.qr_only) {   // the projections were done: only spread the decision to skip
+        if (!grid_barrier(a.ds, gen)) return;
+        if (*(volatile int *)a.snap == a.epoch) return;
+    } else {
+        if (!arn_project<NT, EVEN>(a, s, r0, a.Psi, nullptr, gen, s_off != 0, true)) return;
+        if (!arn_project<NT, EVEN>(a, s, r0, a.Psi2, a.Psi, gen, false, false)) return;
+    }
     bool shifted = false, ill = false;
     int f = arn_qr<NT>(a, s, r0, gen, shifted, &ill);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -530,23 +621,17 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
         a.st->qr_reorth = ill;
     }
     if (f == 0 && ill) {
-        // W = V Psi + Q1 R1, Q1 = V Phi + Q2 C2:  Psi += Phi R1, C = C2 R1
-        double *R1 = s.buf;   // kept beside the second factorization: buf is free between products
-        double keep[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = threadIdx.x + 256 * u;
-            keep[u] = e < p * p ? s.r[(e / p) * LG + e % p] : 0.0;
-        }
+        // W = V Psi + Q1 R1, Q1 = V Phi + Q2 C2:  Psi += Phi R1, C = C2 R1; R1 stays in C meanwhile
+        if (blockIdx.x == 0)
+            for (int e = threadIdx.x; e < p * p; e += 256) a.C[e] = s.r[(e / p) * LG + e % p];
         if (!arn_project<NT, EVEN>(a, s, r0, a.Psi2, nullptr, gen, false, false)) return;
         bool shift2 = false;
         f = arn_qr<NT>(a, s, r0, gen, shift2, nullptr);
         if (f == 0) {
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int e = threadIdx.x + 256 * u;
-                if (e < p * p) R1[e] = keep[u];
+            double *R1 = s.g;
+            for (int e = threadIdx.x; e < PT * PT; e += 256) {
+                const int i = e / PT, j = e % PT;
+                R1[i * LG + j] = i < p && j < p ? __ldcg(a.C + i * p + j) : 0.0;
             }
             __syncthreads();
             const size_t len = (size_t)a.k * p * p;
@@ -554,25 +639,16 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
                 const int b = (int)(e % p);
                 const double *ph = a.Psi2 + e - b;
                 double v = 0.0;
-                for (int c = 0; c <= b; c++) v += __ldcg(ph + c) * R1[c * p + b];
+                for (int c = 0; c <= b; c++) v += __ldcg(ph + c) * R1[c * LG + b];
                 a.Psi[e] += v;
             }
-            double v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int e = threadIdx.x + 256 * u, i = e / p, j = e % p;
-                v[u] = 0.0;
-                if (e < p * p)
-                    for (int c = i; c <= j; c++) v[u] += s.r[i * LG + c] * R1[c * p + j];
-            }
+            // r = C2 R1 in R1's place
+            arn_mul_r<NT>(s.r, R1);
             __syncthreads();
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int e = threadIdx.x + 256 * u;
-                if (e < p * p) s.r[(e / p) * LG + e % p] = v[u];
-            }
+            for (int e = threadIdx.x; e < PT * PT; e += 256) s.r[(e / PT) * LG + e % PT] = R1[(e / PT) * LG + e % PT];
             __syncthreads();
         }
+        if (f != 1 && !grid_barrier(a.ds, gen)) return;   // all have read C
     }
     if (f == 1) return;
     if (f == 2) {   // the host decides whether this iteration counted
@@ -590,18 +666,23 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
         for (int e = threadIdx.x; e < p * p; e += 256) a.C[e] = s.r[(e / p) * LG + e % p];
 }
 
-// Rows of a CTA: all SMs where there are 16 rows for each, fewer CTAs (and shorter sums) otherwise.
-static int arnoldi_rows(const bpf_ctx *ctx, int n) { return std::max(16, ceil_div(ceil_div(n, ctx->num_sms), 8) * 8); }
-
-static size_t arnoldi_smem(int rows, int p) {
-    const int nt = (p + 7) / 8, pt = 8 * nt;
-    return sizeof(double) * ((size_t)rows * (pt + 4) + (size_t)arn_buf(nt) +
-                             4 * (size_t)pt * (pt + 1) + pt);
+// Rows of a CTA: all SMs but eight (the Hessenberg update on the other stream takes a CTA per eight columns)
+// where there are 16 rows for each, fewer CTAs (and shorter sums) otherwise.
+static int arnoldi_rows(const bpf_ctx *ctx, int n) {
+    return std::max(16, ceil_div(ceil_div(n, std::max(1, ctx->num_sms - 8)), 8) * 8);
 }
 
-// Up to 32 columns a warp holds a whole p x p product in registers, and a slab fits beside the Cholesky.
+static int arnoldi_nt(int p) { return p <= 32 ? (p + 7) / 8 : p <= 48 ? 6 : 8; }
+
+static size_t arnoldi_smem(int rows, int p) {
+    const int nt = arnoldi_nt(p), pt = 8 * nt;
+    return sizeof(double) * ((size_t)rows * (pt + 4) + (size_t)arn_area(nt) + 2 * (size_t)pt * (pt + 1) + pt);
+}
+
+// Up to 64 columns a warp or two hold a whole p x p product in registers, and a slab fits beside the Cholesky.
 bool arnoldi_ok(const bpf_ctx *ctx, int n, int p) {
-    return ctx->fp64_mma && p <= 32 && arnoldi_smem(arnoldi_rows(ctx, n), p) + 1024 <= (size_t)ctx->max_smem_optin;
+    return ctx->fp64_mma && p <= 64 &&
+           arnoldi_smem(arnoldi_rows(ctx, n), p) + 1024 <= (size_t)ctx->max_smem_optin;
 }
 
 // Products of 65536 sums (64 blocks of 32 columns) at a time: the partial sums of all CTAs stay within
@@ -613,7 +694,7 @@ size_t arnoldi_partials(const bpf_ctx *ctx, int n, int p, int k) {
 }
 
 bpf_status arnoldi_step(bpf_ctx *ctx, int n, int p, int k, const double *V, size_t strideV, const double *Q, double *Vn,
-                        double *Psi, double *Psi2, double *C, SolveState *st) {
+                        double *Psi, double *Psi2, double *C, SolveState *st, bool qr_only) {
     bpf_status s;
     double *part = (double *)ws_get(ctx, WS_PARTIAL, sizeof(double) * arnoldi_partials(ctx, n, p, k), &s);
     if (!part) return s;
@@ -636,17 +717,20 @@ bpf_status arnoldi_step(bpf_ctx *ctx, int n, int p, int k, const double *V, size
     a.st = st;
     a.snap = &ctx->dstat->pad[1];
     a.epoch = ++ctx->arnoldi_epoch;
+    a.qr_only = qr_only ? 1 : 0;
     a.ds = ctx->dstat;
     const size_t smem = arnoldi_smem(a.rows, p);
-    const bool even = p % 2 == 0 && ((uintptr_t)V & 15) == 0 && strideV % 2 == 0;
+    const bool even = p % 2 == 0;   // every block is 16-byte aligned then (workspaces and multiples of p doubles)
     const void *kern = p <= 8    ? (even ? (const void *)arnoldi_kernel<1, true> : (const void *)arnoldi_kernel<1, false>)
                        : p <= 16 ? (even ? (const void *)arnoldi_kernel<2, true> : (const void *)arnoldi_kernel<2, false>)
                        : p <= 24 ? (even ? (const void *)arnoldi_kernel<3, true> : (const void *)arnoldi_kernel<3, false>)
-                                 : (even ? (const void *)arnoldi_kernel<4, true> : (const void *)arnoldi_kernel<4, false>);
+                       : p <= 32 ? (even ? (const void *)arnoldi_kernel<4, true> : (const void *)arnoldi_kernel<4, false>)
+                       : p <= 48 ? (even ? (const void *)arnoldi_kernel<6, true> : (const void *)arnoldi_kernel<6, false>)
+                                 : (even ? (const void *)arnoldi_kernel<8, true> : (const void *)arnoldi_kernel<8, false>);
     BPF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *args[] = {&a};
     // the basis read four times (two passes), the block in and out; products and updates of both passes
-    KScope ks(ctx, BPF_KC_GRAM, 8.0 * n * p * (4.0 * k + 2.0), 8.0 * n * p * (double)p * k);
+    KScope ks(ctx, BPF_KC_GRAM, 8.0 * n * p * (qr_only ? 2.0 : 4.0 * k + 2.0), 8.0 * n * p * (double)p * (qr_only ? 1 : k));
     BPF_CUDA(ctx, cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(256), args, smem, ctx->stream));
     BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;

@@ -35,9 +35,10 @@ def _solve(bpf, A, B, **kw):
 
 
 # column counts at the edges of the 8-wide tiles; rows: a short last slab, one slab, and more
-# rows than SMs x 16 (slabs of 24 rows); 33 columns go by the kernels for wider blocks
+# rows than SMs x 16 (slabs of 24 rows); other kernels from 65 columns
 @pytest.mark.parametrize("nbus,p", [(20, 1), (40, 7), (300, 8), (300, 9), (300, 16), (301, 17), (300, 24),
-                                    (300, 25), (300, 31), (300, 32), (300, 33), (1400, 5), (1700, 32)])
+                                    (300, 25), (300, 31), (300, 32), (300, 33), (1400, 5), (1700, 32), (300, 34), (300, 48), (301, 50), (300, 64), (1700, 64), (300, 66),
+                                    (300, 47), (300, 63)])
 def test_edges(bpf, nbus, p):
     A = bpf.grid.synthetic_jacobian(nbus, seed=nbus)
     B = np.random.default_rng(p).standard_normal((A.shape[0], p))
@@ -63,3 +64,24 @@ def test_more_blocks_than_a_group(bpf):
     bound = 10 * k * 2.0**-52 * (np.sqrt((A.multiply(A)).sum()) * np.linalg.norm(X) + np.linalg.norm(B))
     assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= bound
     assert bound < 0.1 * st.residuals[-1]
+
+
+@pytest.mark.parametrize("p", [12, 32, 48, 64])
+def test_ill_conditioned_blocks(bpf, p):
+    """The identity's columns make numerically rank-deficient blocks: shift, third pass, re-orthogonalization.  The
+    estimate and the true residual then agree to the stopping bound (a basis that lost orthogonality would not)."""
+    A = bpf.grid.preset_jacobian("case300", 0)
+    B = np.eye(A.shape[0], p)
+    X, st = _solve(bpf, A, B, memory=60)
+    assert st.solved
+    assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= 1e-2 * 1e-8 * np.linalg.norm(B)
+
+
+@pytest.mark.parametrize("p", [3, 8, 15, 24, 31, 32, 40, 45, 48, 61, 64])
+def test_tall_slabs(bpf, p):
+    """Slabs of 72 rows (nine row tiles, the last slab short): coefficients through shared memory."""
+    A = bpf.grid.synthetic_jacobian(5200, seed=7)
+    B = np.random.default_rng(p).standard_normal((A.shape[0], p))
+    X, st = _solve(bpf, A, B, memory=300)
+    assert st.solved
+    assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= 1e-2 * 1e-8 * np.linalg.norm(B)
