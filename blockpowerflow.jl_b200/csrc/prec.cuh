@@ -232,11 +232,12 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
 bpf_status lu_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals);
 bpf_status lu_solve(bpf_ctx *ctx, const bpf_prec *P, int nrhs, double *X, int ldx);   // in place
 // Column-per-CTA triangular solves (trsv_col.cu) of a preconditioner kept for them (P->col):
-// column-major blocks (Y may be X with the same leading dimension), or row-major ones.
+// column-major blocks (Y may be X with the same leading dimension; step: doubles between a column's
+// elements), or row-major ones.
 bool trsv_col_fits(const bpf_ctx *ctx, int n, int fdtype);
 int trsv_col_ring(const bpf_ctx *ctx, int n, int fdtype);
 bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, size_t ldx, double *Y, size_t ldy,
-                    const int *gate = nullptr);
+                    const int *gate = nullptr, size_t step = 1);
 bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y,
                              const int *gate = nullptr);
 bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X,

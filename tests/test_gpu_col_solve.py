@@ -125,3 +125,20 @@ def test_zero_pivot_is_reported_and_the_next_factorization_runs(bpf):
         P.refactor(vals)
     P.refactor(Ad.nzVal)
     np.testing.assert_allclose(P.P.nzVal.cpu().numpy(), O.ilu0(pat).data, rtol=1e-11)
+
+
+@pytest.mark.parametrize("n", [500, 3072, 3073])
+@pytest.mark.parametrize("p", [2, 17])
+@pytest.mark.parametrize("f32", [False, True])
+def test_row_major_blocks(bpf, n, p, f32):
+    """Inside a solver the blocks are row-major: in place up to 3,072 rows, through copies beyond.  A solve whose
+    blocks came back wrong could not reach the bound: 1.01 covers the estimate's rounding."""
+    import torch
+
+    A = _random(n, 3, n + p)
+    B = np.random.default_rng(p).standard_normal((n, p))
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    N = bpf.ilu0(Ad, p, factor_dtype="float32") if f32 else bpf.ilu0(Ad, p)
+    X, st = bpf.block_gmres(Ad, torch.as_tensor(B, device="cuda"), N=N, ldiv=True, memory=40, atol=0.0, rtol=1e-8)
+    assert st.solved
+    assert np.linalg.norm(B - A @ X.cpu().numpy()) <= 1.01e-8 * np.linalg.norm(B)
