@@ -7,13 +7,17 @@
 // gated off nearly always, 3-13 us each: 300 us an iteration of a 300-bus solve with 16 columns,
 // whose arithmetic is worth a few.  Here they are one cooperative launch: a CTA keeps its rows of the
 // new block W in shared memory from the first product to the finished basis block, and what CTAs
-// exchange are p x p partial sums through global memory, one grid barrier each (seven an iteration).
+// exchange are p x p partial sums through global memory: two grid barriers a Gram-Schmidt pass (each group of
+// basis blocks), one a Cholesky pass whose sums every CTA takes itself, two where they are shared out.  Six
+// or eight an ordinary iteration.
 //
 //  * Products V_j^T W: a warp per basis block over the CTA's rows, FP64 tensor pipe (m8n8k4).  A pass'
 //    partial sums are added over the CTAs element by element by all threads, in a fixed order.
 //  * Update W -= sum_j V_j Psi_j: 16 rows a warp, or the blocks j split over warps where rows are few.
 //  * Cholesky-QR: every CTA sums the partial Gram matrices and factors them itself, identically, so the
-//    rare decisions (shift, third pass, re-orthogonalization, breakdown) need no further exchange.
+//    rare decisions (shift, third pass, re-orthogonalization, breakdown) need no further exchange.  A pass
+//    that each CTA sums for itself has no barrier after its reads, so passes alternate between two sets
+//    of partial sums: a set is written again only behind the barrier of the pass between.
 //
 // Same algorithm and decisions as gram / tsmm / cholqr / reorth_fold (dense.cu, small.cu); the sums are
 // grouped differently, so results agree to rounding.
@@ -43,6 +47,7 @@ struct ArnoldiArgs {
     double *Psi, *Psi2;  // k blocks p x p: coefficients, and those of a second pass
     double *C;           // p x p: R of the new block
     double *part;        // gridDim.x blocks of group p^2 partial sums
+    double *part2;       // gridDim.x blocks of p^2: those of every other Cholesky pass
     int group;           // basis blocks whose products are in flight at a time
     double *gsum;        // p^2
     SolveState *st;
@@ -338,10 +343,10 @@ __device__ __forceinline__ void arn_update(const ArnoldiArgs &a, const ArnoldiSm
 }
 
 // Sum over the CTAs of element e of their partial sums; four lanes (8 apart) share an element's CTAs.
-__device__ __forceinline__ double arn_total(const ArnoldiArgs &a, size_t len, size_t e) {
+__device__ __forceinline__ double arn_total(const double *part, size_t len, size_t e) {
     double s = 0.0;
     if (e < len) {
-        const double *q = a.part + e;
+        const double *q = part + e;
 #pragma unroll 8
         for (unsigned c = (threadIdx.x >> 3) & 3; c < gridDim.x; c += 4) s += __ldcg(q + c * len);
     }
@@ -351,12 +356,12 @@ __device__ __forceinline__ double arn_total(const ArnoldiArgs &a, size_t len, si
 
 // f(e, total of e) for this CTA's share of the elements (all: every element).
 template <class F>
-__device__ __forceinline__ void arn_totals(const ArnoldiArgs &a, size_t len, bool all, F f) {
+__device__ __forceinline__ void arn_totals(const double *part, size_t len, bool all, F f) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     for (size_t e0 = ((all ? 0 : (size_t)blockIdx.x) * kArnoldiWarps + w) * 8; e0 < len;
          e0 += (size_t)(all ? 1 : gridDim.x) * kArnoldiWarps * 8) {
         const size_t e = e0 + (l & 7);
-        const double v = arn_total(a, len, e);
+        const double v = arn_total(part, len, e);
         if (l < 8 && e < len) f(e, v);
     }
 }
@@ -372,7 +377,7 @@ __device__ __forceinline__ bool arn_project(const ArnoldiArgs &a, const ArnoldiS
         if (!skip) arn_gram<NT, EVEN>(a, s, r0, a.V + (size_t)j0 * a.strideV, nb, a.part + blockIdx.x * len);
         if (!grid_barrier(a.ds, gen)) return false;
         if (check && *(volatile int *)a.snap == a.epoch) return false;   // some CTA saw the solve stopped
-        arn_totals(a, len, false, [&](size_t e, double v) {
+        arn_totals(a.part, len, false, [&](size_t e, double v) {
             out[j0 * pp + e] = v;
             if (acc) acc[j0 * pp + e] += v;
         });
@@ -406,10 +411,11 @@ __device__ __forceinline__ void arn_mul_r(const double *t, double *r) {
 }
 
 // One pass of Cholesky-QR on the CTAs' rows: s.r <- R s.r (first: R).  0: done; 1: a barrier gave up; 2:
-// breakdown.  shift / ill: set when the pass needed the shift / lost more than eight digits.
+// breakdown.  shift / ill: set when the pass needed the shift / lost more than eight digits.  part: a.part and
+// a.part2 in turn (other CTAs may still be reading those of the pass before).
 template <int NT>
-__device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSmem<NT> &s, int r0, bool first, unsigned &gen,
-                                          bool &shifted, bool *ill) {
+__device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSmem<NT> &s, int r0, double *part, bool first,
+                                          unsigned &gen, bool &shifted, bool *ill) {
     constexpr int PT = ArnoldiSmem<NT>::PT, LW = ArnoldiSmem<NT>::LW, LG = ArnoldiSmem<NT>::LG;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3, p = a.p, tid = threadIdx.x;
     const size_t pp = (size_t)p * p;
@@ -436,7 +442,7 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
                 for (int i = 0; i < 2; i++) {
                     const int row = 8 * mi + g, col = 8 * ni + 2 * t4 + i;
                     if (PARTS > 1) s.buf[q * PT * PT + row * PT + col] = acc[ni][i];
-                    else if (row < p && col < p) a.part[blockIdx.x * pp + (size_t)row * p + col] = acc[ni][i];
+                    else if (row < p && col < p) part[blockIdx.x * pp + (size_t)row * p + col] = acc[ni][i];
                 }
         }
         if (PARTS > 1) {
@@ -445,7 +451,7 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
                 double v = 0.0;
 #pragma unroll
                 for (int u = 0; u < PARTS; u++) v += s.buf[u * PT * PT + (e / p) * PT + e % p];
-                a.part[blockIdx.x * pp + e] = v;
+                part[blockIdx.x * pp + e] = v;
             }
         }
     }
@@ -453,14 +459,14 @@ __device__ __forceinline__ int arn_cholqr(const ArnoldiArgs &a, const ArnoldiSme
     // the sum over the CTAs: each its own, or, where that is much to read, shared out first
     const bool shared_out = pp * gridDim.x > 16384;
     if (shared_out) {
-        arn_totals(a, pp, false, [&](size_t e, double v) { a.gsum[e] = v; });
+        arn_totals(part, pp, false, [&](size_t e, double v) { a.gsum[e] = v; });
         if (!grid_barrier(a.ds, gen)) return 1;
     }
     double trace = 0.0;
     if (shared_out)
         for (int e = tid; e < p * p; e += 256) s.t[(e / p) * LG + e % p] = __ldcg(a.gsum + e);
     else
-        arn_totals(a, pp, true, [&](size_t e, double v) { s.t[((int)e / p) * LG + (int)e % p] = v; });
+        arn_totals(part, pp, true, [&](size_t e, double v) { s.t[((int)e / p) * LG + (int)e % p] = v; });
     __syncthreads();
     for (int i = 0; i < p; i++) trace += s.t[i * LG + i];
     int fail = 0;
@@ -571,11 +577,11 @@ template <int NT>
 __device__ __forceinline__ int arn_qr(const ArnoldiArgs &a, const ArnoldiSmem<NT> &s, int r0, unsigned &gen, bool &shifted,
                                       bool *ill) {
     shifted = false;
-    int f = arn_cholqr<NT>(a, s, r0, true, gen, shifted, ill);
-    if (f == 0) f = arn_cholqr<NT>(a, s, r0, false, gen, shifted, nullptr);
+    int f = arn_cholqr<NT>(a, s, r0, a.part, true, gen, shifted, ill);
+    if (f == 0) f = arn_cholqr<NT>(a, s, r0, a.part2, false, gen, shifted, nullptr);
     if (f == 0 && shifted) {
         bool again = false;
-        f = arn_cholqr<NT>(a, s, r0, false, gen, again, nullptr);
+        f = arn_cholqr<NT>(a, s, r0, a.part, false, gen, again, nullptr);
     }
     return f;
 }
@@ -621,6 +627,7 @@ __global__ void __launch_bounds__(256, 1) arnoldi_kernel(ArnoldiArgs a) {
         a.st->qr_reorth = ill;
     }
     if (f == 0 && ill) {
+        if (!grid_barrier(a.ds, gen)) return;   // the last pass' sums have been read: the products reuse their place
         // W = V Psi + Q1 R1, Q1 = V Phi + Q2 C2:  Psi += Phi R1, C = C2 R1; R1 stays in C meanwhile
         if (blockIdx.x == 0)
             for (int e = threadIdx.x; e < p * p; e += 256) a.C[e] = s.r[(e / p) * LG + e % p];
@@ -690,7 +697,7 @@ bool arnoldi_ok(const bpf_ctx *ctx, int n, int p) {
 static int arnoldi_group(int p, int k) { return std::min(k, 65536 / (p * p)); }
 
 size_t arnoldi_partials(const bpf_ctx *ctx, int n, int p, int k) {
-    return ((size_t)ceil_div(n, arnoldi_rows(ctx, n)) * arnoldi_group(p, k) + 1) * p * p;
+    return ((size_t)ceil_div(n, arnoldi_rows(ctx, n)) * (arnoldi_group(p, k) + 1) + 1) * p * p;
 }
 
 bpf_status arnoldi_step(bpf_ctx *ctx, int n, int p, int k, const double *V, size_t strideV, const double *Q, double *Vn,
@@ -714,6 +721,7 @@ bpf_status arnoldi_step(bpf_ctx *ctx, int n, int p, int k, const double *V, size
     const int grid = ceil_div(n, a.rows);
     a.gsum = part;
     a.part = part + (size_t)p * p;
+    a.part2 = a.part + (size_t)grid * a.group * p * p;
     a.st = st;
     a.snap = &ctx->dstat->pad[1];
     a.epoch = ++ctx->arnoldi_epoch;

@@ -85,3 +85,26 @@ def test_tall_slabs(bpf, p):
     X, st = _solve(bpf, A, B, memory=300)
     assert st.solved
     assert abs(np.linalg.norm(B - A @ X) - st.residuals[-1]) <= 1e-2 * 1e-8 * np.linalg.norm(B)
+
+
+@pytest.mark.parametrize("overlap", ["1", "0"])
+@pytest.mark.parametrize("nbus,p,ill", [(300, 1, False), (300, 8, False), (300, 16, False), (300, 16, True), (1400, 9, False),
+                                        (1400, 8, True), (300, 32, False), (300, 32, True)])
+def test_repeated_solves_agree_to_the_bit(bpf, monkeypatch, nbus, p, ill, overlap):
+    """Every sum has a fixed order, so CTAs that read one another's partial sums too late or too early are the only
+    way for two runs to differ: 10 columns and fewer (16 up to 1,024 rows) sum them in every CTA, more share them out."""
+    import torch
+
+    monkeypatch.setenv("BPF_OVERLAP", overlap)
+    monkeypatch.setattr(bpf._lib, "_ctxs", {})   # a context made with this setting
+    A = bpf.grid.synthetic_jacobian(nbus, seed=nbus)
+    n = A.shape[0]
+    B = torch.as_tensor(np.eye(n, p) if ill else np.random.default_rng(p).standard_normal((n, p)), device="cuda")
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    N = bpf.ilu0(Ad, p)
+    first = None
+    for _ in range(40):
+        X, st = bpf.block_gmres(Ad, B, N=N, ldiv=True, memory=60, atol=0.0, rtol=1e-8, history=True)
+        if first is None:
+            first = X.clone(), list(st.residuals)
+        assert torch.equal(X, first[0]) and list(st.residuals) == first[1]
