@@ -58,7 +58,7 @@ __device__ __forceinline__ void lu_dmma(double &d0, double &d1, double a, double
 // thread, and an entry costs one barrier.  Front rows depend on one another as in factor_df_kernel
 // (values are their own ready marks; positions in dependency order, all CTAs resident, bounded polls).
 struct CtaRowsArgs {
-    int count, s, mp, nmax, wmax;
+    int count, s, m, mp, nmax, wmax;
     const int *order, *rp, *ci, *diag, *fend, *fsrc, *pp, *pdst;
     const double *vals;
     double *fv, *S;
@@ -72,6 +72,10 @@ __global__ void __launch_bounds__(256) lu_cta_rows_kernel(CtaRowsArgs a) {
     int *p0 = reinterpret_cast<int *>(lv + a.nmax), *src = p0 + a.nmax + 1;   // pair range, source - pair
     const int tid = threadIdx.x;
     const long long lim = a.ds->wait_limit > 0 ? a.ds->wait_limit : kSpinLimit;
+    // the tail's rows past the last are the identity: written every time, since the tail's factorization
+    // spreads a NaN or an infinity into them
+    for (size_t e = (size_t)a.m * a.mp + blockIdx.x * 256 + tid; e < (size_t)a.mp * a.mp; e += (size_t)gridDim.x * 256)
+        a.S[e] = e / a.mp == e % a.mp ? 1.0 : 0.0;
     for (int q = blockIdx.x; q < a.count; q += gridDim.x) {
         const int i = __ldg(a.order + q);
         const bool tail = i >= a.s;
@@ -611,7 +615,7 @@ bpf_status lu_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     if (!taken) return set_error(ctx, BPF_ERR_NOT_SUPPORTED, "LU refactorization: a row of %d entries", P->max_row);
     const int nb = P->tail_mp / kNB, count = P->nlong + P->tail_m;
     if (count > 0) {
-        CtaRowsArgs a{count, P->tail_s, P->tail_mp, P->cta_nmax, P->cta_wmax, P->forder + P->nshort, P->rp, P->ci, P->diag,
+        CtaRowsArgs a{count, P->tail_s, P->tail_m, P->tail_mp, P->cta_nmax, P->cta_wmax, P->forder + P->nshort, P->rp, P->ci, P->diag,
                       P->fend, P->fsrc, P->pp, P->pdst, vals, P->fv, P->tail_S, sweep_store(P), ctx->dstat};
         const size_t smem = cta_rows_smem(P->cta_nmax, P->cta_wmax);
         BPF_CUDA(ctx, cudaFuncSetAttribute(lu_cta_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -922,14 +926,11 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
             up_v(&P->cs[w].head, cs[w].head);
             up_v(&P->cs[w].bytes, cs[w].bytes);
         }
-    std::vector<double> S;
     if (mp > 0) {
-        // rows past the last: the identity, once (no elimination step changes it)
-        S.assign((size_t)mp * mp, 0.0);
-        for (int r = m; r < mp; r++) S[(size_t)r * mp + r] = 1.0;
-        up_v(&P->tail_S, S);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_F, sizeof(double) * S.size());
-        if (e == cudaSuccess) e = cudaMemsetAsync(P->tail_F, 0, sizeof(double) * S.size(), ctx->stream);
+        const size_t tail_bytes = sizeof(double) * (size_t)mp * mp;
+        if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_S, tail_bytes);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_F, tail_bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(P->tail_F, 0, tail_bytes, ctx->stream);
         if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_inv, sizeof(double) * 2 * (size_t)nb * kNB * kNB);
     }
     if (e == cudaSuccess && P->nnz > 0) e = cudaMalloc((void **)&P->fv, sizeof(double) * P->nnz);

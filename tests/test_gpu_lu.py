@@ -2,6 +2,8 @@
 around the 64-column tile, fronts of every row length, the last system the column solves take and the
 first that goes by row sweeps (each width class of those), distinct replicas, pivots that vanish in
 the front and in the tail, and a right-hand side with a NaN column beside finite ones."""
+import contextlib
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -133,3 +135,24 @@ def test_nan_column_leaves_the_others_alone(bpf, buses):
     keep = [c for c in range(40) if c != 3]
     np.testing.assert_array_equal(X[:, keep].cpu().numpy(), ref[:, keep].cpu().numpy())
     assert np.isnan(X[:, 3].cpu().numpy()).any()
+
+
+# tails of two to nine tiles: the last one partly, or wholly, rows of the matrix
+@pytest.mark.parametrize("n", [65, 100, 128, 180, 240, 500])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("at", [0, -1])
+def test_a_refactorization_with_a_nan_leaves_the_next_one_alone(bpf, n, bad, at):
+    A = sp.csr_matrix(np.random.default_rng(n).standard_normal((n, n)) + 2.0 * n * np.eye(n))
+    rf, gA = _check(bpf, A, (1,), "NATURAL")
+    good = gA.nzVal.clone()
+    B = np.random.default_rng(1).standard_normal((n, 3))
+    before = _block(B)
+    bpf.CUSOLVERRF.ldiv_(rf, before)
+    gA.nzVal[at] = bad
+    with contextlib.suppress(bpf.SingularException):
+        bpf.CUSOLVERRF.update_(rf, gA)
+    gA.nzVal.copy_(good)
+    bpf.CUSOLVERRF.update_(rf, gA)
+    X = _block(B)
+    bpf.CUSOLVERRF.ldiv_(rf, X)
+    np.testing.assert_array_equal(X.cpu().numpy(), before.cpu().numpy())
