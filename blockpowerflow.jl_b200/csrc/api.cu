@@ -167,8 +167,10 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     }
     if (P->col) {
         const int nring = trsv_col_ring(ctx, n, fdtype);
-        tri_to_stream(lo, fdtype, nring, 0, n, false, pos0, cs[0], tpos[0]);
-        tri_to_stream(up, fdtype, nring, (int)cs[0].coff.size() - 1, n, false, pos1, cs[1], tpos[1]);
+        P->col = tri_to_stream(lo, fdtype, nring, 0, n, false, pos0, cs[0], tpos[0]) &&
+                 tri_to_stream(up, fdtype, nring, (int)cs[0].coff.size() - 1, n, false, pos1, cs[1], tpos[1]);
+    }
+    if (P->col) {
         for (int q = 0; q < n; q++) pos01[q] = pos0[up.rows[q]];
         if (!perm.empty()) {   // positions of the block's rows: factor row i is row perm[i]
             std::vector<int> b0(n), b1(n);
@@ -182,6 +184,7 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     } else if (kind != PREC_LU) {
         for (int w = 0; w < 2; w++) {
             const TriHost &t = w == 0 ? lo : up;
+            std::fill(tpos[w].begin(), tpos[w].end(), -1);
             for (size_t k = 0; k < t.map.size(); k++) tpos[w][t.map[k]] = (int)k;
             for (size_t q = 0; q < t.dmap.size(); q++) tpos[w][t.dmap[q]] = -2 - (int)q;
         }

@@ -761,7 +761,7 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
     // Tail size: estimated microseconds of the levels (1.5 a level in the factorization, and in each
     // sweep 0.4 in shared memory or 1.5 through L2) against the dense block (28 a 64-column step of
     // factorization and solve, and its tiles 7 each over the SMs).
-    const bool col = n > 0 && trsv_col_fits(ctx, n, BPF_F64);
+    bool col = n > 0 && trsv_col_fits(ctx, n, BPF_F64);
     std::vector<int> bl;
     int best = 0;
     double best_us = -1.0;
@@ -842,7 +842,6 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
     P->cta_pairs = (long long)pdst.size();
     P->cta_nmax = nmax;
     P->cta_wmax = wmax;
-    P->col = col;
     P->tail_s = s;
     P->tail_m = m;
     P->tail_mp = mp;
@@ -869,8 +868,11 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
     tpos[1].assign(P->nnz, -1);
     if (col) {
         const int nring = trsv_col_ring(ctx, n, BPF_F64);
-        tri_to_stream(lo, BPF_F64, nring, 0, n, true, pos0, cs[0], tpos[0]);
-        tri_to_stream(up, BPF_F64, nring, (int)cs[0].coff.size() - 1, n, true, pos1, cs[1], tpos[1]);
+        col = tri_to_stream(lo, BPF_F64, nring, 0, n, true, pos0, cs[0], tpos[0]) &&
+              tri_to_stream(up, BPF_F64, nring, (int)cs[0].coff.size() - 1, n, true, pos1, cs[1], tpos[1]);
+    }
+    P->col = col;
+    if (col) {
         for (int q = 0; q < n; q++) pos01[q] = q < s ? pos0[up.rows[q]] : q;
         std::vector<int> b0(n), b1(n);   // positions of the block's rows
         for (int i = 0; i < n; i++) {
@@ -882,6 +884,7 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
     } else {
         for (int w = 0; w < 2; w++) {
             const TriHost &t = w == 0 ? lo : up;
+            std::fill(tpos[w].begin(), tpos[w].end(), -1);
             for (size_t k = 0; k < t.map.size(); k++) tpos[w][t.map[k]] = (int)k;
             for (size_t q = 0; q < t.dmap.size(); q++) tpos[w][t.dmap[q]] = -2 - (int)q;
         }

@@ -123,7 +123,7 @@ struct TriStream {
     int diag = 0, nstage = 0;
 };
 // ntot: unknowns (rows from t.n on keep their positions); lu: long rows over a whole warp
-void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
+bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
                    TriStream &out, std::vector<int> &tpos);
 // values = false: the schedule only (the values are kept elsewhere)
 bpf_status tri_upload(bpf_ctx *ctx, const TriHost &h, TriDev &d, bool values = true);

@@ -54,6 +54,10 @@ constexpr int kChunk = 16384;      // bytes of a chunk, at most
 constexpr int kWideRow = 16;       // entries past which an LU's row takes a whole warp
 constexpr int kColWarps = 23;      // computing warps, at most
 constexpr int kChunkRing = 6;      // chunks in flight, at most (as many as fit beside the column)
+// Bytes of a sweep's stream, at most: offsets are int, and a slab of one row takes 1,280 bytes per four entries,
+// up to 32 times the level-sorted form where every level holds one long row (12,000 rows of 200 lower
+// entries: 768 MB for 48).  Grids' factors take 1 to 20 MB.
+constexpr size_t kStreamMax = size_t(1) << 28;
 
 // A group of four entries of 32 rows: [lane][4] 16-bit columns, then the values as [2][lane][2]
 // doubles or [lane][4] floats.
@@ -453,7 +457,8 @@ bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const doubl
 // ... follow); pos[i] = position of row i; tpos[k] = value index (in units of the factor type) of
 // pattern entry k in the stream (-2 - index: its reciprocal's).  nring: slots of the ring; chunk0:
 // chunks of the sweep before.
-void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
+// False, with out and tpos in part filled, when the stream would pass kStreamMax.
+bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
                    TriStream &out, std::vector<int> &tpos) {
     const int wide_row = lu ? kWideRow : 2147483647;
     const size_t es = fdtype == BPF_F32 ? sizeof(float) : sizeof(double);
@@ -488,7 +493,7 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
     const int gmax = (int)((kChunk - 32 * es) / gb);   // groups of one part
     std::vector<Part> cur;
     int nslab = 0, stage = 0;
-    size_t body = 0;
+    size_t body = 0, total = 0;
     out.coff.assign(1, 0);
     out.cslab.assign(1, 0);
     auto close = [&]() {
@@ -548,6 +553,8 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
                 rest = std::max(rest, parts - 1);
                 if (pass >= parts) continue;
                 const int g0 = pass * gmax;
+                total += part_bytes(std::min(gmax, ng - g0));
+                if (total > kStreamMax) return false;
                 add(Part{q0, rows, (wide ? 128 : 4) * g0, std::min(gmax, ng - g0), pass == parts - 1 ? 1 : 0, stage, wide});
             }
         }
@@ -555,6 +562,7 @@ void tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
     close();
     out.diag = t.unit ? 0 : 1;
     out.nstage = stage;
+    return true;
 }
 
 }  // namespace bpf

@@ -142,3 +142,23 @@ def test_row_major_blocks(bpf, n, p, f32):
     X, st = bpf.block_gmres(Ad, torch.as_tensor(B, device="cuda"), N=N, ldiv=True, memory=40, atol=0.0, rtol=1e-8)
     assert st.solved
     assert np.linalg.norm(B - A @ X.cpu().numpy()) <= 1.01e-8 * np.linalg.norm(B)
+
+
+def test_a_stream_past_its_limit_is_not_kept(bpf):
+    """Single-row levels of 160 entries: the column solves' storage would be 307 MB, most of it padding.  The
+    level-sorted form takes 20 MB, the lists of the factorization 618."""
+    import torch
+
+    n, w, p = 6000, 160, 3
+    A = sp.csr_matrix(sp.diags([np.full(n - d, 0.5 / w) for d in range(w + 1)], [-d for d in range(w + 1)]) + 2.0 * sp.eye(n))
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    X = np.random.default_rng(6).standard_normal((n, p))
+    B = _block(X)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    P = bpf.ilu0(Ad, p)
+    used = free - torch.cuda.mem_get_info()[0]
+    ref = O.prec_apply(1, O.ilu0(A), X)
+    Y = P.ldiv(B).cpu().numpy()
+    assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
+    assert used < 700 << 20
