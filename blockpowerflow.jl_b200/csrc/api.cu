@@ -194,12 +194,26 @@ bpf_status prec_setup(bpf_ctx *ctx, int kind, int n, const std::vector<int> &rp,
     std::vector<long long> goff;
     PairVec gsrc;
     for (int i = 0; i < n; i++) P->max_row = std::max(P->max_row, rp[i + 1] - rp[i]);
-    const bool pairs_ok = kind != PREC_LU && (kind != PREC_ILU0 || P->max_row > kGatherRow
-                                                  ? build_pairs(n, rp.data(), ci.data(), diag.data(), ic, pp, pdst, psrc)
-                                                  : true);
-    long long gathered = 0;
-    if (kind == PREC_ILU0) gathered = build_gather(n, rp, ci, diag, {}, goff, gsrc);
-    P->npairs = std::max((long long)pdst.size(), gathered);
+    auto pairs = [&](bool count_only) {
+        return build_pairs(n, rp.data(), ci.data(), diag.data(), ic, pp, pdst, psrc, count_only);
+    };
+    bool pairs_ok = kind != PREC_LU;
+    if (ic) pairs_ok = pairs(false);
+    if (kind == PREC_ILU0) {
+        // lists of at most kGatherFree ints hold fewer updates than pairs may number: nothing to count
+        const long long ints = gather_ints(n, rp, diag, {});
+        bool lists = gather_fits(ints, 0);
+        if (!lists) {
+            pairs_ok = pairs(true);
+            lists = pairs_ok && gather_fits(ints, pp[nnz]);
+        }
+        P->pair_row = P->max_row > kGatherRow || !lists ? P->max_row : 0;
+        if (pairs_ok && P->pair_row > 0) pairs_ok = pairs(false);
+        else std::vector<int>().swap(pp);
+        if (pairs_ok && lists) P->npairs = build_gather(n, rp, ci, diag, {}, goff, gsrc);
+        else goff.assign(std::max(n, 1), -1);
+    }
+    P->npairs = std::max((long long)pdst.size(), P->npairs);
     auto fail = [&](bpf_status s) {
         cudaStreamSynchronize(ctx->stream);
         bpf_prec_destroy(P);

@@ -782,11 +782,16 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
     // rows a CTA takes: the tail's, front rows with a long U part or too many entries for gather lists,
     // and the rows that depend on those
     std::vector<char> cta(n, 0);
+    long long warp_pairs = 0;   // update pairs of the other rows
+    for (int i = 0; i < n; i++) {
+        cta[i] = i >= s || rp[i + 1] - diag[i] > kCtaRow || rp[i + 1] - rp[i] > kGatherRow;
+        for (int k = rp[i]; k < diag[i] && !cta[i]; k++) cta[i] = cta[ci[k]];
+        for (int k = rp[i]; k < diag[i] && !cta[i]; k++) warp_pairs += rp[ci[k] + 1] - diag[ci[k]] - 1;
+    }
+    if (!gather_fits(gather_ints(s, rp, diag, cta), warp_pairs)) cta.assign(n, 1);
     int nmax = 0, wmax = 0;
     for (int i = 0; i < n; i++) {
         const int len = rp[i + 1] - rp[i];
-        cta[i] = i >= s || rp[i + 1] - diag[i] > kCtaRow || len > kGatherRow;
-        for (int k = rp[i]; k < diag[i] && !cta[i]; k++) cta[i] = cta[ci[k]];
         if (!cta[i]) continue;
         nmax = std::max(nmax, i < s ? diag[i] - rp[i] : fend[i] - rp[i]);
         wmax = std::max(wmax, i < s ? len : fend[i] - rp[i] + mp);

@@ -136,7 +136,7 @@ TriHost build_tri(int n, const int *rp, const int *ci, const int *diag, int part
 // IC(0) pairs: for the L entry e = (i,k), every j < k with (i,j) and (k,j) in the lower
 // pattern gives (pos(i,j), pos(k,j)); fv[e] -= sum fv[pos(i,j)] * fv[pos(k,j)].
 bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
-                 std::vector<int> &pp, PairVec &pdst, PairVec &psrc) {
+                 std::vector<int> &pp, PairVec &pdst, PairVec &psrc, bool count_only) {
     const int nnz = rp[n];
     pp.assign(nnz + 1, 0);
     // rows [i0, i1): pass 0 counts the pairs of every entry into pp[e + 1]; pass 1 writes them at
@@ -205,10 +205,20 @@ bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
         }
         pp[e + 1] = (int)total;
     }
+    if (count_only) return true;
     pdst.resize(pp[nnz]);   // left uninitialised (NoInitAlloc): pass 1 writes every entry
     psrc.resize(pp[nnz]);
     run(1);
     return true;
+}
+
+long long gather_ints(int nrows, const std::vector<int> &rp, const std::vector<int> &diag, const std::vector<char> &skip) {
+    long long total = 0;
+    for (int i = 0; i < nrows; i++) {
+        const int len = rp[i + 1] - rp[i];
+        if (len <= kGatherRow && (skip.empty() || !skip[i])) total += (long long)len * (diag[i] - rp[i]);
+    }
+    return total;
 }
 
 long long build_gather(int nrows, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &diag,
@@ -470,7 +480,7 @@ __global__ void fill_pending_kernel(size_t len, double *__restrict__ x) {
 }
 
 struct FactorDfArgs {
-    int n, max_row;          // rows to factor; longest row that goes through shared memory
+    int n, pair_row;         // rows to factor; longest row that goes through shared memory
     const int *rows, *rp, *ci, *diag, *pp, *pdst, *psrc, *gsrc;
     const long long *goff;
     const double *vals;      // A's values
@@ -690,7 +700,7 @@ __global__ void __launch_bounds__(256) factor_df_kernel(FactorDfArgs a) {
         const long long go = __ldg(a.goff + i);
         const int *gs = a.gsrc + go;
         bool ok = true;
-        if (RMAX == 8 && go < 0) ok = df_long_row(a, i, df_rows + (size_t)(threadIdx.x >> 5) * a.max_row, lim);
+        if (RMAX == 8 && go < 0) ok = df_long_row(a, i, df_rows + (size_t)(threadIdx.x >> 5) * a.pair_row, lim);
         else if (RMAX == 1 || len <= 32) ok = df_row<1, RMAX == 8 ? 8 : 4>(a, i, rs, len, nl, gs, lane, lim);
         else if (RMAX == 2 || len <= 64) ok = df_row<2, 4>(a, i, rs, len, nl, gs, lane, lim);
         else if (RMAX == 8 && len <= 128) ok = df_row<4, 2>(a, i, rs, len, nl, gs, lane, lim);
@@ -1245,12 +1255,12 @@ bpf_status prec_load_values(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     return BPF_SUCCESS;
 }
 
-// Data-flow factorization.  Rows too long for gather lists go through shared memory, eight warps per
+// Data-flow factorization.  Rows without gather lists go through shared memory, eight warps per
 // CTA while they fit (3,600 entries), else as many as do; longer rows are not taken.
 bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const int *order, int rows, const double *vals, bool *taken) {
     *taken = false;
     int wpb = 8;
-    const size_t row_bytes = P->max_row > kGatherRow ? sizeof(double) * (size_t)P->max_row : 0;
+    const size_t row_bytes = sizeof(double) * (size_t)P->pair_row;
     while (wpb > 1 && wpb * row_bytes > (size_t)ctx->max_smem_optin) wpb >>= 1;
     if (wpb * row_bytes > (size_t)ctx->max_smem_optin) return BPF_SUCCESS;
     *taken = true;
@@ -1259,11 +1269,13 @@ bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const int *order, int rows, cons
     BPF_LAUNCHED(ctx);
     if (rows == 0) return BPF_SUCCESS;
     const size_t smem = wpb * row_bytes;
-    auto kern = P->max_row <= 32 ? factor_df_kernel<1> : P->max_row <= 64 ? factor_df_kernel<2> : factor_df_kernel<8>;
+    auto kern = P->pair_row > 0 || P->max_row > 64 ? factor_df_kernel<8>
+                : P->max_row > 32                  ? factor_df_kernel<2>
+                                                   : factor_df_kernel<1>;
     BPF_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int grid = 1;
     BPF_TRY(coop_grid(ctx, kern, 32 * wpb, smem, ceil_div(rows, wpb), &grid));
-    FactorDfArgs a{rows, P->max_row, order, P->rp, P->ci, P->diag, P->pp, P->pdst, P->psrc, P->gsrc, P->goff,
+    FactorDfArgs a{rows, P->pair_row, order, P->rp, P->ci, P->diag, P->pp, P->pdst, P->psrc, P->gsrc, P->goff,
                    vals, P->fsrc, P->fv, sweep_store(P), ctx->dstat};
     void *args[] = {&a};
     KScope ks(ctx, BPF_KC_FACTOR, 44.0 * P->nnz + 12.0 * (P->n + 1) + 8.0 * P->npairs, 2.0 * P->npairs);

@@ -108,14 +108,22 @@ void run_threads(bool large, const F &f) {
     f();
     for (auto &th : pool) th.join();
 }
-// Gather lists (bpf_prec::goff, gsrc) of the first `rows` rows but those `skip` marks (if not empty);
-// returns the number of updates.
+// Gather lists (bpf_prec::goff, gsrc) of the first `rows` rows of up to kGatherRow entries but those `skip` marks
+// (if not empty); returns the number of updates.
 constexpr int kGatherRow = 256;
+// A list has an int per L entry and entry of its row, updated or not, where an update is two ints as a pair: lists
+// are made while they take 256 MB or no more than the pairs would beyond that (grids: 25 ints a row), and never
+// past 2^32 ints.
+constexpr long long kGatherFree = 1LL << 26;
+inline bool gather_fits(long long ints, long long pairs) {
+    return ints <= kGatherFree || (ints <= (1LL << 32) && ints <= kGatherFree + 2 * pairs);
+}
+long long gather_ints(int rows, const std::vector<int> &rp, const std::vector<int> &diag, const std::vector<char> &skip);
 long long build_gather(int rows, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &diag,
                        const std::vector<char> &skip, std::vector<long long> &goff, PairVec &gsrc);
-// false (and empty outputs) when the pair count exceeds INT_MAX
+// false (and empty outputs) when the pair count exceeds INT_MAX; count_only: pp alone
 bool build_pairs(int n, const int *rp, const int *ci, const int *diag, bool ic,
-                 std::vector<int> &pp, PairVec &pdst, PairVec &psrc);
+                 std::vector<int> &pp, PairVec &pdst, PairVec &psrc, bool count_only = false);
 // A sweep's factor as the byte stream of the column solves (trsv_col.cu).
 struct TriStream {
     std::vector<unsigned char> bytes;
@@ -141,12 +149,12 @@ struct bpf_prec {
     // pattern (0-based device copies) and factor values in pattern order
     int *rp = nullptr, *ci = nullptr, *diag = nullptr;
     double *fv = nullptr;
-    // Data-flow factorization: the longest row, and the source entry of A per pattern entry (null: the
+    // Data-flow factorization: the longest row, the longest that goes by pairs (0: none), and the source entry of A per pattern entry (null: the
     // same position; -1: fill, zero)
-    int max_row = 0;
+    int max_row = 0, pair_row = 0;
     int *fsrc = nullptr;
     // Rows of up to kGatherRow entries: per L entry and entry of the row, the position of U's entry that
-    // updates it (-1: none), from goff[i] on (-1: a longer row, which goes by its update pairs).
+    // updates it (-1: none), from goff[i] on (-1: a longer row, or lists past their limit: by its update pairs).
     long long *goff = nullptr;
     int *gsrc = nullptr;
     int *pp = nullptr, *pdst = nullptr, *psrc = nullptr;

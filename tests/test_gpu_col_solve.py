@@ -162,3 +162,50 @@ def test_a_stream_past_its_limit_is_not_kept(bpf):
     Y = P.ldiv(B).cpu().numpy()
     assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
     assert used < 700 << 20
+
+
+def test_update_lists_past_their_limit(bpf):
+    """Rows of 162 entries with 159 updates each: lists would take 622 MB, pairs 8."""
+    import torch
+
+    n, w = 6000, 160
+    A = sp.csr_matrix(sp.diags([np.full(n - d, 0.5 / w) for d in range(w + 1)] + [np.full(n - 1, 0.1)],
+                               [-d for d in range(w + 1)] + [1]) + 2.0 * sp.eye(n))
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    P = bpf.ilu0(Ad, 1)
+    used = free - torch.cuda.mem_get_info()[0]
+    F = O.ilu0(A)
+    np.testing.assert_allclose(P.P.nzVal.cpu().numpy(), F.data, rtol=1e-12)
+    P.refactor(2.0 * Ad.nzVal)
+    at = np.flatnonzero(A.indices == np.repeat(np.arange(n), np.diff(A.indptr)))   # the diagonal
+    np.testing.assert_allclose(P.P.nzVal.cpu().numpy()[at], 2.0 * F.data[at], rtol=1e-12)
+    assert used < 200 << 20
+
+
+def test_factors_by_lists_and_by_pairs_agree(bpf):
+    """Short rows beside one of 300 entries (which takes all update pairs along), and rows of up to 64 by lists alone."""
+    for per_row, long in ((4, 300), (20, 0)):
+        A = _random(2000, per_row, per_row).tolil()
+        if long:
+            A[1500, :long] = 1e-3
+        A = A.tocsr()
+        A.sort_indices()
+        P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), 1)
+        F = O.ilu0(A)
+        np.testing.assert_allclose(P.P.nzVal.cpu().numpy(), F.data, rtol=1e-11, atol=1e-11 * np.abs(F.data).max())
+
+
+def test_too_many_update_pairs_are_refused(bpf):
+    """387 dense blocks of 256 rows: 387 x 5,559,680 pairs exceed 2^31 - 1."""
+    import torch
+
+    m, nb = 256, 387
+    n = m * nb
+    ptr = torch.arange(0, n * m + 1, m, dtype=torch.int32, device="cuda")
+    col = (torch.arange(m, dtype=torch.int32, device="cuda").repeat(n).view(nb, m * m)
+           + m * torch.arange(nb, dtype=torch.int32, device="cuda")[:, None]).reshape(-1)
+    A = bpf.CuSparseMatrixCSR(ptr, col, torch.ones(n * m, dtype=torch.float64, device="cuda"), n)
+    with pytest.raises(bpf.BPFError, match="2\\^31"):
+        bpf.ilu0(A, 1)
