@@ -877,6 +877,7 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
               tri_to_stream(up, BPF_F64, nring, (int)cs[0].coff.size() - 1, n, true, pos1, cs[1], tpos[1]);
     }
     P->col = col;
+    P->lev = !col;
     if (col) {
         for (int q = 0; q < n; q++) pos01[q] = q < s ? pos0[up.rows[q]] : q;
         std::vector<int> b0(n), b1(n);   // positions of the block's rows

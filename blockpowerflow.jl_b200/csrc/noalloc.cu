@@ -102,7 +102,7 @@ extern "C" bpf_status bpf_prec_apply_noalloc(bpf_prec *P, int p, const double *X
     BPF_TRY(noalloc_scratch(ctx, &buf));
     for (int c0 = 0; c0 < p; c0 += chunk) {
         const int pc = std::min(chunk, p - c0);
-        if (P->col) {   // column solves: in place on a column-major copy
+        if (prec_by_columns(ctx, P, pc, false)) {   // column solves: in place on a column-major copy
             BPF_CUDA(ctx, cudaMemcpy2DAsync(buf, sizeof(double) * n, X + (size_t)c0 * ldx, sizeof(double) * ldx,
                                             sizeof(double) * n, pc, cudaMemcpyDeviceToDevice, ctx->stream));
             BPF_TRY(trsv_col(ctx, P, pc, buf, n, buf, n));
@@ -111,7 +111,8 @@ extern "C" bpf_status bpf_prec_apply_noalloc(bpf_prec *P, int p, const double *X
             continue;
         }
         BPF_TRY(colmajor_to_rowmajor(ctx, n, pc, X + (size_t)c0 * ldx, ldx, buf));
-        BPF_TRY(prec_apply_rowmajor(ctx, P, pc, buf, buf));
+        if (P->kind == PREC_BJ) BPF_TRY(prec_apply_rowmajor(ctx, P, pc, buf, buf));
+        else BPF_TRY(prec_apply_levels(ctx, P, pc, buf, buf));
         BPF_TRY(rowmajor_to_colmajor(ctx, n, pc, buf, Y + (size_t)c0 * ldy, ldy));
     }
     return BPF_SUCCESS;

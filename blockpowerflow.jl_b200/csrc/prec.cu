@@ -342,6 +342,7 @@ SweepStore sweep_store(const bpf_prec *P) {
     const TriDev *t[2] = {&P->lower, &P->upper};
     for (int w = 0; w < 2; w++) {
         s.tpos[w] = P->tpos[w];
+        s.lpos[w] = P->lpos[w];
         s.val[w] = t[w]->val;
         s.valf[w] = t[w]->valf;
         s.dinv[w] = t[w]->dinv;
@@ -1202,6 +1203,37 @@ static bpf_status trsv2_dispatch(bpf_ctx *ctx, const TriDev &t0, const TriDev &t
     return set_error(ctx, BPF_ERR_NOT_SUPPORTED, "triangular solve: p=%d > 256 per call", p);
 }
 
+// Estimated microseconds of both ways, from 716 measured solves (grids of 100 to 26,000 buses in natural, minimum-
+// degree and reverse Cuthill-McKee order, meshes, bands, random and wide-level patterns, 1 to 256 columns).
+// A column solve takes a CTA a column: its levels' barriers, and the rows and groups of entries that one SM gets
+// through, once per wave of columns.  The level-sorted kernels share rows over the chip, at a hop through L2 a
+// level: natural-order grids (28 levels) are theirs from 14,000 rows and 17 columns on (17,098 rows, 64 columns
+// 95 / 117 us, 23,748 rows 99 / 173), minimum-degree order (68 levels) stays with the columns at 17,098 rows (173 /
+// 136) but not at 23,748 (56 levels, 157 / 186), reverse Cuthill-McKee order (900 levels and more) always does
+// (2,160 / 640), as do up to 16 columns (17,098 rows, one column, 224 / 131), except where a level holds thousands
+// of long rows (17,000 rows of 80 entries in 4 levels, 64 columns 120 / 670).  The columns must win by a
+// tenth.  Row-major blocks: the columns' copies on one side, none on the other.
+bool prec_by_columns(const bpf_ctx *ctx, const bpf_prec *P, int p, bool rowmajor) {
+    if (!P->col || !P->lev) return P->col;
+    p = std::min(p, 256);
+    const double n = P->n, nnz = (double)P->lower.nnz + P->upper.nnz + P->n, levels = P->lower.nlev + P->upper.nlev;
+    const double waves = ceil_div(p, ctx->num_sms), f = P->fdtype == BPF_F32 ? 0.7 : 1.0;
+    double col = (5.0 + 0.45 * P->col_stages + f * std::max(0.0021 * n + 0.05 * P->col_groups, 0.08 * P->col_groups)) *
+                 (0.3 + 0.7 * waves);
+    double lev;
+    if (p <= 16) lev = 24.0 + 3.2 * levels + 0.9 * P->col_chain + 1.5e-5 * nnz;
+    else if (std::max(P->lower.max_level_rows, P->upper.max_level_rows) <= 32) return true;   // one CTA, level by level
+    else
+        lev = 16.0 + 2.4 * levels + (p <= 64 ? 0.25 : p <= 128 ? 0.37 : 1.07) * P->long_rows +
+              (p > 128 ? 0.4 * P->col_chain : 0.0) + 8e-7 * nnz * std::max(p, 100) + 5e-6 * n * p;
+    if (rowmajor && p > 1) {   // two transposes of the block, ours or the caller's (in place up to 3,072 rows)
+        const double turn = 2.0 * (2.0 + 2e-6 * n * p);
+        if (P->n > 3072) col += turn;
+        lev -= turn;
+    }
+    return 1.1 * col <= lev;
+}
+
 // Y = P \ X on row-major n x p blocks (FP64 in/out).  Blocks wider than 256 columns are
 // solved in 256-column slices by the caller.
 bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X,
@@ -1212,7 +1244,11 @@ bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const dou
         return set_error(ctx, BPF_ERR_NOT_SUPPORTED,
                          "reordered preconditioner: %d right-hand sides exceed the %d-column scratch "
                          "reserved for it", p, P->zcols);
-    if (P->col) return trsv_col_rowmajor(ctx, P, p, X, Y, gate);
+    if (prec_by_columns(ctx, P, p, true)) return trsv_col_rowmajor(ctx, P, p, X, Y, gate);
+    return prec_apply_levels(ctx, P, p, X, Y, gate);
+}
+
+bpf_status prec_apply_levels(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y, const int *gate) {
     if (P->fdtype == BPF_F32)
         return trsv2_dispatch<float, false, false>(ctx, P->lower, P->upper, p, X, Y, gate, P->perm, P->zbuf,
                                                    P->sf_flags, ++P->sf_epoch);
@@ -1223,7 +1259,7 @@ bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const dou
 bpf_status prec_reserve_z(bpf_ctx *ctx, bpf_prec *P, int p) {
     if (!P->perm || p <= P->zcols) return BPF_SUCCESS;
     const int cols = std::min(std::max(p, 1), 256);
-    if (P->col) {   // the column solves need no scratch: only the width is kept
+    if (!P->lev) {   // the column solves need no scratch: only the width is kept
         P->zcols = cols;
         return BPF_SUCCESS;
     }
@@ -1287,7 +1323,7 @@ bpf_status factor_df(bpf_ctx *ctx, bpf_prec *P, const int *order, int rows, cons
 bpf_status prec_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
     if (P->kind == PREC_ILU0 && P->n > 0) {
         bool taken = false;
-        BPF_TRY(factor_df(ctx, P, P->lower.rows, P->n, vals, &taken));
+        BPF_TRY(factor_df(ctx, P, P->forder ? P->forder : P->lower.rows, P->n, vals, &taken));
         if (taken) return BPF_SUCCESS;
     }
     BPF_TRY(prec_load_values(ctx, P, vals));

@@ -129,6 +129,7 @@ struct TriStream {
     std::vector<unsigned char> bytes;
     std::vector<int> coff, cslab, head;   // per chunk: byte offset, first slab; slab headers
     int diag = 0, nstage = 0;
+    long long groups = 0, chain = 0;   // groups of entries; their sum over the stages' longest slabs
 };
 // ntot: unknowns (rows from t.n on keep their positions); lu: long rows over a whole warp
 bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
@@ -170,6 +171,7 @@ struct bpf_prec {
     // cta_nmax / cta_wmax: most entries to eliminate, longest storage of a CTA's row.
     int tail_s = 0, tail_m = 0, tail_mp = 0, nshort = 0, nlong = 0, cta_nmax = 0, cta_wmax = 0;
     long long cta_pairs = 0;
+    // (ILU(0) kept for column solves: the stream's order, long rows of a level first.)
     int *forder = nullptr;
     int *fend = nullptr;
     double *tail_S = nullptr, *tail_F = nullptr, *tail_inv = nullptr;
@@ -197,10 +199,13 @@ struct bpf_prec {
     // level-sorted val, or the stream in units of the factor type), -1 nowhere, -2 - index its
     // reciprocal (the level-sorted dinv, or the stream).
     int *tpos[2] = {nullptr, nullptr};
-    // Column solves (trsv_col.cu): each sweep's factor as a byte stream in place of the level-sorted
-    // storage; pos0[r] / pos1[r] = forward / backward position of the block's row r, pos01[q] =
+    // Column solves (trsv_col.cu): each sweep's factor as a byte stream; lev: the level-sorted storage is kept too,
+    // at lpos (as tpos), because some number of columns goes faster that way (prec_by_columns);
+    // sums and longest rows of both sweeps that tell which.  pos0[r] / pos1[r] = forward / backward position of the block's row r, pos01[q] =
     // forward position of the row at backward position q.
-    bool col = false;
+    bool col = false, lev = true;
+    int *lpos[2] = {nullptr, nullptr};
+    double col_groups = 0.0, col_chain = 0.0, col_stages = 0.0, long_rows = 0.0;
     struct ColStream {
         unsigned char *bytes = nullptr;
         int *coff = nullptr, *cslab = nullptr, *head = nullptr;
@@ -248,6 +253,10 @@ bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, siz
                     const int *gate = nullptr, size_t step = 1);
 bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y,
                              const int *gate = nullptr);
+// Whether a solve of p columns goes by the column solves or by the level-sorted kernels.
+bool prec_by_columns(const bpf_ctx *ctx, const bpf_prec *P, int p, bool rowmajor);
+// Row-major blocks by the level-sorted kernels (no allocation).
+bpf_status prec_apply_levels(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, double *Y, const int *gate = nullptr);
 bpf_status prec_apply_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X,
                                double *Y, const int *gate = nullptr);
 // Reordered preconditioners: make the factor-ordered scratch hold p columns (allocates when it
@@ -263,14 +272,26 @@ bpf_status lu_solve_push_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, double
 }  // namespace bpf
 
 namespace bpf {
-// The storage of the two sweeps that a factor entry goes to (bpf_prec::tpos), CSR or stream.
+// The storage of the two sweeps that a factor entry goes to: CSR or stream (bpf_prec::tpos), and CSR besides the
+// stream (lpos).
 struct SweepStore {
-    const int *tpos[2];
+    const int *tpos[2], *lpos[2];
     double *val[2], *dinv[2];      // level-sorted storage, FP64 and FP32
     float *valf[2], *dinvf[2];
     unsigned char *stream[2];      // or the streams (column solves), of FP32 values if f32
     int col, f32;
 };
+
+__device__ __forceinline__ void sweep_put_level(const SweepStore &s, int w, int t, double v) {
+    const int k = t >= 0 ? t : -2 - t;
+    if (t >= 0) {
+        s.val[w][k] = v;
+        s.valf[w][k] = (float)v;
+    } else {
+        s.dinv[w][k] = v;
+        s.dinvf[w][k] = (float)v;
+    }
+}
 
 __device__ __forceinline__ void sweep_put(const SweepStore &s, int e, double x) {
 #pragma unroll
@@ -279,16 +300,10 @@ __device__ __forceinline__ void sweep_put(const SweepStore &s, int e, double x) 
         if (t == -1) continue;
         const double v = t >= 0 ? x : 1.0 / x;
         const int k = t >= 0 ? t : -2 - t;
-        if (s.col) {
-            if (s.f32) reinterpret_cast<float *>(s.stream[w])[k] = (float)v;
-            else reinterpret_cast<double *>(s.stream[w])[k] = v;
-        } else if (t >= 0) {
-            s.val[w][k] = v;
-            s.valf[w][k] = (float)v;
-        } else {
-            s.dinv[w][k] = v;
-            s.dinvf[w][k] = (float)v;
-        }
+        if (!s.col) sweep_put_level(s, w, t, v);
+        else if (s.f32) reinterpret_cast<float *>(s.stream[w])[k] = (float)v;
+        else reinterpret_cast<double *>(s.stream[w])[k] = v;
+        if (s.lpos[w]) sweep_put_level(s, w, __ldg(s.lpos[w] + e), v);
     }
 }
 

@@ -540,6 +540,7 @@ bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
     for (int l = 0; l < t.nlev; l++) {
         int rest = 0;   // further parts the widest slab needs (each a stage of its own)
         for (int pass = 0; pass <= rest; pass++, stage++) {
+            int longest = 0;
             for (int q0 = t.lev_ptr[l], rows; q0 < t.lev_ptr[l + 1]; q0 += rows) {
                 const int wide = t.rp[q0 + 1] - t.rp[q0] > wide_row;
                 int w = 0;
@@ -553,10 +554,14 @@ bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
                 rest = std::max(rest, parts - 1);
                 if (pass >= parts) continue;
                 const int g0 = pass * gmax;
-                total += part_bytes(std::min(gmax, ng - g0));
+                const int groups = std::min(gmax, ng - g0);
+                total += part_bytes(groups);
                 if (total > kStreamMax) return false;
-                add(Part{q0, rows, (wide ? 128 : 4) * g0, std::min(gmax, ng - g0), pass == parts - 1 ? 1 : 0, stage, wide});
+                out.groups += groups;
+                longest = std::max(longest, groups);
+                add(Part{q0, rows, (wide ? 128 : 4) * g0, groups, pass == parts - 1 ? 1 : 0, stage, wide});
             }
+            out.chain += longest;
         }
     }
     close();

@@ -209,3 +209,57 @@ def test_too_many_update_pairs_are_refused(bpf):
     A = bpf.CuSparseMatrixCSR(ptr, col, torch.ones(n * m, dtype=torch.float64, device="cuda"), n)
     with pytest.raises(bpf.BPFError, match="2\\^31"):
         bpf.ilu0(A, 1)
+
+
+def _wide_levels(n, per_row):
+    """Four levels of n / 4 rows, each reading (and read by) random rows of its neighbours."""
+    rng = np.random.default_rng(n)
+    h = n // 4
+    r = np.repeat(np.arange(h, 4 * h), per_row)
+    c = rng.integers(0, h, len(r)) + (r // h - 1) * h
+    A = sp.coo_matrix((rng.standard_normal(2 * len(r)), (np.concatenate([r, c]), np.concatenate([c, r]))), shape=(n, n)).tocsr()
+    return (A + sp.diags(1.0 + np.asarray(abs(A).sum(axis=1)).ravel())).tocsr()
+
+
+# one factor whose solves take either way by their number of columns: both kinds of storage, before and after new
+# values, in place, overlapping, and inside a solver.  A substitution's computed y solves a system whose entries are
+# off by at most k eps each (k: the longest row, a reciprocal and the roundings of values and results come on top), so
+# |X - L U Y| <= 2 (k + 4) eps |L| |U| |Y|; the residual's own rounding is another 2 k eps of the same.
+@pytest.mark.parametrize("dtype,eps", [("float64", 2.0**-52), ("float32", 2.0**-23)])
+@pytest.mark.parametrize("case", ["grid natural", "grid AMD", "wide natural", "wide RCM"])
+def test_both_ways_of_one_factor(bpf, case, dtype, eps):
+    import torch
+
+    kind, ordering = case.split()
+    A = bpf.grid.synthetic_jacobian(12500) if kind == "grid" else _wide_levels(8000, 40)
+    n = A.shape[0]
+    Ad = bpf.CuSparseMatrixCSR.from_scipy(A)
+    P = bpf.ilu0(Ad, 200, dtype, ordering=ordering)
+    perm = P.perm
+    S = sp.csr_matrix(A[perm][:, perm])
+    S.sort_indices()
+
+    def check(X, Y):
+        F = sp.csr_matrix((P.P.nzVal.cpu().numpy(), S.indices, S.indptr), shape=S.shape)
+        L, U = sp.tril(F, -1, format="csr") + sp.eye(n, format="csr"), sp.triu(F, format="csr")
+        c = 4 * (np.diff(S.indptr).max() + 4) * eps
+        Y = Y.cpu().numpy()[perm]
+        assert np.all(np.abs(X[perm] - L @ (U @ Y)) <= c * (abs(L) @ (abs(U) @ np.abs(Y))))
+
+    X = np.random.default_rng(7).standard_normal((n, 200))
+    for scale in (1.0, 4.0):
+        P.refactor(scale * Ad.nzVal)
+        for p in (1, 5, 16, 17, 64, 65, 128, 129, 200):
+            check(X[:, :p], P.ldiv(_block(X[:, :p])))
+    P.refactor(Ad.nzVal)
+    for p in (3, 40):
+        W = _block(X[:, :p])
+        bpf.ldiv_(W, P, W)
+        check(X[:, :p], W)
+        W = _block(X[:, :p + 1])
+        bpf.ldiv_(W[:, 1:], P, W[:, :p])
+        check(X[:, :p], W[:, 1:])
+    B = np.random.default_rng(8).standard_normal((n, 20))
+    for p in (3, 20):
+        Z, st = bpf.block_gmres(Ad, torch.as_tensor(B[:, :p], device="cuda"), N=P, ldiv=True, memory=250, atol=0.0, rtol=1e-8)
+        assert st.solved and np.linalg.norm(B[:, :p] - A @ Z.cpu().numpy()) <= 1.01e-8 * np.linalg.norm(B[:, :p])
