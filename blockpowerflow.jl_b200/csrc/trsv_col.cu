@@ -21,7 +21,9 @@
 //    is a zero times the unknown after the last, which is zero: no branch or predicate between the
 //    barrier and the result (with them a slab took ~1,000 cycles).
 //  * An LU's long rows (more than kWideRow entries) are slabs of their own, a row's entries over the
-//    32 lanes and a warp sum at the end.
+//    32 lanes and a warp sum at the end; an ILU(0)'s too, past kWideIlu entries, where the level's slab would be
+//    mostly padding (a slab of one row takes 1,280 bytes per four entries: 3,000 levels of one row of 200
+//    entries made 186 MB and 18.0 ms, 2.2 ms so).
 //  * Slab g goes to warp g mod nw, levels notwithstanding: a warp fetches its next slab's
 //    entries, if they have arrived, then passes the level barriers that separate it from the last,
 //    so in a long chain of narrow levels the fetches of the coming levels overlap the current one.
@@ -39,7 +41,8 @@
 // of level barriers (113 / 868 us: nearly every warp waits, and the polls take the issue slots from
 // the others).
 //
-// Same products and summation order per row as the level-scheduled kernel: identical results.
+// Same products and summation order per row as the level-scheduled kernel, but for the rows over all lanes:
+// identical results.
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -52,11 +55,11 @@ namespace bpf {
 
 constexpr int kChunk = 16384;      // bytes of a chunk, at most
 constexpr int kWideRow = 16;       // entries past which an LU's row takes a whole warp
+constexpr int kWideIlu = 32;       // and an ILU(0)'s or IC(0)'s, where its level has too few of them for its lanes
 constexpr int kColWarps = 23;      // computing warps, at most
 constexpr int kChunkRing = 6;      // chunks in flight, at most (as many as fit beside the column)
-// Bytes of a sweep's stream, at most: offsets are int, and a slab of one row takes 1,280 bytes per four entries,
-// up to 32 times the level-sorted form where every level holds one long row (12,000 rows of 200 lower
-// entries: 768 MB for 48).  Grids' factors take 1 to 20 MB.
+// Bytes of a sweep's stream, at most (offsets are int): 25 million entries of long rows, or every row with a level
+// of its own.  Grids' factors take 1 to 20 MB.
 constexpr size_t kStreamMax = size_t(1) << 28;
 
 // A group of four entries of 32 rows: [lane][4] 16-bit columns, then the values as [2][lane][2]
@@ -460,7 +463,6 @@ bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const doubl
 // False, with out and tpos in part filled, when the stream would pass kStreamMax.
 bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool lu, std::vector<int> &pos,
                    TriStream &out, std::vector<int> &tpos) {
-    const int wide_row = lu ? kWideRow : 2147483647;
     const size_t es = fdtype == BPF_F32 ? sizeof(float) : sizeof(double);
     const int n = t.n;
     std::vector<int> ord(n);
@@ -542,11 +544,17 @@ bool tri_to_stream(TriHost &t, int fdtype, int nring, int chunk0, int ntot, bool
         for (int pass = 0; pass <= rest; pass++, stage++) {
             int longest = 0;
             for (int q0 = t.lev_ptr[l], rows; q0 < t.lev_ptr[l + 1]; q0 += rows) {
-                const int wide = t.rp[q0 + 1] - t.rp[q0] > wide_row;
+                const int first = t.rp[q0 + 1] - t.rp[q0];
+                int wide = lu ? first > kWideRow : 0;
+                if (!lu && first > kWideIlu) {   // the rows of this slab are no longer than its first one
+                    int cnt = 1;
+                    while (cnt < 32 && q0 + cnt < t.lev_ptr[l + 1] && t.rp[q0 + cnt + 1] - t.rp[q0 + cnt] > kWideIlu) cnt++;
+                    wide = cnt * ((first + 127) / 128) < (first + 3) / 4;
+                }
                 int w = 0;
                 for (rows = 0; rows < (wide ? 1 : 32) && q0 + rows < t.lev_ptr[l + 1]; rows++) {
                     const int len = t.rp[q0 + rows + 1] - t.rp[q0 + rows];
-                    if (!wide && len > wide_row) break;
+                    if (lu && !wide && len > kWideRow) break;
                     w = std::max(w, len);
                 }
                 const int ng = wide ? (w + 127) / 128 : (w + 3) / 4;

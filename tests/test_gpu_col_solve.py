@@ -144,9 +144,9 @@ def test_row_major_blocks(bpf, n, p, f32):
     assert np.linalg.norm(B - A @ X.cpu().numpy()) <= 1.01e-8 * np.linalg.norm(B)
 
 
-def test_a_stream_past_its_limit_is_not_kept(bpf):
-    """Single-row levels of 160 entries: the column solves' storage would be 307 MB, most of it padding.  The
-    level-sorted form takes 20 MB, the lists of the factorization 618."""
+def test_long_rows_in_levels_of_their_own(bpf):
+    """Levels of one row of 160 entries: over the lanes of a warp they take 15 MB (in slabs of 32 rows 307), the lists
+    of the factorization 618."""
     import torch
 
     n, w, p = 6000, 160, 3
@@ -162,6 +162,46 @@ def test_a_stream_past_its_limit_is_not_kept(bpf):
     Y = P.ldiv(B).cpu().numpy()
     assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
     assert used < 700 << 20
+
+
+def test_a_stream_past_its_limit_is_not_kept(bpf):
+    """A dense lower triangle of 7,600 rows: 292 MB."""
+    n, p = 7600, 3
+    ptr = np.concatenate([[0], np.cumsum(np.arange(1, n + 1))])
+    col = np.concatenate([np.arange(i + 1) for i in range(n)])
+    val = np.full(len(col), 0.5 / n)
+    val[ptr[1:] - 1] = 2.0
+    A = sp.csr_matrix((val, col, ptr), shape=(n, n))
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), p)
+    X = np.random.default_rng(6).standard_normal((n, p))
+    ref = O.prec_apply(1, O.ilu0(A), X)
+    Y = P.ldiv(_block(X)).cpu().numpy()
+    assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+# rows over the lanes of a warp: in one part, in several (more than 1,536 entries of FP64, 2,688 of FP32), several rows in
+# a level, and levels with too many long rows for it; the bound is test_both_ways_of_one_factor's
+@pytest.mark.parametrize("dtype,eps", [("float64", 2.0**-52), ("float32", 2.0**-23)])
+@pytest.mark.parametrize("kind", ["arrow", "few", "many"])
+def test_rows_over_a_warp(bpf, kind, dtype, eps):
+    if kind == "arrow":
+        A = _arrow(4000)
+    else:
+        A = sp.csr_matrix(_random(1200, 3, 11))
+        rows = np.arange(600, 600 + (7 if kind == "few" else 90))
+        extra = sp.coo_matrix((np.full(len(rows) * 200, 1e-2), (np.repeat(rows, 200), np.tile(np.arange(0, 400, 2), len(rows)))),
+                              shape=A.shape)
+        A = sp.csr_matrix(A + extra + extra.T + 20.0 * sp.eye(1200))
+    A.sort_indices()
+    n = A.shape[0]
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), 4, dtype)
+    F = sp.csr_matrix((P.P.nzVal.cpu().numpy(), A.indices, A.indptr), shape=A.shape)
+    L, U = sp.tril(F, -1, format="csr") + sp.eye(n, format="csr"), sp.triu(F, format="csr")
+    c = 4 * (np.diff(A.indptr).max() + 4) * eps
+    X = np.random.default_rng(4).standard_normal((n, 4))
+    for p in (1, 4):
+        Y = P.ldiv(_block(X[:, :p])).cpu().numpy()
+        assert np.all(np.abs(X[:, :p] - L @ (U @ Y)) <= c * (abs(L) @ (abs(U) @ np.abs(Y))))
 
 
 def test_update_lists_past_their_limit(bpf):
