@@ -256,11 +256,11 @@ __device__ __forceinline__ unsigned barrier_gen_start(DevStatus *ds) {
 // ------------------------------------------------------------------------------------
 // launchers implemented in the .cu files
 // ------------------------------------------------------------------------------------
-// Column-major (ld) <-> row-major (n x p, ld = p) block conversions.
+// Column-major (ld) <-> row-major (n x p, ld = p) block conversions (skipped when *gate is 0).
 bpf_status colmajor_to_rowmajor(bpf_ctx *ctx, int n, int p, const double *src, int ld,
-                                double *dst);
+                                double *dst, const int *gate = nullptr);
 bpf_status rowmajor_to_colmajor(bpf_ctx *ctx, int n, int p, const double *src, double *dst,
-                                int ld);
+                                int ld, const int *gate = nullptr);
 
 // CSR SpMM on row-major blocks: Y = alpha*A*X + beta*Y, or (residual) Y = B - A*X when
 // B != nullptr.  base = index base of the CSR arrays.

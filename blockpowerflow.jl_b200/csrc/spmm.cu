@@ -402,7 +402,8 @@ bpf_status spmm_colmajor(bpf_ctx *ctx, int n, long long nnz, const int *rp, cons
 // layout conversions (32x32 tiles through shared memory)
 // ------------------------------------------------------------------------------------
 __global__ void cm_to_rm_kernel(int n, int p, const double *__restrict__ src, int ld,
-                                double *__restrict__ dst) {
+                                double *__restrict__ dst, const int *gate) {
+    if (gate && *gate == 0) return;
     __shared__ double tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -417,7 +418,8 @@ __global__ void cm_to_rm_kernel(int n, int p, const double *__restrict__ src, in
 }
 
 __global__ void rm_to_cm_kernel(int n, int p, const double *__restrict__ src,
-                                double *__restrict__ dst, int ld) {
+                                double *__restrict__ dst, int ld, const int *gate) {
+    if (gate && *gate == 0) return;
     __shared__ double tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -432,19 +434,19 @@ __global__ void rm_to_cm_kernel(int n, int p, const double *__restrict__ src,
 }
 
 bpf_status colmajor_to_rowmajor(bpf_ctx *ctx, int n, int p, const double *src, int ld,
-                                double *dst) {
+                                double *dst, const int *gate) {
     if (n == 0 || p == 0) return BPF_SUCCESS;
     dim3 grid(ceil_div(n, 32), ceil_div(p, 32)), block(32, 8);
-    cm_to_rm_kernel<<<grid, block, 0, ctx->stream>>>(n, p, src, ld, dst);
+    cm_to_rm_kernel<<<grid, block, 0, ctx->stream>>>(n, p, src, ld, dst, gate);
     BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;
 }
 
 bpf_status rowmajor_to_colmajor(bpf_ctx *ctx, int n, int p, const double *src, double *dst,
-                                int ld) {
+                                int ld, const int *gate) {
     if (n == 0 || p == 0) return BPF_SUCCESS;
     dim3 grid(ceil_div(n, 32), ceil_div(p, 32)), block(32, 8);
-    rm_to_cm_kernel<<<grid, block, 0, ctx->stream>>>(n, p, src, dst, ld);
+    rm_to_cm_kernel<<<grid, block, 0, ctx->stream>>>(n, p, src, dst, ld, gate);
     BPF_LAUNCHED(ctx);
     return BPF_SUCCESS;
 }

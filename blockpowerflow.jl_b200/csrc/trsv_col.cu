@@ -451,9 +451,9 @@ bpf_status trsv_col_rowmajor(bpf_ctx *ctx, const bpf_prec *P, int p, const doubl
     bpf_status s;
     double *buf = (double *)ws_get(ctx, WS_COL, sizeof(double) * (size_t)P->n * p, &s);
     if (!buf) return s;
-    BPF_TRY(rowmajor_to_colmajor(ctx, P->n, p, X, buf, P->n));
+    BPF_TRY(rowmajor_to_colmajor(ctx, P->n, p, X, buf, P->n, gate));
     BPF_TRY(trsv_col(ctx, P, p, buf, P->n, buf, P->n, gate));
-    return colmajor_to_rowmajor(ctx, P->n, p, buf, P->n, Y);
+    return colmajor_to_rowmajor(ctx, P->n, p, buf, P->n, Y, gate);
 }
 
 // The byte stream of a level-sorted factor.  Rows of a level are re-sorted by length (t.rows, t.rp,
