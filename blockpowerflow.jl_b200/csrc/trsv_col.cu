@@ -157,8 +157,9 @@ struct RingState {
 };
 
 // The producer: brings the chunks of both sweeps in order, a chunk into its slot once every slab of
-// the slot's previous chunk is finished, and counts the arrived ones in r.ready.
-__device__ __forceinline__ void col_produce(const ColArgs &a, unsigned char *ring, RingState &r) {
+// the slot's previous chunk is finished, and counts the arrived ones in r.ready.  Gives up after lim polls
+// without a change (the computing warps' own waits report it), its copies landed.
+__device__ __forceinline__ void col_produce(const ColArgs &a, unsigned char *ring, RingState &r, long long lim) {
     const int total = a.nchunk[0] + a.nchunk[1];
     int issued = 0, arrived = 0, islot = 0, aslot = 0;
     unsigned aparity = 0;
@@ -190,7 +191,14 @@ __device__ __forceinline__ void col_produce(const ColArgs &a, unsigned char *rin
             moved = true;
         }
         if (moved) idle = 0;
-        else if (++idle > 4 * kSpinLimit) return;   // the computing warps' own waits report it
+        else if (++idle > lim) break;
+    }
+    for (; arrived < issued; arrived++) {
+        mbar_wait_bounded(r.full + aslot, aparity);
+        if (++aslot == a.nring) {
+            aslot = 0;
+            aparity ^= 1u;
+        }
     }
 }
 
@@ -199,7 +207,7 @@ __device__ __forceinline__ void col_produce(const ColArgs &a, unsigned char *rin
 // further part of its long rows).
 template <typename TF>
 __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstage, bool diag, unsigned y,
-                                          unsigned ring, RingState &r, int nw, bool ok) {
+                                          unsigned ring, RingState &r, int nw, long long lim, bool ok) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int passed = 0, seen = -1;
     // Headers of the warp's next 32 slabs, one a lane: a global load in flight would be waited for at
@@ -223,9 +231,9 @@ __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstag
         for (; passed < h.z; passed++) col_barrier(32 * nw);
         if (!early) {
             long long it = 0;
-            while (!(ld_relaxed_cta(&r.ready) >= want && mbar_try_wait(r.full + slot, parity)) && ++it < kSpinLimit) {
+            while (!(ld_relaxed_cta(&r.ready) >= want && mbar_try_wait(r.full + slot, parity)) && ++it < lim) {
             }
-            ok = __all_sync(0xffffffffu, it < kSpinLimit);
+            ok = __all_sync(0xffffffffu, it < lim);
             if (!ok) break;
             if (ng > 0) e.load(ch, lane);
         }
@@ -323,8 +331,9 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, s
     __syncthreads();
     if (s_off) return;
     unsigned char *ring = col_smem;
+    const long long lim = ds->wait_limit > 0 ? ds->wait_limit : kSpinLimit;   // polls of the computing warps' waits
     if ((int)(threadIdx.x >> 5) == nw) {
-        if ((threadIdx.x & 31) == 0) col_produce(a, ring, r);
+        if ((threadIdx.x & 31) == 0) col_produce(a, ring, r, 4 * lim);
         return;
     }
     const int n = a.n, tid = threadIdx.x, nt = 32 * nw;
@@ -346,7 +355,7 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, s
             if (i0 + u * nt < n) col_put(y, at[u], (TF)v[u]);
     }
     col_barrier(nt);
-    bool ok = col_sweep<TF>(a.head[0], a.nslab[0], a.nstage[0], a.diag[0] != 0, y, rbase, r, nw, true);
+    bool ok = col_sweep<TF>(a.head[0], a.nslab[0], a.nstage[0], a.diag[0] != 0, y, rbase, r, nw, lim, true);
     if constexpr (std::is_same<TF, double>::value)
         if (a.nb > 0) {
             __shared__ double z[64];
@@ -374,7 +383,7 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, s
     }
     for (int i = n + tid; i <= a.s + 64 * a.nb; i += nt) col_put(y, i, (TF)0);   // (the tail's padding)
     col_barrier(nt);
-    ok = col_sweep<TF>(a.head[1], a.nslab[1], a.nstage[1], a.diag[1] != 0, y, rbase, r, nw, ok);
+    ok = col_sweep<TF>(a.head[1], a.nslab[1], a.nstage[1], a.diag[1] != 0, y, rbase, r, nw, lim, ok);
     if (!ok) atomicCAS(&ds->err, 0, (int)DEV_BARRIER_TIMEOUT);
     for (int i0 = tid; i0 < n; i0 += 8 * nt) {
         int at[8];

@@ -67,3 +67,29 @@ def test_selftest_arguments_are_checked(bpf):
     assert lib.bpf_selftest_grid_barrier(ctx, 1, -1, None) == _lib.BPF_ERR_INVALID_VALUE
     assert lib.bpf_selftest_grid_barrier(ctx, 4, 4, None) == _lib.BPF_ERR_INVALID_VALUE
     assert lib.bpf_ctx_set_wait_limit(ctx, -1) == _lib.BPF_ERR_INVALID_VALUE
+
+
+def test_column_solves_keep_to_the_wait_limit(bpf):
+    """With a limit of one poll some warp of 148 columns' CTAs finds its entries still on their way and gives up; the
+    next call that looks at the status reports it, and the same solve is right again without the limit."""
+    import torch
+
+    from blockpowerflow_b200 import _lib
+
+    lib = _lib.load()
+    ctx = _lib.context()
+    A = bpf.grid.synthetic_jacobian(9000)
+    X = np.random.default_rng(6).standard_normal((A.shape[0], 148))
+    Xd = torch.as_tensor(X, device="cuda").t().contiguous().t()
+    P = bpf.ilu0(bpf.CuSparseMatrixCSR.from_scipy(A), 148)
+    ref = P.ldiv(Xd).cpu().numpy()
+    assert lib.bpf_ctx_set_wait_limit(ctx, 1) == _lib.BPF_SUCCESS
+    try:
+        P.ldiv(Xd)
+    finally:
+        assert lib.bpf_ctx_set_wait_limit(ctx, 0) == _lib.BPF_SUCCESS
+    arrived = C.c_int(-1)
+    assert lib.bpf_selftest_grid_barrier(ctx, 8, -1, C.byref(arrived)) == _lib.BPF_ERR_TIMEOUT
+    assert "timed out" in _lib.last_error(ctx)
+    np.testing.assert_array_equal(P.ldiv(Xd).cpu().numpy(), ref)
+    assert lib.bpf_selftest_grid_barrier(ctx, 8, -1, C.byref(arrived)) == _lib.BPF_SUCCESS
