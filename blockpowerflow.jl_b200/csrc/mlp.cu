@@ -64,18 +64,19 @@ namespace bpf {
 // elementwise kernels
 // ---------------------------------------------------------------------------------------
 // Columns are summed in kNormParts parts (one CTA each: 64 CTAs, one a column, took 36 us for 9 MB), which the
-// reader adds in order: part[which][s][j], which 0: B, 1: X.
+// reader adds in order: part[which][s][j], which 0: B, 1: X / scale (whose squares stay in range at any scale of X).
 constexpr int kNormParts = 8;
 __global__ void __launch_bounds__(256)
-col_norms_kernel(int n, const double *__restrict__ B, int ldb, const double *__restrict__ X, int ldx,
+col_norms_kernel(int n, const double *__restrict__ B, int ldb, const double *__restrict__ X, int ldx, double inv_scale,
                  double *__restrict__ part) {
     const int j = blockIdx.x, s = blockIdx.y;
     const double *V = blockIdx.z ? X + (size_t)j * ldx : B + (size_t)j * ldb;
+    const double f = blockIdx.z ? inv_scale : 1.0;
     const int len = (n + kNormParts - 1) / kNormParts, i1 = min(n, (s + 1) * len);
     double t = 0.0;
 #pragma unroll 8
     for (int i = s * len + threadIdx.x; i < i1; i += 256) {
-        const double v = __ldg(V + i);
+        const double v = f * __ldg(V + i);
         t += v * v;
     }
     __shared__ double red[8];
@@ -184,7 +185,7 @@ loss_grad_kernel(int n, int np, int p, const float *__restrict__ Y, int splits, 
         double w = 0.0, f = 0.0;
         if (j < p && bn[j] > 0.f) {
             f = scale * (double)bn[j];
-            const float tn = (float)(norm_total(part, 1, j) / (f * f));
+            const float tn = (float)(norm_total(part, 1, j) / ((double)bn[j] * (double)bn[j]));
             w = tn > 0.f ? 1.0 / ((double)p * (double)tn) : 0.0;
         }
         s_w[j] = w;
@@ -323,7 +324,7 @@ static bpf_status mlp_forward_core(bpf_mlp *m, int p, const double *B, int ldb, 
     const int H = m->H, np = m->np, P = kMlpBatch;
     const dim3 act(H / 32, P / 8);
     TcProduct q;
-    col_norms_kernel<<<dim3(p, kNormParts, X ? 2 : 1), 256, 0, ctx->stream>>>(m->n, B, ldb, X, ldx, m->norms);
+    col_norms_kernel<<<dim3(p, kNormParts, X ? 2 : 1), 256, 0, ctx->stream>>>(m->n, B, ldb, X, ldx, 1.0 / m->scale, m->norms);
     BPF_LAUNCHED(ctx);
     prep_input_kernel<<<dim3(np / 64, P / 64), 256, 0, ctx->stream>>>(m->n, np, p, B, ldb, m->norms, m->bn, m->Ub, m->Utb);
     BPF_LAUNCHED(ctx);

@@ -72,3 +72,27 @@ def test_product(bpf, M, N, K, ldd, splits, acc):
     assert float((D[:, :N].double() - want).norm()) <= 1e-5 * float(want.norm())
     if splits == 1 or acc:
         assert torch.equal(D[:, N:], rest)
+
+
+@pytest.mark.parametrize("exponent", [-560, 560])
+def test_targets_of_any_scale(bpf, exponent):
+    """X and the scale times a power of two give the same normalized targets, to the bit, although X's squares leave
+    the range of FP64; the loss is added up in any order over at most n p terms (2^-52 each)."""
+    import torch
+
+    from blockpowerflow_b200.learned import PARAMS, WarmStartMLP
+
+    n, p, H, s = 700, 33, 128, 0.05
+    rng = np.random.default_rng(2)
+    B = rng.standard_normal((n, p))
+    X = s * np.linalg.norm(B, axis=0) * rng.standard_normal((n, p)) / np.sqrt(n)
+    out = []
+    for k in (0, exponent):
+        mlp = WarmStartMLP(n, hidden=H, seed=1)
+        mlp.set_scale(s * 2.0**k)
+        loss = mlp.gradients(bpf.colmajor(torch.as_tensor(B, device="cuda")), bpf.colmajor(torch.as_tensor(X * 2.0**k, device="cuda")))
+        out.append((loss, [mlp.param(q, grad=True).cpu().numpy() for q in PARAMS]))
+    assert out[0][0] > 0.5
+    assert abs(out[1][0] - out[0][0]) <= n * p * 2.0**-52 * out[0][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
