@@ -94,10 +94,14 @@ def ld(X) -> int:
 
 
 def to_host(X, negate: bool = False) -> np.ndarray:
-    """A 2-D device block (or its negative) as a host array, in Fortran order if X is column-major."""
-    if X.dim() != 2 or (X.stride(0) != 1 and X.shape[0] > 1) or ld(X) < X.shape[0]:
+    """A block (or its negative) as a host array, in Fortran order if X is column-major; FP64 blocks on a device go
+    through pinned pieces."""
+    import torch
+
+    if (not X.is_cuda or X.dtype != torch.float64 or X.dim() != 2 or (X.stride(0) != 1 and X.shape[0] > 1)
+            or ld(X) < X.shape[0]):
         S = X.cpu().numpy()
-        return np.negative(S, out=S) if negate else S
+        return np.negative(S, out=S if X.is_cuda else None) if negate else S   # a host X's memory is the caller's
     n, p = X.shape
     out = np.empty((p, n)).T
     ctx = _lib.context(X.device.index)

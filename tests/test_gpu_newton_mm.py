@@ -155,3 +155,17 @@ def test_block_to_host(n, p, ldx, negate):
     H = to_host(X, negate)
     assert H.shape == (n, p) and (H.flags.f_contiguous or p == 1 or n == 1)
     np.testing.assert_array_equal(H, -X.cpu().numpy() if negate else X.cpu().numpy())
+
+
+@pytest.mark.parametrize("negate", [False, True])
+def test_to_host_of_other_types(negate):
+    import torch
+
+    from blockpowerflow_b200.sparse import to_host
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    for dtype in (torch.float32, torch.int64):
+        X = torch.arange(6, device="cuda").to(dtype).reshape(2, 3).t()
+        keep = X.cpu().numpy()
+        np.testing.assert_array_equal(to_host(X, negate), -keep if negate else keep)

@@ -87,3 +87,17 @@ def test_jacobian_values_match_the_sparse_product_jacobian(prob):
     cached = prob.__dict__["_coupling_cache"]
     NT.jacobian_values(prob, NT.perturbed_start(prob, 0.05, seed=5))
     assert prob.__dict__["_coupling_cache"] is cached
+
+
+def test_to_host_takes_any_block():
+    """What does not go through the device's pinned pieces comes back as it is; a host block's memory stays untouched."""
+    import torch
+
+    from blockpowerflow_b200.sparse import to_host
+
+    for X in (torch.arange(6, dtype=torch.float32).reshape(3, 2), torch.arange(6, dtype=torch.float64).reshape(2, 3).t(),
+              torch.arange(4, dtype=torch.float64)):
+        keep = X.clone()
+        np.testing.assert_array_equal(to_host(X), keep.numpy())
+        np.testing.assert_array_equal(to_host(X, negate=True), -keep.numpy())
+        assert torch.equal(X, keep)
