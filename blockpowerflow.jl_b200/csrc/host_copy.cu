@@ -8,10 +8,9 @@
 #include <algorithm>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 #include "bpf_internal.cuh"
 
@@ -19,6 +18,7 @@ namespace bpf {
 
 constexpr size_t kSlotDoubles = size_t(1) << 20;   // 8 MB
 constexpr int kSlots = 4;
+constexpr int kCopyThreads = 8;
 
 static void copy_out(double *dst, const double *src, size_t len, bool negate) {
     if (!negate) {
@@ -28,14 +28,15 @@ static void copy_out(double *dst, const double *src, size_t len, bool negate) {
     for (size_t i = 0; i < len; i++) dst[i] = -src[i];
 }
 
-// What the copying threads and the issuing one share: pieces that have arrived, and how many threads
-// are through with each.
+// What the copying threads and the issuing one share: how many threads copy (-1: not known yet), pieces that have
+// arrived, and threads through with the latest.
 struct CopyBoard {
     std::mutex mu;
     std::condition_variable cv;
+    int threads = -1;
     size_t arrived = 0;
     bool stop = false;
-    std::vector<int> done;
+    int done = 0;
 };
 
 }  // namespace bpf
@@ -54,10 +55,10 @@ extern "C" bpf_status bpf_block_to_host(bpf_ctx *ctx, int n, int p, const double
     const size_t piece = linear ? kSlotDoubles : kSlotDoubles / n * n;
     if (total >= kSlotDoubles / 4 && piece > 0 && !ctx->stage) {
         void *s = nullptr;
+        for (int k = 0; k < kSlots; k++)
+            if (!ctx->ev_stage[k]) BPF_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_stage[k], cudaEventDisableTiming));
         if (cudaMallocHost(&s, sizeof(double) * kSlots * kSlotDoubles) == cudaSuccess) ctx->stage = (double *)s;
         else cudaGetLastError();
-        for (int k = 0; k < kSlots && ctx->stage; k++)
-            if (!ctx->ev_stage[k]) BPF_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_stage[k], cudaEventDisableTiming));
     }
     if (total < kSlotDoubles / 4 || piece == 0 || !ctx->stage) {   // small, a huge column, or no pinned memory
         BPF_CUDA(ctx, cudaMemcpy2DAsync(host, sizeof(double) * n, X, sizeof(double) * ldx, sizeof(double) * n, p,
@@ -78,42 +79,40 @@ extern "C" bpf_status bpf_block_to_host(bpf_ctx *ctx, int n, int p, const double
         return e;
     };
     CopyBoard b;
-    b.done.assign(npieces, 0);
     auto part = [&](size_t k, int t, int nt) {   // thread t's share of piece k
         const size_t at = k * piece, len = std::min(piece, total - at);
         const size_t lo = len * t / nt, hi = len * (t + 1) / nt;
         copy_out(host + at + lo, ctx->stage + (k % kSlots) * kSlotDoubles + lo, hi - lo, negate != 0);
     };
-    const int want = (int)std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    int nt = 0;   // copying threads; every one is told before the first piece
-    std::mutex start;
-    start.lock();
+    const int want = (int)std::max(1u, std::min((unsigned)kCopyThreads, std::thread::hardware_concurrency()));
+    std::thread pool[kCopyThreads];
+    int nt = 0;
     auto work = [&](int t) {
-        { std::lock_guard<std::mutex> g(start); }
         for (size_t k = 0; k < npieces; k++) {
+            int threads;
             {
                 std::unique_lock<std::mutex> l(b.mu);
                 b.cv.wait(l, [&]() { return b.stop || b.arrived > k; });
                 if (b.stop) return;
+                threads = b.threads;
             }
-            part(k, t, nt);
+            part(k, t, threads);
             {
                 std::lock_guard<std::mutex> l(b.mu);
-                b.done[k]++;
+                b.done++;
             }
             b.cv.notify_all();
         }
     };
     try {
-        for (int t = 0; t < want; t++) {
-            pool.emplace_back(work, t);
-            nt++;
-        }
-    } catch (const std::system_error &) {
-        // a thread limit: those that started do it, or this one alone
+        for (; nt < want; nt++) pool[nt] = std::thread(work, nt);
+    } catch (const std::exception &) {
+        // a thread limit, or no memory for one: those that started do it, or this one alone
     }
-    start.unlock();
+    {
+        std::lock_guard<std::mutex> l(b.mu);
+        b.threads = nt;
+    }
     cudaError_t e = cudaSuccess;
     for (size_t k = 0; k < std::min<size_t>(kSlots, npieces) && e == cudaSuccess; k++) e = issue(k);
     for (size_t k = 0; k < npieces && e == cudaSuccess; k++) {
@@ -123,9 +122,10 @@ extern "C" bpf_status bpf_block_to_host(bpf_ctx *ctx, int n, int p, const double
             part(k, 0, 1);
         } else {
             std::unique_lock<std::mutex> l(b.mu);
+            b.done = 0;
             b.arrived = k + 1;
             b.cv.notify_all();
-            b.cv.wait(l, [&]() { return b.done[k] == nt; });
+            b.cv.wait(l, [&]() { return b.done == nt; });
         }
         if (k + kSlots < npieces) e = issue(k + kSlots);
     }
@@ -134,7 +134,7 @@ extern "C" bpf_status bpf_block_to_host(bpf_ctx *ctx, int n, int p, const double
         b.stop = true;
     }
     b.cv.notify_all();
-    for (auto &t : pool) t.join();
+    for (int t = 0; t < nt; t++) pool[t].join();
     if (e != cudaSuccess) return cuda_error(ctx, e, "block_to_host", __FILE__, __LINE__);
     return BPF_SUCCESS;
 }
