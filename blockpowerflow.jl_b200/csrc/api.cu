@@ -765,7 +765,7 @@ bpf_status bpf_prec_destroy(bpf_prec *P) {
     cudaFree(P->forder);
     cudaFree(P->tail_S);
     cudaFree(P->tail_F);
-    cudaFree(P->tail_inv);
+    cudaFree(P->tail_D);
     cudaFree(P->cl_lev_ptr);
     cudaFree(P->cl_ent);
     cudaFree(P->cl_row);

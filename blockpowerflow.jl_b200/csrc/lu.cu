@@ -14,8 +14,8 @@
 //    to dense storage, take a CTA each (lu_cta_rows_kernel).  No atomics: the factors are deterministic.
 //  * Tail: blocked right-looking LU without pivoting (the pivot order is the analysis's) in one
 //    cooperative launch, 64 x 64 tiles on the FP64 tensor pipe.  A step costs one grid barrier: a tile
-//    multiplies by the inverted diagonal factors of its own row and column panels itself, and
-//    CTA 0 factors the next diagonal tile as soon as it is updated.
+//    substitutes its own row and column panels with the diagonal factors itself, and CTA 0 factors the
+//    next diagonal tile as soon as it is updated.
 //  * Solves: up to 24,800 rows one right-hand side per CTA in shared memory (trsv_col.cu, the dense
 //    tail between the sweeps); larger systems by a data flow over rows, a warp per row with the
 //    right-hand sides over the lanes, the tail on the FP64 tensor pipe eight columns a CTA.
@@ -41,6 +41,7 @@ namespace bpf {
 
 constexpr int kNB = 64;          // tail tile
 constexpr int kCtaRow = 96;      // entries of a row from the diagonal on past which a CTA takes it
+constexpr int kTailSolveThreads = 640;   // 1,024 leave the substitution 64 registers (25,000 buses, 256 columns 1,054 / 1,029 us)
 constexpr int kTS = kNB + 4;     // tile row stride in shared memory (conflict-free DMMA fragments)
 
 __device__ __forceinline__ void lu_dmma(double &d0, double &d1, double a, double b) {
@@ -215,22 +216,18 @@ __device__ __forceinline__ void tile_zero(double (&acc)[2][4][2]) {
         for (int ni = 0; ni < 4; ni++) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
 }
 
-// LU of the shared tile T (no pivoting) with L^{-1} and U^{-1} from the same 64 steps: step k
-// eliminates column k below the diagonal by row operations (applied to the identity: L^{-1}) and row
-// k right of it by column operations (applied to the identity: U^{-1}, its columns scaled at the
-// end).  Thread (ti, tj) of 16 x 16 holds rows ti + 16 r, columns tj + 16 c; a pivot row and
-// column go through shared memory, one barrier a step.
-__device__ __forceinline__ void tile_lu(double *T, double *bufs, double *Linv, double *Uinv, int row0, DevStatus *ds) {
-    double *rowA = bufs, *colA = bufs + 128, *rowB = bufs + 256, *colC = bufs + 384, *dinv = bufs + 512;
+// LU of the shared tile T (no pivoting): the packed factors row by row into F (row stride ld) and column by column
+// into D, the pivots' reciprocals into R.  Thread (ti, tj) of 16 x 16 holds rows ti + 16 r, columns tj + 16 c; a
+// pivot row and column go through shared memory, one barrier a step.
+__device__ __forceinline__ void tile_lu(double *T, double *bufs, double *F, size_t ld, double *D, double *R, int row0,
+                                        DevStatus *ds) {
+    double *rowA = bufs, *colA = bufs + 128;
     const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
-    double a[4][4], b[4][4], cc[4][4];
+    double a[4][4];
 #pragma unroll
     for (int r = 0; r < 4; r++)
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            a[r][c] = T[(ti + 16 * r) * kTS + tj + 16 * c];
-            b[r][c] = cc[r][c] = (ti + 16 * r == tj + 16 * c) ? 1.0 : 0.0;
-        }
+        for (int c = 0; c < 4; c++) a[r][c] = T[(ti + 16 * r) * kTS + tj + 16 * c];
 #pragma unroll
     for (int kk = 0; kk < 4; kk++)
 #pragma unroll 1
@@ -238,25 +235,17 @@ __device__ __forceinline__ void tile_lu(double *T, double *bufs, double *Linv, d
             const int k = 16 * kk + kl, o = 64 * (k & 1);
             if (ti == kl)
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    rowA[o + tj + 16 * c] = a[kk][c];
-                    rowB[o + tj + 16 * c] = b[kk][c];
-                }
+                for (int c = 0; c < 4; c++) rowA[o + tj + 16 * c] = a[kk][c];
             if (tj == kl)
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    colA[o + ti + 16 * r] = a[r][kk];
-                    colC[o + ti + 16 * r] = cc[r][kk];
-                }
+                for (int r = 0; r < 4; r++) colA[o + ti + 16 * r] = a[r][kk];
             __syncthreads();
             const double piv = rowA[o + k], inv = 1.0 / piv;
             if (threadIdx.x == 0) {
-                dinv[k] = inv;
+                R[k] = inv;
                 if (piv == 0.0 && atomicCAS(&ds->err, 0, (int)DEV_ZERO_PIVOT) == 0) ds->aux = row0 + k;
             }
-            // blocks of 16 that step k can change: rows and columns from kk on of the tile, rows from kk
-            // and columns up to kk of L^{-1}, rows up to kk and columns from kk of U^{-1}
-            double l[4], u[4], ui[4];
+            double l[4], u[4];
 #pragma unroll
             for (int r = kk; r < 4; r++) {
                 const int i = ti + 16 * r;
@@ -266,174 +255,230 @@ __device__ __forceinline__ void tile_lu(double *T, double *bufs, double *Linv, d
             for (int c = kk; c < 4; c++) {
                 const int j = tj + 16 * c;
                 u[c] = j > k ? rowA[o + j] : 0.0;
-                ui[c] = u[c] * inv;
             }
 #pragma unroll
             for (int r = kk; r < 4; r++)
 #pragma unroll
                 for (int c = kk; c < 4; c++) a[r][c] -= l[r] * u[c];
-#pragma unroll
-            for (int c = 0; c <= kk; c++) {
-                const double rb = rowB[o + tj + 16 * c];
-#pragma unroll
-                for (int r = kk; r < 4; r++) b[r][c] -= l[r] * rb;
-            }
-#pragma unroll
-            for (int r = 0; r <= kk; r++) {
-                const double cb = colC[o + ti + 16 * r];
-#pragma unroll
-                for (int c = kk; c < 4; c++) cc[r][c] -= cb * ui[c];
-            }
             if (tj == kl)
 #pragma unroll
                 for (int r = 0; r < 4; r++)
                     if (ti + 16 * r > k) a[r][kk] = l[r];
         }
-    __syncthreads();
 #pragma unroll
     for (int r = 0; r < 4; r++)
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const int i = ti + 16 * r, j = tj + 16 * c;
-            Linv[i * kNB + j] = b[r][c];
-            Uinv[i * kNB + j] = cc[r][c] * dinv[j];
+            F[i * ld + j] = a[r][c];
+            D[j * kNB + i] = a[r][c];
         }
 }
 
-// S (mp x mp, nb tiles a side; destroyed) -> F: the off-diagonal tiles of L and U; Linv, Uinv: the
-// inverted diagonal factors.  row0: the first row of the tail (diagnostics).
+// Substitution with a 64 x 64 triangle, 8 Q right-hand sides a warp: x[q][b][i] is unknown 8 b + 2 t4 + i of right-hand
+// side 8 q + g (a DMMA's accumulators); m(k, j): what unknown k takes from j, j > k (DESC: j < k); SCALE: unknowns
+// times rinv[k].  Eight unknowns at a time by broadcasts within four lanes, the others by the tensor pipe, whose
+// operand is the solved block as it lies.  (Products with an inverted triangle are as many, but lose its condition
+// where it grows: 1e-7 for a triangle of ones on the diagonal and -0.54 above, 1e-17 so.)
+template <bool DESC, bool SCALE, int Q, class M>
+__device__ __forceinline__ void tri_substitute(double (&x)[Q][8][2], M m, const double *rinv) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int bi = 0; bi < 8; bi++) {
+        const int b = DESC ? 7 - bi : bi;
+#pragma unroll
+        for (int ci = 0; ci < 8; ci++) {
+            const int c = DESC ? 7 - ci : ci, k = 8 * b + c;
+            const double a0 = m(k, 8 * b + 2 * t4), a1 = m(k, 8 * b + 2 * t4 + 1);
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                double v = x[q][b][c & 1];
+                if (SCALE) v *= rinv[k];
+                const double xk = __shfl_sync(0xffffffffu, v, (lane & 28) | (c >> 1));
+                if (SCALE && t4 == c >> 1) x[q][b][c & 1] = xk;
+                if (DESC ? 2 * t4 < c : 2 * t4 > c) x[q][b][0] -= xk * a0;
+                if (DESC ? 2 * t4 + 1 < c : 2 * t4 + 1 > c) x[q][b][1] -= xk * a1;
+            }
+        }
+#pragma unroll
+        for (int ni = DESC ? 0 : b + 1; ni < (DESC ? b : 8); ni++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const double v = m(8 * b + 2 * t4 + i, 8 * ni + g);
+#pragma unroll
+                for (int q = 0; q < Q; q++) lu_dmma(x[q][ni][0], x[q][ni][1], -x[q][b][i], v);
+            }
+    }
+}
+
+// S (mp x mp, nb tiles a side; destroyed) -> F: the tiles of L and U; D: the diagonal ones column by column; R: the
+// pivots' reciprocals.  row0: the first row of the tail (diagnostics).
 __global__ void __launch_bounds__(256, 1)
-lu_tail_factor_kernel(int nb, double *S, double *F, double *Linv, double *Uinv, int row0, DevStatus *ds) {
+lu_tail_factor_kernel(int nb, double *S, double *F, double *D, double *R, int row0, DevStatus *ds) {
     extern __shared__ __align__(16) double tiles[];
     __shared__ unsigned s_gen;
     if (threadIdx.x == 0) s_gen = barrier_gen_start(ds);
     __syncthreads();
     unsigned gen = s_gen;
-    double *T0 = tiles, *T1 = T0 + kNB * kTS, *T2 = T1 + kNB * kTS, *T3 = T2 + kNB * kTS, *bufs = T3 + kNB * kTS;
+    double *T0 = tiles, *T1 = T0 + kNB * kTS, *T2 = T1 + kNB * kTS, *T3 = T2 + kNB * kTS, *bufs = T3 + kNB * kTS,
+           *rinv = bufs + 256;
     const size_t ld = (size_t)nb * kNB;
     auto at = [&](int i, int j) { return (size_t)i * kNB * ld + (size_t)j * kNB; };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
     if (blockIdx.x == 0) {
         tile_in(T0, S, ld);
         __syncthreads();
-        tile_lu(T0, bufs, Linv, Uinv, row0, ds);
+        tile_lu(T0, bufs, F, ld, D, R, row0, ds);
     }
     if (nb > 1 && !grid_barrier(ds, gen)) return;
     for (int k = 0; k + 1 < nb; k++) {
         const int side = nb - 1 - k, ntile = side * side;
+        // the diagonal tile, U's rows in T1 and L's columns in T2
+        tile_in(T1, F + at(k, k), ld);
+        tile_in(T2, D + (size_t)k * kNB * kNB, kNB);
+        if (threadIdx.x < kNB) rinv[threadIdx.x] = __ldcg(R + k * kNB + threadIdx.x);
         // tile 0, the next diagonal one, is CTA 0's alone; the others go round the other CTAs
         for (int t = blockIdx.x; t < ntile; t += (gridDim.x > 1 && t == 0) ? ntile : max(1, (int)gridDim.x - 1)) {
             const int i = k + 1 + t / side, j = k + 1 + t % side;
             __syncthreads();
             tile_in(T0, S + at(i, k), ld);
-            tile_in(T1, Uinv + (size_t)k * kNB * kNB, kNB);
-            tile_in(T2, Linv + (size_t)k * kNB * kNB, kNB);
             tile_in(T3, S + at(k, j), ld);
             __syncthreads();
-            double l[2][4][2], u[2][4][2], s[2][4][2];
-            tile_zero(l);
-            tile_zero(u);
+            // T0 <- T0 U^{-1}, a row per right-hand side, on warps 0 - 3; T3 <- L^{-1} T3, a column each, on 4 - 7
+            double x[2][8][2];
+            const int v0 = 16 * (warp & 3) + g;
+            if (warp < 4) {
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+#pragma unroll
+                    for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) x[q][ni][e] = T0[(v0 + 8 * q) * kTS + 8 * ni + 2 * t4 + e];
+                tri_substitute<false, true, 2>(x, [&](int kc, int jc) { return T1[kc * kTS + jc]; }, rinv);
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+#pragma unroll
+                    for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int r = v0 + 8 * q, c = 8 * ni + 2 * t4 + e;
+                            T0[r * kTS + c] = x[q][ni][e];
+                            if (j == k + 1) F[at(i, k) + r * ld + c] = x[q][ni][e];
+                        }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+#pragma unroll
+                    for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) x[q][ni][e] = T3[(8 * ni + 2 * t4 + e) * kTS + v0 + 8 * q];
+                tri_substitute<false, false, 2>(x, [&](int kc, int jc) { return T2[kc * kTS + jc]; }, rinv);
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+#pragma unroll
+                    for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int r = 8 * ni + 2 * t4 + e, c = v0 + 8 * q;
+                            T3[r * kTS + c] = x[q][ni][e];
+                            if (i == k + 1) F[at(k, j) + r * ld + c] = x[q][ni][e];
+                        }
+            }
+            __syncthreads();
+            double s[2][4][2];
             tile_zero(s);
-            tile_mul(l, T0, T1);
-            tile_mul(u, T2, T3);
-            __syncthreads();
-            tile_each(l, [&](int r, int c, double v) {
-                T0[r * kTS + c] = v;
-                if (j == k + 1) F[at(i, k) + r * ld + c] = v;
-            });
-            tile_each(u, [&](int r, int c, double v) {
-                T1[r * kTS + c] = v;
-                if (i == k + 1) F[at(k, j) + r * ld + c] = v;
-            });
-            __syncthreads();
-            tile_mul(s, T0, T1);
-            double *g = S + at(i, j);
+            tile_mul(s, T0, T3);
+            double *gs = S + at(i, j);
             if (t == 0) __syncthreads();
             tile_each(s, [&](int r, int c, double v) {
-                const double x = __ldcg(g + r * ld + c) - v;
-                if (t == 0) T0[r * kTS + c] = x;
-                else g[r * ld + c] = x;
+                const double y = __ldcg(gs + r * ld + c) - v;
+                if (t == 0) T0[r * kTS + c] = y;
+                else gs[r * ld + c] = y;
             });
             if (t == 0) {
                 __syncthreads();
-                tile_lu(T0, bufs, Linv + (size_t)(k + 1) * kNB * kNB, Uinv + (size_t)(k + 1) * kNB * kNB,
+                tile_lu(T0, bufs, F + at(k + 1, k + 1), ld, D + (size_t)(k + 1) * kNB * kNB, R + (k + 1) * kNB,
                         row0 + (k + 1) * kNB, ds);
             }
         }
         if (!grid_barrier(ds, gen)) return;
     }
 }
-constexpr size_t kTailFactorSmem = sizeof(double) * (4 * kNB * kTS + 640);
+constexpr size_t kTailFactorSmem = sizeof(double) * (4 * kNB * kTS + 256 + kNB);
 
 // ------------------------------------------------------------------------------------
 // dense tail: solves of row-major blocks
 // ------------------------------------------------------------------------------------
 // Rows s.. of the n x p block Z hold the tail's right-hand sides; rows s.. of W receive U^{-1} L^{-1}
-// of them.  A CTA takes eight columns, kept in shared memory; a block step multiplies by the
-// inverted diagonal factor, then updates the other rows, eight rows a warp on the tensor pipe.
-__global__ void __launch_bounds__(1024)
-lu_tail_solve_kernel(int s, int m, int nb, const double *__restrict__ F, const double *__restrict__ Linv,
-                     const double *__restrict__ Uinv, int p, const double *__restrict__ Z, double *W) {
-    extern __shared__ __align__(16) double ysm[];   // [mp][8]
-    __shared__ double z[kNB * 8];
+// of them.  A CTA takes eight columns, kept in shared memory; a block step solves with the diagonal tile (warp 0, the
+// tile in shared memory), then updates the other rows, eight rows a warp on the tensor pipe.
+__global__ void __launch_bounds__(kTailSolveThreads)
+lu_tail_solve_kernel(int s, int m, int nb, const double *__restrict__ F, const double *__restrict__ D,
+                     const double *__restrict__ R, int p, const double *__restrict__ Z, double *W) {
+    extern __shared__ __align__(16) double ysm[];   // [mp][8], then the diagonal tile by columns [64][kTS]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, g = lane >> 2, t4 = lane & 3;
     const int c0 = 8 * blockIdx.x, mp = nb * kNB;
     const size_t ld = mp;
+    double *tile = ysm + 8 * (size_t)mp;
     for (int e = threadIdx.x; e < 8 * mp; e += blockDim.x) {
         const int r = e >> 3, c = c0 + (e & 7);
         ysm[e] = r < m && c < p ? __ldcg(Z + (size_t)(s + r) * p + c) : 0.0;
     }
-    __syncthreads();
-    // eight rows of A (row stride lda), and their sums over 64 columns times x ([64][8])
-    auto fetch = [&](const double *A, size_t lda, double (&a)[16]) {
+    auto fetch = [&](const double *A, size_t lda, double (&a)[16]) {   // eight rows of A, 64 columns
 #pragma unroll
         for (int ks = 0; ks < 16; ks++) a[ks] = __ldg(A + g * lda + 4 * ks + t4);
     };
-    auto times = [&](const double (&a)[16], const double *x, double &d0, double &d1) {
-        double e0 = 0.0, e1 = 0.0;
-        d0 = d1 = 0.0;
-#pragma unroll
-        for (int ks = 0; ks < 16; ks += 2) {
-            lu_dmma(d0, d1, a[ks], x[(4 * ks + t4) * 8 + g]);
-            lu_dmma(e0, e1, a[ks + 1], x[(4 * ks + 4 + t4) * 8 + g]);
-        }
-        d0 += e0;
-        d1 += e1;
-    };
-    for (int sweep = 0; sweep < 2; sweep++) {
-        const double *D = sweep == 0 ? Linv : Uinv;
+    for (int sweep = 0; sweep < 2; sweep++)
         for (int bi = 0; bi < nb; bi++) {
             const int b = sweep == 0 ? bi : nb - 1 - bi;
             const int r0 = sweep == 0 ? 8 * (b + 1) : 0, r1 = sweep == 0 ? 8 * nb : 8 * b;
             double *yb = ysm + (size_t)b * kNB * 8;
-            double a[16], d0, d1;
-            // warps 0-7 multiply by the diagonal factor; every warp's first tile is under way meanwhile
-            if (warp < 8) {
-                double dg[16];
-                fetch(D + (size_t)b * kNB * kNB + (size_t)8 * warp * kNB, kNB, dg);
-                if (r0 + warp < r1) fetch(F + (size_t)8 * (r0 + warp) * ld + (size_t)b * kNB, ld, a);
-                times(dg, yb, d0, d1);
-                z[(8 * warp + g) * 8 + 2 * t4] = d0;
-                z[(8 * warp + g) * 8 + 2 * t4 + 1] = d1;
-            } else if (r0 + warp < r1) {
+            // U's rows and right-hand sides times the pivots' reciprocals: no product in the substitution's chain
+            for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x)
+                tile[(e >> 6) * kTS + (e & 63)] =
+                    __ldg(D + (size_t)b * kNB * kNB + e) * (sweep == 0 ? 1.0 : __ldg(R + b * kNB + (e & 63)));
+            __syncthreads();
+            double a[16];
+            if (warp == 0) {
+                double x[1][8][2];
+#pragma unroll
+                for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const int r = 8 * ni + 2 * t4 + e;
+                        x[0][ni][e] = yb[r * 8 + g] * (sweep == 0 ? 1.0 : __ldg(R + b * kNB + r));
+                    }
+                auto by_column = [&](int k, int j) { return tile[k * kTS + j]; };
+                if (sweep == 0) tri_substitute<false, false, 1>(x, by_column, nullptr);
+                else tri_substitute<true, false, 1>(x, by_column, nullptr);
+#pragma unroll
+                for (int ni = 0; ni < 8; ni++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) yb[(8 * ni + 2 * t4 + e) * 8 + g] = x[0][ni][e];
+            } else if (r0 + warp < r1) {   // the other warps' first tiles are under way meanwhile
                 fetch(F + (size_t)8 * (r0 + warp) * ld + (size_t)b * kNB, ld, a);
             }
             __syncthreads();
-            for (int e = threadIdx.x; e < kNB * 8; e += blockDim.x) yb[e] = z[e];
             for (int t = r0 + warp; t < r1; t += nw) {
-                if (t >= r0 + nw) fetch(F + (size_t)8 * t * ld + (size_t)b * kNB, ld, a);
-                times(a, z, d0, d1);
+                if (warp == 0 || t >= r0 + nw) fetch(F + (size_t)8 * t * ld + (size_t)b * kNB, ld, a);
+                double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
+#pragma unroll
+                for (int ks = 0; ks < 16; ks += 2) {
+                    lu_dmma(d0, d1, a[ks], yb[(4 * ks + t4) * 8 + g]);
+                    lu_dmma(e0, e1, a[ks + 1], yb[(4 * ks + 4 + t4) * 8 + g]);
+                }
                 double *y = ysm + (size_t)(8 * t + g) * 8 + 2 * t4;
-                y[0] -= d0;
-                y[1] -= d1;
+                y[0] -= d0 + e0;
+                y[1] -= d1 + e1;
             }
             __syncthreads();
         }
-    }
     for (int e = threadIdx.x; e < 8 * m; e += blockDim.x) {
         const int r = e >> 3, c = c0 + (e & 7);
         if (c < p) W[(size_t)(s + r) * p + c] = ysm[e];
     }
 }
+static size_t tail_solve_smem(int mp) { return sizeof(double) * (8 * (size_t)mp + kNB * kTS); }
 
 // ------------------------------------------------------------------------------------
 // front sweeps of row-major blocks as a data flow
@@ -633,10 +678,10 @@ bpf_status lu_factor(bpf_ctx *ctx, bpf_prec *P, const double *vals) {
                                        (int)kTailFactorSmem));
     // at most a tile each in the first step; one CTA fills an SM's shared memory
     const int grid = std::min(ctx->num_sms, std::max(1, (nb - 1) * (nb - 1)));
-    double *S = P->tail_S, *F = P->tail_F, *Li = P->tail_inv, *Ui = Li + (size_t)nb * kNB * kNB;
+    double *S = P->tail_S, *F = P->tail_F, *D = P->tail_D, *R = D + (size_t)nb * kNB * kNB;
     int row0 = P->tail_s, nbv = nb;
     DevStatus *ds = ctx->dstat;
-    void *args[] = {&nbv, &S, &F, &Li, &Ui, &row0, &ds};
+    void *args[] = {&nbv, &S, &F, &D, &R, &row0, &ds};
     const double m = P->tail_mp;
     KScope ks(ctx, BPF_KC_FACTOR, 16.0 * m * m, 2.0 / 3.0 * m * m * m);
     BPF_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)lu_tail_factor_kernel, dim3(grid), dim3(256), args,
@@ -674,7 +719,7 @@ bpf_status lu_solve(bpf_ctx *ctx, const bpf_prec *P, int nrhs, double *X, int ld
     bpf_status st;
     double *buf = (double *)ws_get(ctx, WS_A, sizeof(double) * 3 * (size_t)n * std::min(nrhs, chunk), &st);
     if (!buf) return st;
-    const size_t tail_smem = sizeof(double) * 8 * (size_t)P->tail_mp;
+    const size_t tail_smem = tail_solve_smem(P->tail_mp);
     BPF_CUDA(ctx, cudaFuncSetAttribute(lu_tail_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_smem));
     for (int c0 = 0; c0 < nrhs; c0 += chunk) {
         const int p = std::min(chunk, nrhs - c0);
@@ -686,8 +731,8 @@ bpf_status lu_solve(bpf_ctx *ctx, const bpf_prec *P, int nrhs, double *X, int ld
         if (nb > 0) {
             KScope ks(ctx, BPF_KC_TRSV, 8.0 * P->tail_mp * P->tail_mp + 16.0 * P->tail_m * (double)p,
                       2.0 * P->tail_mp * (double)P->tail_mp * p);
-            lu_tail_solve_kernel<<<ceil_div(p, 8), 1024, tail_smem, ctx->stream>>>(
-                s, P->tail_m, nb, P->tail_F, P->tail_inv, P->tail_inv + (size_t)nb * kNB * kNB, p, Z, W);
+            lu_tail_solve_kernel<<<ceil_div(p, 8), kTailSolveThreads, tail_smem, ctx->stream>>>(
+                s, P->tail_m, nb, P->tail_F, P->tail_D, P->tail_D + (size_t)nb * kNB * kNB, p, Z, W);
             BPF_LAUNCHED(ctx);
         }
         BPF_TRY(lu_sweep(ctx, P->upper, p, Z, nullptr, W));
@@ -775,7 +820,7 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
             best = m;
         }
     }
-    const int mp = best, s = std::max(0, n - mp), m = n - s, nb = mp / kNB;
+    const int mp = best, s = std::max(0, n - mp), m = n - s;
     std::vector<int> fend(n, 0);   // end of a row's entries before column s
     for (int i = 0; i < n; i++)
         fend[i] = (int)(std::lower_bound(ci.begin() + rp[i], ci.begin() + rp[i + 1], s) - ci.begin());
@@ -940,7 +985,7 @@ bpf_status lu_setup(bpf_ctx *ctx, int n, const std::vector<int> &rp, const std::
         if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_S, tail_bytes);
         if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_F, tail_bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(P->tail_F, 0, tail_bytes, ctx->stream);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_inv, sizeof(double) * 2 * (size_t)nb * kNB * kNB);
+        if (e == cudaSuccess) e = cudaMalloc((void **)&P->tail_D, sizeof(double) * (size_t)mp * (kNB + 1));
     }
     if (e == cudaSuccess && P->nnz > 0) e = cudaMalloc((void **)&P->fv, sizeof(double) * P->nnz);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);   // host vectors die on return

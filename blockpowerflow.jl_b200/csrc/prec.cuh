@@ -164,7 +164,7 @@ struct bpf_prec {
     bpf::TriDev upper;   // backward solve (U for ILU0; L' for IC0)
     // LU on a fill pattern (the RF refactorization, lu.cu): rows and columns from tail_s on, tail_m of
     // them padded to tail_mp, are a dense block: tail_S receives the Schur complement, tail_F holds
-    // the off-diagonal 64 x 64 tiles of its factors, tail_inv the inverted diagonal ones (L, then U).
+    // the 64 x 64 tiles of its factors, tail_D the diagonal ones by columns and then the pivots' reciprocals.
     // fend[i]: end of row i's entries before column tail_s.
     // forder: the rows in the order of the factorization, nshort rows a warp takes, then nlong front
     // rows a CTA takes (long rows, and what depends on them), then the tail;
@@ -174,7 +174,7 @@ struct bpf_prec {
     // (ILU(0) kept for column solves: the stream's order, long rows of a level first.)
     int *forder = nullptr;
     int *fend = nullptr;
-    double *tail_S = nullptr, *tail_F = nullptr, *tail_inv = nullptr;
+    double *tail_S = nullptr, *tail_F = nullptr, *tail_D = nullptr;
     // LU whose front still has more than 2^31 - 1 update pairs (or BPF_LU_PAIRLESS=1): right-looking
     // column steps that find an entry's updates by a search in its row.  Step k (scale column k of L by
     // 1 / u_kk, then apply its updates) waits for the steps that update row k or column k;

@@ -223,7 +223,7 @@ static std::vector<SolveArray> solve_arrays(bpf_prec *P) {
         }
     if (P->tail_mp > 0) {
         v.push_back({(void **)&P->tail_F, sizeof(double) * (size_t)P->tail_mp * P->tail_mp});
-        v.push_back({(void **)&P->tail_inv, sizeof(double) * 2 * (size_t)P->tail_mp * 64});
+        v.push_back({(void **)&P->tail_D, sizeof(double) * (size_t)P->tail_mp * 65});
     }
     return v;
 }

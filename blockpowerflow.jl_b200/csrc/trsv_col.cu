@@ -128,7 +128,7 @@ struct ColArgs {
     const int *pos0, *pos01, *pos1;
     // the LU's dense tail: unknowns s.. of both sweeps, nb tiles of 64 (0: none)
     int s, nb;
-    const double *F, *Linv, *Uinv;
+    const double *F, *D, *R;   // its tiles, the diagonal ones by columns, the pivots' reciprocals
 };
 
 // Counters of the ring, relaxed: `ready` only tells that a slot's mbarrier phase is over (its own wait
@@ -267,49 +267,90 @@ __device__ __forceinline__ bool col_sweep(const int4 *head, int nslab, int nstag
     return ok;
 }
 
-// y[0..64) of a dense tail in shared memory, at address y: U^{-1} L^{-1} y by 64-wide block steps.  A
-// warp takes four rows at a time, two columns a lane; z: 64 values of scratch.
-__device__ __forceinline__ void col_tail(const ColArgs &a, unsigned y, double *z, int nw) {
+// A warp's four columns of diagonal tile b of the dense tail, rows lane and lane + 32; of U each row times its
+// pivot's reciprocal (r), which takes the product out of the substitution's chain.
+template <bool UP>
+__device__ __forceinline__ void col_tail_load(const ColArgs &a, int b, double (&d)[4][2], double (&r)[2]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (b < 0 || b >= a.nb || warp >= 16) return;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const double *col = a.D + (size_t)b * 4096 + 64 * (UP ? 63 - 4 * warp - c : 4 * warp + c) + lane;
+        d[c][0] = __ldg(col);
+        d[c][1] = __ldg(col + 32);
+    }
+    if (UP) {
+        r[0] = __ldg(a.R + 64 * b + lane);
+        r[1] = __ldg(a.R + 64 * b + 32 + lane);
+    }
+}
+
+// One sweep over a dense tail in shared memory, at address y, by 64-wide block steps.  The diagonal tile's
+// substitution passes through warps 0 - 15, four unknowns each, whose columns of the tile were fetched during the
+// step before; then a warp updates four rows at a time, two columns a lane.
+template <bool UP>
+__device__ __forceinline__ void col_tail(const ColArgs &a, unsigned y, int nw) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t ld = (size_t)a.nb * 64;
-    // sums over 64 columns of rows r (< r1) of A (row stride lda) times x (shared): f(r, sum)
-    auto rows = [&](const double *A, size_t lda, int r0, int r1, unsigned x, auto f) {
+    double d[4][2], r[2];
+    col_tail_load<UP>(a, UP ? a.nb - 1 : 0, d, r);
+#pragma unroll 1
+    for (int bi = 0; bi < a.nb; bi++) {
+        const int b = UP ? a.nb - 1 - bi : bi;
+        const unsigned yb = y + 512 * b;
+        const int k0 = UP ? 63 - 4 * warp : 4 * warp;   // the first of the warp's unknowns, downwards in U
+        const bool high = (k0 & 32) != 0;
+        if (UP) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                d[c][0] *= r[0];
+                d[c][1] *= r[1];
+            }
+        }
+#pragma unroll 1
+        for (int w = 0; w < 16; w++) {
+            if (warp == w) {
+                double v0, v1;
+                col_get(yb, lane, v0);
+                col_get(yb, lane + 32, v1);
+                if (UP && w == 0) {
+                    v0 *= r[0];
+                    v1 *= r[1];
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int k = UP ? k0 - c : k0 + c;
+                    const double xk = __shfl_sync(0xffffffffu, high ? v1 : v0, k & 31);
+                    if (UP ? lane < k : lane > k) v0 -= d[c][0] * xk;
+                    if (UP ? lane + 32 < k : lane + 32 > k) v1 -= d[c][1] * xk;
+                }
+                col_put(yb, lane, v0);
+                col_put(yb, lane + 32, v1);
+            }
+            col_barrier(32 * nw);
+        }
+        col_tail_load<UP>(a, UP ? b - 1 : b + 1, d, r);
         double x0, x1;
-        col_get(x, 2 * lane, x0);
-        col_get(x, 2 * lane + 1, x1);
-        for (int r = r0 + 4 * warp; r < r1; r += 4 * nw) {
+        col_get(yb, 2 * lane, x0);
+        col_get(yb, 2 * lane + 1, x1);
+        const double *A = a.F + (size_t)b * 64;
+        const int r1 = UP ? 64 * b : 64 * a.nb;
+        for (int q = (UP ? 0 : 64 * (b + 1)) + 4 * warp; q < r1; q += 4 * nw) {
             double2 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = __ldg(reinterpret_cast<const double2 *>(A + (size_t)(r + u) * lda) + lane);
+            for (int u = 0; u < 4; u++) v[u] = __ldg(reinterpret_cast<const double2 *>(A + (size_t)(q + u) * ld) + lane);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const double s = warp_sum(v[u].x * x0 + v[u].y * x1);
-                if (lane == 0) f(r + u, s);
+                if (lane == 0) {
+                    double o;
+                    col_get(y, q + u, o);
+                    col_put(y, q + u, o - s);
+                }
             }
         }
-    };
-    const unsigned zs = smem_u32(z);
-#pragma unroll 1
-    for (int sweep = 0; sweep < 2; sweep++)
-#pragma unroll 1
-        for (int bi = 0; bi < a.nb; bi++) {
-            const int b = sweep == 0 ? bi : a.nb - 1 - bi;
-            rows((sweep == 0 ? a.Linv : a.Uinv) + (size_t)b * 4096, 64, 0, 64, y + 512 * b,
-                 [&](int r, double v) { col_put(zs, r, v); });
-            col_barrier(32 * nw);
-            if (threadIdx.x < 64) {
-                double v;
-                col_get(zs, threadIdx.x, v);
-                col_put(y, 64 * b + threadIdx.x, v);
-            }
-            rows(a.F + (size_t)b * 64, ld, sweep == 0 ? 64 * (b + 1) : 0, sweep == 0 ? 64 * a.nb : 64 * b, zs,
-                 [&](int r, double v) {
-                     double o;
-                     col_get(y, r, o);
-                     col_put(y, r, o - v);
-                 });
-            col_barrier(32 * nw);
-        }
+        col_barrier(32 * nw);
+    }
 }
 
 template <typename TF>
@@ -358,8 +399,8 @@ trsv_col_kernel(ColArgs a, const double *X, size_t ldx, double *Y, size_t ldy, s
     bool ok = col_sweep<TF>(a.head[0], a.nslab[0], a.nstage[0], a.diag[0] != 0, y, rbase, r, nw, lim, true);
     if constexpr (std::is_same<TF, double>::value)
         if (a.nb > 0) {
-            __shared__ double z[64];
-            col_tail(a, y + 8 * a.s, z, nw);
+            col_tail<false>(a, y + 8 * a.s, nw);
+            col_tail<true>(a, y + 8 * a.s, nw);
         }
     for (int i0 = tid; i0 < n; i0 += 8 * nt) {   // forward results in backward positions, through Y
         int at[8];
@@ -417,8 +458,8 @@ bpf_status trsv_col(bpf_ctx *ctx, const bpf_prec *P, int p, const double *X, siz
     a.s = P->tail_s;
     a.nb = P->tail_mp / 64;
     a.F = P->tail_F;
-    a.Linv = P->tail_inv;
-    a.Uinv = P->tail_inv + (size_t)P->tail_mp * 64;
+    a.D = P->tail_D;
+    a.R = P->tail_D + (size_t)P->tail_mp * 64;
     const size_t smem = (size_t)a.nring * kChunk + (std::max(P->n, a.s + P->tail_mp) + 1) * es;
     double fb = 0.0;
     for (int w = 0; w < 2; w++) {

@@ -156,3 +156,50 @@ def test_a_refactorization_with_a_nan_leaves_the_next_one_alone(bpf, n, bad, at)
     X = _block(B)
     bpf.CUSOLVERRF.ldiv_(rf, X)
     np.testing.assert_array_equal(X.cpu().numpy(), before.cpu().numpy())
+
+
+def _growing(kind, n):
+    """(L, U) of triangles whose inverses grow like 1.4^n within a tile: ones on the diagonal, -0.4 beside it."""
+    K = np.eye(n)
+    for b in range(0, n, 64):
+        e = min(n, b + 64)
+        K[b:e, b:e] -= 0.4 * np.triu(np.ones((e - b, e - b)), 1)
+    if kind == "upper":
+        return np.eye(n), K
+    if kind == "lower":
+        return K.T.copy(), np.eye(n)
+    C = np.random.default_rng(n).standard_normal((n, n)) / n   # tiles below the diagonal ones
+    for b in range(0, n, 64):
+        C[b:b + 64, b:] = 0.0
+    if kind == "rows":        # U grows: the panels of L
+        return np.eye(n) + C, K
+    return K.T.copy(), np.eye(n) + C.T   # L grows: the panels of U
+
+
+# Substitution computes factors and solutions with |A - L U| <= n eps |L| |U| and |B - L U X| <= 2 n eps |L| |U| |X|,
+# whatever the condition; the factors of A differ from L and U by at most 64 eps 1.4^64 < 1e-4; another n eps for
+# the residual and n eps for A's rounding.  Products with inverted triangles miss it by 1.4^64.
+@pytest.mark.parametrize("kind", ["upper", "lower", "rows", "columns"])
+@pytest.mark.parametrize("n,before", [(64, 0), (65, 0), (130, 0), (200, 0), (200, 25_000)])
+def test_tails_that_grow(bpf, kind, n, before):
+    """before: rows of a diagonal ahead of the dense block (so many that the solves go by rows)."""
+    import torch
+
+    RF = bpf.CUSOLVERRF
+    L, U = _growing(kind, n)
+    safe = np.random.default_rng(1).standard_normal((n, n)) + 2.0 * n * np.eye(n)   # the analysis keeps the order
+    D = sp.identity(before, format="csr")
+    gA = bpf.CuSparseMatrixCSR.from_scipy(sp.csr_matrix(sp.block_diag([D, sp.csr_matrix(safe)])))
+    rf = RF.CusolverRfLU(gA, ordering="NATURAL")
+    A = L @ U
+    gA.nzVal[before:] = torch.as_tensor(A.reshape(-1), device="cuda")
+    RF.update_(rf, gA)
+    rng = np.random.default_rng(n)
+    for p in (1, 5, 17):
+        Xt = rng.standard_normal((n, p))
+        B = A @ Xt
+        X = _block(np.vstack([np.ones((before, p)), B]))
+        RF.ldiv_(rf, X)
+        X = X.cpu().numpy()[before:]
+        bound = 6 * n * 2.0**-52 * ((np.abs(L) + 1e-4) @ ((np.abs(U) + 1e-4) @ np.abs(X)))
+        assert np.all(np.abs(B - A @ X) <= bound), p
