@@ -401,9 +401,18 @@ bpf_status spmm_colmajor(bpf_ctx *ctx, int n, long long nnz, const int *rp, cons
 // ------------------------------------------------------------------------------------
 // layout conversions (32x32 tiles through shared memory)
 // ------------------------------------------------------------------------------------
+// *gate may be cleared by another stream meanwhile: a CTA decides once.
+__device__ __forceinline__ bool gated_off(const int *gate) {
+    if (!gate) return false;
+    __shared__ int off;
+    if (threadIdx.x == 0 && threadIdx.y == 0) off = *gate == 0;
+    __syncthreads();
+    return off != 0;
+}
+
 __global__ void cm_to_rm_kernel(int n, int p, const double *__restrict__ src, int ld,
                                 double *__restrict__ dst, const int *gate) {
-    if (gate && *gate == 0) return;
+    if (gated_off(gate)) return;
     __shared__ double tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -419,7 +428,7 @@ __global__ void cm_to_rm_kernel(int n, int p, const double *__restrict__ src, in
 
 __global__ void rm_to_cm_kernel(int n, int p, const double *__restrict__ src,
                                 double *__restrict__ dst, int ld, const int *gate) {
-    if (gate && *gate == 0) return;
+    if (gated_off(gate)) return;
     __shared__ double tile[32][33];
     const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
