@@ -20,10 +20,12 @@
 //    tail between the sweeps); larger systems by a data flow over rows, a warp per row with the
 //    right-hand sides over the lanes, the tail on the FP64 tensor pipe eight columns a CTA.
 //
-// Measured: 25,000 buses, refactor 14.5 -> 1.32 ms, solve of 256 columns 10.8 -> 1.04 ms; 9,000 buses
-// refactor 2.7 ms -> 436 us, 64 columns 2.8 ms -> 266 us; 300 buses, refactor + one column 578 -> 144 us.
-// What bounds it now (25,000 buses): the level chains of the short rows (450 us) and of the rows a CTA
-// takes (456 us), and the tail's 12 block steps (412 us, of which the diagonal tiles ~23 us each).
+// Measured (cold caches, column steps and push solves -> this): 25,000 buses, refactor 14.3 -> 1.45 ms, 256 columns
+// 11.2 -> 1.13 ms; 9,000 buses, refactor 3.6 ms -> 666 us, 64 columns 2.6 ms -> 377 us; 300 buses, refactor 273 ->
+// 104 us, one column 351 -> 49 us.  Errors: 0.89 of those of the column steps (forward, geometric mean over 70 grids
+// of 300 to 9,000 buses against solutions refined in extended precision).
+// What bounds it now (25,000 buses): the level chains of the short rows (470 us) and of the rows a CTA
+// takes (465 us), and the tail's 12 block steps (363 us, of which the diagonal tiles ~20 us each).
 #include <algorithm>
 #include <atomic>
 #include <cmath>

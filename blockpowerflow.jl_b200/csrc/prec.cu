@@ -7,13 +7,13 @@
 // Design (B200):
 //  * One host analysis per sparsity pattern: dependency levels of the forward and backward
 //    solves, rows stored level by level (so a level's rows are contiguous), and for the
-//    numeric factorization the list of (destination, source) update pairs of every L entry.
+//    numeric factorization the updates of every L entry, as lists over its row or as pairs.
 //  * ILU(0) is factored as a data flow (factor_df_kernel: rows wait for the values they read);
 //    IC(0), and rows too long for shared memory, by a cooperative kernel with a grid barrier per
 //    level (factor_coop_kernel).
-//  * ldiv! solves one right-hand side per CTA in shared memory while the column fits
-//    (trsv_col.cu); larger factors run here in ONE cooperative launch, sync-free for 17-256 columns
-//    (trsv_sf_kernel), level by level otherwise (trsv2_coop_kernel): a group of G lanes per row,
+//  * ldiv! solves one right-hand side per CTA in shared memory (trsv_col.cu) where the column fits
+//    and that is faster (prec_by_columns); others run here in ONE cooperative launch, sync-free for 17-256
+//    columns (trsv_sf_kernel), level by level otherwise (trsv2_coop_kernel): a group of G lanes per row,
 //    lanes over the p right-hand sides of the row-major block, the row's (col, val) pairs broadcast
 //    by shuffles.
 //  * FP32 factors (factor_dtype = BPF_F32) keep float copies of L, U and 1/diag, read half the

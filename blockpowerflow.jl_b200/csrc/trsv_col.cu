@@ -1,5 +1,6 @@
 // Triangular solves with one right-hand side per CTA, the whole column in shared memory
-// (ILU(0) / IC(0) factors of up to 24,800 rows in FP64, 49,600 in FP32).
+// (ILU(0) / IC(0) factors of up to 24,767 rows in FP64, about 49,600 in FP32, where that is the faster way:
+// prec_by_columns in prec.cu has the line and both sides' times).
 //
 // Reference: ldiv! of src/preconditioners_nvidia.jl:13-35,49-71 (two cusparseSpSM / SpSV).
 //
